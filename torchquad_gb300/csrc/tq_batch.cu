@@ -237,24 +237,24 @@ __global__ void __launch_bounds__(256) batch_grid_kernel(BatchArgs a) {
     rt = &rt_s;
   }
   for (int64_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
-    if (threadIdx.x == 0) {
-      int64_t lo = 0, hi = a.n_int;  // largest i with tile_start[i] <= tile
-      while (hi - lo > 1) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (a.tile_start[mid] <= tile) lo = mid;
-        else hi = mid;
+    if (threadIdx.x < 32) {
+      const int64_t i = warp_find_start(a.tile_start, a.n_int, tile);
+      if (threadIdx.x == 0) {
+        d = a.desc[i];
+        tile0 = a.tile_start[i];
       }
-      d = a.desc[lo];
-      tile0 = a.tile_start[lo];
+      __syncwarp();
       geo_setup<T, T>(g, d.rule, d.dim, d.n, (const T*)a.domains + d.dom_off);
       load_family<T>(fam, a.family >= 0 ? a.family : d.family, d.dim, a.params + d.par_off);
-      uint64_t st = 1;
-      for (int k = d.dim - 2; k >= 0; --k) {
-        rstride[k] = st;
-        st *= (uint64_t)d.n;
-      }
       if constexpr (std::is_same<T, float>::value)
-        for (int k = 0; k < d.dim; ++k) wsf[k] = f2_from_double(g.wscale[k]);
+        if (threadIdx.x < d.dim) wsf[threadIdx.x] = f2_from_double(g.wscale[threadIdx.x]);
+      if (threadIdx.x == 0) {
+        uint64_t st = 1;
+        for (int k = d.dim - 2; k >= 0; --k) {
+          rstride[k] = st;
+          st *= (uint64_t)d.n;
+        }
+      }
     }
     __syncthreads();
     Acc acc{CUDART_NAN, 0.0};  // an unknown family (rejected on the host) gives NaN
@@ -288,8 +288,7 @@ __global__ void batch_finalize_kernel(const int64_t* tile_start, int64_t n_int, 
   const int64_t t0 = tile_start[w], t1 = tile_start[w + 1];
   Acc a{0.0, 0.0};
   for (int64_t t = t0 + lane; t < t1; t += 32) acc_merge(a, partials[t]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc_merge(a, acc_shfl_down(a, o));
+  a = warp_reduce(a);
   if (lane == 0) {
     const double v = a.s + a.c;
     if (out_dtype == TQ_F64)
@@ -431,18 +430,17 @@ __global__ void __launch_bounds__(256) batch_mc_kernel(BatchMcArgs a) {
   __shared__ McDesc d;
   __shared__ int64_t tile0;
   for (int64_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
-    if (threadIdx.x == 0) {
-      int64_t l = 0, h = a.n_req;
-      while (h - l > 1) {
-        const int64_t m = (l + h) >> 1;
-        if (a.tile_start[m] <= tile) l = m;
-        else h = m;
+    if (threadIdx.x < 32) {
+      const int64_t i = warp_find_start(a.tile_start, a.n_req, tile);
+      if (threadIdx.x == 0) {
+        d = a.desc[i];
+        tile0 = a.tile_start[i];
       }
-      d = a.desc[l];
-      tile0 = a.tile_start[l];
+      __syncwarp();
       load_family<T>(fam, a.family >= 0 ? a.family : d.family, d.dim, a.params + d.par_off);
       const T* dom = (const T*)a.domains + d.dom_off;
-      for (int k = 0; k < d.dim; ++k) {
+      const int k = threadIdx.x;
+      if (k < d.dim) {
         lo[k] = dom[2 * k];
         wid[k] = dom[2 * k + 1] - dom[2 * k];
       }
@@ -486,11 +484,8 @@ __global__ void batch_mc_finalize_kernel(const int64_t* tile_start, int64_t n_re
     acc_merge(s1, partials[2 * t]);
     acc_merge(s2, partials[2 * t + 1]);
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    acc_merge(s1, acc_shfl_down(s1, o));
-    acc_merge(s2, acc_shfl_down(s2, o));
-  }
+  s1 = warp_reduce(s1);
+  s2 = warp_reduce(s2);
   if (lane == 0) {
     Acc r1{acc[4 * w], acc[4 * w + 1]}, r2{acc[4 * w + 2], acc[4 * w + 3]};
     acc_merge(r1, s1);

@@ -64,28 +64,147 @@ __device__ __forceinline__ Acc acc_shfl_down(const Acc& a, int off) {
   r.c = __shfl_down_sync(0xffffffffu, a.c, off);
   return r;
 }
-// Fixed-order reduction of one Acc per thread (blockDim.x <= BLOCK, whole
-// warps); result valid in thread 0.  One warp combines the partials: lane l
-// merges partials l, l + 32, ... in order, then the lanes in a shuffle tree.
-// (Merging in every warp first ran five compensated merges on all 256
-// threads: on GB300, where an FP64 warp instruction holds the FP64 unit for
-// about 64 cycles, that cost more than the grid itself for a C1-sized
-// fused launch.)
+// ------------------------------------------------------ exact CTA sums
+// Sums of doubles as fixed-point integers.  A compensated fp64 tree over a
+// CTA takes about 130 dependent FP64 warp instructions, and on GB300 each
+// holds a sub-partition's FP64 unit for about 64 cycles (4 us a reduction,
+// more than the work of a small launch).  Here every value is placed in a
+// 96-bit window below the CTA's largest binary exponent, as four signed
+// 24-bit limbs (integer shifts only), the limbs are summed over a warp by
+// redux.sync and over the CTA as 64-bit integers, and one thread turns the
+// total into hi + lo doubles by bit moves.  Integer sums are exact and do
+// not depend on their order; a value loses only bits below 2^-95 of the
+// largest.  A 101^3 fused Simpson launch (252 CTAs): 25.5 us with the fp64
+// trees, 18.7 us with these sums and the
+// dimensions set up in parallel; a 10001-node rule over 200 components (50
+// reductions a component group): 969 and 431 us.
+__device__ __forceinline__ int exp_field(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+
+// L += v in units of 2^(emax - 1118) (limb i has weight 2^(24 i)); v finite,
+// its exponent field at most emax, emax >= 1.
+__device__ __forceinline__ void fix_add(int (&L)[4], double v, int emax) {
+  const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+  const int ef = (int)(hi >> 20) & 0x7ff;
+  const uint32_t mh = (hi & 0xfffffu) | (ef ? 0x100000u : 0u);
+  const int s = emax - (ef ? ef : 1);
+  const uint32_t w2 = (mh << 11) | (lo >> 21), w1 = lo << 11;  // mantissa << 43, 96 bits
+  uint32_t a2 = w2 >> (s & 31), a1 = __funnelshift_r(w1, w2, s), a0 = __funnelshift_r(0u, w1, s);
+  const int q = s >> 5;
+  a0 = q == 0 ? a0 : q == 1 ? a1 : q == 2 ? a2 : 0u;
+  a1 = q == 0 ? a1 : q == 1 ? a2 : 0u;
+  a2 = q == 0 ? a2 : 0u;
+  const int sg = (int)hi >> 31;
+  L[0] += ((int)(a0 & 0xffffffu) ^ sg) - sg;
+  L[1] += ((int)(__funnelshift_r(a0, a1, 24) & 0xffffffu) ^ sg) - sg;
+  L[2] += ((int)(__funnelshift_r(a1, a2, 16) & 0xffffffu) ^ sg) - sg;
+  L[3] += ((int)(a2 >> 8) ^ sg) - sg;
+}
+
+// The leading 53 bits of A 2^p as a double (truncated); A keeps the rest.
+__device__ __forceinline__ double fix_take(unsigned __int128& A, int p) {
+  const uint64_t ah = (uint64_t)(A >> 64), al = (uint64_t)A;
+  if ((ah | al) == 0) return 0.0;
+  const int n = ah ? 127 - __clzll((long long)ah) : 63 - __clzll((long long)al);  // leading bit
+  uint64_t top;
+  if (n > 52) {
+    top = (uint64_t)(A >> (n - 52));
+    A -= (unsigned __int128)top << (n - 52);
+  } else {
+    top = al << (52 - n);
+    A = 0;
+  }
+  const int e = n + p + 1023;
+  if (e >= 1 && e <= 2046)
+    return __longlong_as_double((long long)(((uint64_t)e << 52) | (top & 0xfffffffffffffull)));
+  return scalbn((double)(long long)top, n - 52 + p);  // subnormal or infinite
+}
+// The total of the limb sums S in units of 2^(emax - 1118) as hi + lo.
+__device__ __forceinline__ Acc fix_value(const int64_t (&S)[4], int emax) {
+  __int128 t = (__int128)S[0] + ((__int128)S[1] << 24) + ((__int128)S[2] << 48) + ((__int128)S[3] << 72);
+  const bool neg = t < 0;
+  unsigned __int128 A = neg ? (unsigned __int128)(-t) : (unsigned __int128)t;
+  Acc r;
+  r.s = fix_take(A, emax - 1118);
+  r.c = fix_take(A, emax - 1118);
+  if (neg) {
+    r.s = -r.s;
+    r.c = -r.c;
+  }
+  return r;
+}
+
+// Sum of one Acc per lane over a warp; result valid in lane 0.
+__device__ __forceinline__ Acc warp_reduce(Acc a) {
+  const int emax = max(1, __reduce_max_sync(0xffffffffu, max(exp_field(a.s), exp_field(a.c))));
+  if (emax == 0x7ff) {  // infinities or NaN: in the floating format
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) acc_merge(a, acc_shfl_down(a, off));
+    return a;
+  }
+  int L[4] = {0, 0, 0, 0};
+  fix_add(L, a.s, emax);
+  fix_add(L, a.c, emax);
+  int64_t S[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) S[i] = __reduce_add_sync(0xffffffffu, L[i]);
+  return fix_value(S, emax);
+}
+
+// Sum of one Acc per thread over the CTA (blockDim.x <= BLOCK, whole
+// warps); result valid in thread 0.
 template <int BLOCK>
 __device__ __forceinline__ Acc block_reduce(Acc a) {
-  __shared__ Acc part[BLOCK];
-  part[threadIdx.x] = a;
+  constexpr int kW = BLOCK / 32;
+  __shared__ int wexp[kW];
+  __shared__ int wlimb[kW][4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+  const int e = __reduce_max_sync(0xffffffffu, max(exp_field(a.s), exp_field(a.c)));
+  if (lane == 0) wexp[warp] = e;
   __syncthreads();
-  if (threadIdx.x < 32) {
-    const int nt = min(BLOCK, (int)blockDim.x);
-    Acc r = part[threadIdx.x];
-    for (int i = threadIdx.x + 32; i < nt; i += 32) acc_merge(r, part[i]);
+  int emax = 1;
+  for (int i = 0; i < nw; ++i) emax = max(emax, wexp[i]);
+  if (emax == 0x7ff) {  // infinities or NaN: in the floating format
+    __shared__ Acc part[kW];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc_merge(r, acc_shfl_down(r, off));
-    a = r;
+    for (int off = 16; off > 0; off >>= 1) acc_merge(a, acc_shfl_down(a, off));
+    if (lane == 0) part[warp] = a;
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int i = 1; i < nw; ++i) acc_merge(a, part[i]);
+    __syncthreads();
+    return a;
+  }
+  int L[4] = {0, 0, 0, 0};
+  fix_add(L, a.s, emax);
+  fix_add(L, a.c, emax);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) L[i] = __reduce_add_sync(0xffffffffu, L[i]);
+  if (lane == 0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) wlimb[warp][i] = L[i];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int64_t S[4] = {0, 0, 0, 0};
+    for (int w = 0; w < nw; ++w) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) S[i] += wlimb[w][i];
+    }
+    a = fix_value(S, emax);
   }
   __syncthreads();
   return a;
+}
+
+// Sum of the partials [0, n) of a launch's CTAs by the last of them; result
+// valid in thread 0.
+template <int BLOCK>
+__device__ __forceinline__ Acc partials_reduce(const Acc* partials, int n) {
+  Acc t{0.0, 0.0};
+  int i = threadIdx.x;
+  if (i < n) t = partials[i];
+  for (i += blockDim.x; i < n; i += blockDim.x) acc_merge(t, partials[i]);
+  return block_reduce<BLOCK>(t);
 }
 
 // fp32 compensated strip accumulator (cheap on the FP32 pipe).
@@ -335,17 +454,22 @@ struct Family {
   T a[kMaxDim];
   T u[kMaxDim];
 };
+// One dimension per thread (threads 0 .. kMaxDim - 1 of the CTA; the caller
+// puts a barrier before the first use): a conversion from fp64 holds the
+// FP64 unit as long for one lane as for a warp.
 template <typename T>
 __device__ __forceinline__ void load_family(Family<T>& f, int id, int dim,
                                             const double* __restrict__ p) {
-  f.id = id;
-  f.dim = dim;
-  f.c = (T)p[0];
-  f.b = (T)p[1];
-#pragma unroll
-  for (int k = 0; k < kMaxDim; ++k) {
+  const int k = threadIdx.x;
+  if (k < kMaxDim) {
     f.a[k] = k < dim ? (T)p[2 + k] : T(0);
     f.u[k] = (k < dim && id == TQ_FN_GAUSSIAN) ? (T)p[2 + dim + k] : T(0);
+  }
+  if (k == 0) {
+    f.id = id;
+    f.dim = dim;
+    f.c = (T)p[0];
+    f.b = (T)p[1];
   }
 }
 // g_k(x_k): the per-dimension term of the separable sum.

@@ -479,9 +479,9 @@ __global__ void __launch_bounds__(kBlock) grid_adjoint_kernel(GradArgs args) {
   __shared__ uint64_t rstride[kMaxDim];
   __shared__ double sh[kBlock / 32][2 + 4 * DM];
   __shared__ AdjTab tab;
+  geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
+  load_family<T>(fam, args.family, args.dim, args.params);
   if (threadIdx.x == 0) {
-    geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
-    load_family<T>(fam, args.family, args.dim, args.params);
     uint64_t st = 1;
     for (int k = args.dim - 2; k >= 0; --k) {
       rstride[k] = st;
@@ -515,8 +515,7 @@ __global__ void __launch_bounds__(kBlock) grid_adjoint_kernel(GradArgs args) {
     for (int i = warp; i < nacc; i += blockDim.x >> 5) {
       Acc a{0.0, 0.0};
       for (unsigned b = lane; b < gridDim.x; b += 32) acc_add(a, args.partials[(int64_t)b * nacc + i]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc_merge(a, acc_shfl_down(a, o));
+      a = warp_reduce(a);
       if (lane == 0) tot[i] = a.s + a.c;
     }
     __syncthreads();
@@ -606,15 +605,13 @@ __global__ void __launch_bounds__(kBlock, DM <= 4 ? 2 : 1) batch_adjoint_kernel(
   __shared__ int64_t tile0;
   constexpr bool kF32 = std::is_same<D, float>::value;
   for (int64_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
-    if (threadIdx.x == 0) {
-      int64_t lo = 0, hi = a.n_int;  // largest i with tile_start[i] <= tile
-      while (hi - lo > 1) {
-        const int64_t mid = (lo + hi) >> 1;
-        if (a.tile_start[mid] <= tile) lo = mid;
-        else hi = mid;
+    if (threadIdx.x < 32) {
+      const int64_t i = warp_find_start(a.tile_start, a.n_int, tile);
+      if (threadIdx.x == 0) {
+        d = a.desc[i];
+        tile0 = a.tile_start[i];
       }
-      d = a.desc[lo];
-      tile0 = a.tile_start[lo];
+      __syncwarp();
       const int fid = a.family >= 0 ? a.family : d.family;
       const D* dom = (const D*)a.domains + d.dom_off;
       if (kF32 && d.rule != TQ_RULE_GAUSS) {
@@ -624,10 +621,12 @@ __global__ void __launch_bounds__(kBlock, DM <= 4 ? 2 : 1) batch_adjoint_kernel(
         geo_setup<double, D>(g64, d.rule, d.dim, d.n, dom);
         load_family<double>(fam64, fid, d.dim, a.params + d.par_off);
       }
-      uint64_t st = 1;
-      for (int k = d.dim - 2; k >= 0; --k) {
-        rstride[k] = st;
-        st *= (uint64_t)d.n;
+      if (threadIdx.x == 0) {
+        uint64_t st = 1;
+        for (int k = d.dim - 2; k >= 0; --k) {
+          rstride[k] = st;
+          st *= (uint64_t)d.n;
+        }
       }
     }
     __syncthreads();
@@ -656,8 +655,7 @@ __global__ void batch_adjoint_finalize_kernel(BatchGradArgs a, double* out_value
   for (int i = 0; i < nacc; ++i) {
     Acc s{0.0, 0.0};
     for (int64_t t = t0 + lane; t < t1; t += 32) acc_add(s, a.partials[t * a.stride + i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc_merge(s, acc_shfl_down(s, o));
+    s = warp_reduce(s);
     if (lane == 0) tot[wib][i] = s.s + s.c;
   }
   __syncwarp();

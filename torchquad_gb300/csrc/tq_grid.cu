@@ -104,9 +104,9 @@ __global__ void __launch_bounds__(kBlock, 2) grid_fused_kernel(FusedArgs args) {
   __shared__ Geo<T> g;
   __shared__ Family<T> fam;
   __shared__ uint64_t rstride[kMaxDim];
+  geo_setup<T, D>(g, RULE, args.dim, args.n, (const D*)args.domain);
+  load_family<T>(fam, args.family, args.dim, args.params);
   if (threadIdx.x == 0) {
-    geo_setup<T, D>(g, RULE, args.dim, args.n, (const D*)args.domain);
-    load_family<T>(fam, args.family, args.dim, args.params);
     uint64_t st = 1;
     for (int k = args.dim - 2; k >= 0; --k) {
       rstride[k] = st;
@@ -214,9 +214,7 @@ __global__ void __launch_bounds__(kBlock, 2) grid_fused_kernel(FusedArgs args) {
   acc = block_reduce<kBlock>(acc);
   if (threadIdx.x == 0) args.partials[blockIdx.x] = acc;
   if (last_block_arrives(args.ticket)) {
-    Acc t{0.0, 0.0};
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) acc_merge(t, args.partials[i]);
-    t = block_reduce<kBlock>(t);
+    const Acc t = partials_reduce<kBlock>(args.partials, (int)gridDim.x);
     if (threadIdx.x == 0) {
       write_result(args.out, args.out_dtype, args.out64, t.s + t.c);
       *args.ticket = 0u;
@@ -239,8 +237,8 @@ template <typename T, typename D, bool GL>
 __global__ void __launch_bounds__(kBlock) grid_points_kernel(PointsArgs args) {
   __shared__ Geo<T> g;
   __shared__ uint64_t stride[kMaxDim];
+  geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
   if (threadIdx.x == 0) {
-    geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
     uint64_t s = 1;
     for (int k = args.dim - 1; k >= 0; --k) {
       stride[k] = s;
@@ -283,8 +281,8 @@ __global__ void __launch_bounds__(kBlock) grid_points_tiled_kernel(PointsArgs ar
   __shared__ Geo<T> g;
   __shared__ FastDiv fd_n;
   __shared__ T nodes[kPtsTab];  // nodes[k * n + j], when dim * n fits
+  geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
   if (threadIdx.x == 0) {
-    geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
     fd_n = make_fastdiv((uint32_t)args.n);
   }
   __syncthreads();
@@ -358,7 +356,7 @@ struct WeightsArgs {
 template <typename T, typename D, bool GL>
 __global__ void __launch_bounds__(kBlock) grid_weights_kernel(WeightsArgs args) {
   __shared__ Geo<T> g;
-  if (threadIdx.x == 0) geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
+  geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
   __syncthreads();
   const int dim = args.dim;
   const uint64_t n = (uint64_t)args.n;
@@ -395,7 +393,7 @@ struct WsumArgs {
 template <typename T, typename D, bool GL, typename F, int P>
 __global__ void __launch_bounds__(kBlock) weighted_sum_kernel(WsumArgs args) {
   __shared__ Geo<T> g;
-  if (threadIdx.x == 0) geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
+  geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
   __syncthreads();
   const int dim = args.dim, rule = args.rule;
   const uint64_t n = (uint64_t)args.n;
@@ -503,9 +501,7 @@ __device__ __forceinline__ void wsum_finish(const WsumArgs& args, Acc acc) {
   acc = block_reduce<kBlock>(acc);
   if (threadIdx.x == 0) args.partials[blockIdx.x] = acc;
   if (last_block_arrives(args.ticket)) {
-    Acc t{0.0, 0.0};
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) acc_merge(t, args.partials[i]);
-    t = block_reduce<kBlock>(t);
+    const Acc t = partials_reduce<kBlock>(args.partials, (int)gridDim.x);
     if (threadIdx.x == 0) {
       Acc run{args.acc[0], args.acc[1]};
       acc_merge(run, t);
@@ -525,8 +521,8 @@ __global__ void __launch_bounds__(kBlock) weighted_sum1_kernel(WsumArgs args) {
   __shared__ Geo<T> g;
   __shared__ FastDiv fd_n;
   __shared__ F wt[kWTab];
+  geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
   if (threadIdx.x == 0) {
-    geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
     fd_n = make_fastdiv((uint32_t)args.n);
   }
   const int dim = args.dim, rule = args.rule, last = dim - 1;
@@ -618,8 +614,8 @@ __global__ void __launch_bounds__(kBlock) weighted_sum_rows_kernel(WsumArgs args
   __shared__ FastDiv fd_n;
   __shared__ F wl[kRowTab];       // unscaled last-dimension weights
   __shared__ double wo[kRowTab];  // wo[k*n + j] = wscale_k * W_k(j), outer dimensions k
+  geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
   if (threadIdx.x == 0) {
-    geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
     fd_n = make_fastdiv((uint32_t)args.n);
   }
   __syncthreads();
@@ -695,8 +691,8 @@ __global__ void __launch_bounds__(kBlock) weighted_sum_rows_f2_kernel(WsumArgs a
   __shared__ F2 red[kBlock / 32];
   __shared__ unsigned umin_bits, umax_bits;  // extreme |unit weight| (Gauss), as float bits
   __shared__ int use_f2;
+  geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
   if (threadIdx.x == 0) {
-    geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
     fd_n = make_fastdiv((uint32_t)args.n);
     umin_bits = 0x7f7fffffu;
     umax_bits = 0u;
@@ -853,9 +849,7 @@ __global__ void __launch_bounds__(kBlock) weighted_sum_rows_f2_kernel(WsumArgs a
   }
   if (threadIdx.x == 0) args.partials[blockIdx.x] = acc;
   if (last_block_arrives(args.ticket)) {
-    Acc t{0.0, 0.0};
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) acc_merge(t, args.partials[i]);
-    t = block_reduce<kBlock>(t);
+    const Acc t = partials_reduce<kBlock>(args.partials, (int)gridDim.x);
     if (threadIdx.x == 0) {
       Acc run{args.acc[0], args.acc[1]};
       acc_merge(run, t);

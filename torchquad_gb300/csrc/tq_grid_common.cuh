@@ -16,6 +16,22 @@ struct Geo {
   double half[kMaxDim], mid[kMaxDim];  // Gauss node map (b-a)/2 * r + (a+b)/2
 };
 
+// Largest i in [0, n) with start[i] <= t (start[0] = 0 <= t): a 32-ary search
+// by one whole warp (three probes of a batch of 4096, where one thread's
+// bisection takes twelve dependent loads).
+__device__ __forceinline__ int64_t warp_find_start(const int64_t* __restrict__ start, int64_t n, int64_t t) {
+  const int lane = threadIdx.x & 31;
+  int64_t lo = 0, hi = n;
+  while (hi - lo > 1) {
+    const int64_t step = (hi - lo + 31) / 32;
+    const int64_t pos = lo + lane * step;
+    const unsigned m = __ballot_sync(0xffffffffu, pos < hi && __ldg(start + pos) <= t);
+    lo += (int64_t)(31 - __clz(m)) * step;
+    hi = min(hi, lo + step);
+  }
+  return lo;
+}
+
 // Integer part of the Newton-Cotes weights (exact in any float type).
 __device__ __forceinline__ int nc_int(int rule, int64_t i, int64_t n) {
   if (rule == TQ_RULE_TRAPEZOID) return (i == 0 || i == n - 1) ? 1 : 2;
@@ -28,10 +44,14 @@ __host__ __device__ __forceinline__ double nc_den(int rule) {
   return rule == TQ_RULE_TRAPEZOID ? 2.0 : (rule == TQ_RULE_SIMPSON ? 3.0 : 22.5);
 }
 
-// D = domain type.  Fills g from domain[dim][2] (device, read by thread 0).
+// D = domain type.  Fills g from domain[dim][2] on the device, one dimension
+// per thread (threads 0 .. dim - 1; the caller puts a barrier before the
+// first use): the two fp64 divisions of a dimension cost thousands of cycles
+// when one thread does the dimensions in turn.
 template <typename T, typename D>
 __device__ void geo_setup(Geo<T>& g, int rule, int dim, int64_t n, const D* __restrict__ dom) {
-  for (int k = 0; k < dim; ++k) {
+  const int k = threadIdx.x;
+  if (k < dim) {
     const D a = dom[2 * k], b = dom[2 * k + 1];
     g.a[k] = (T)a;
     g.b[k] = (T)b;

@@ -44,17 +44,12 @@ template <typename T, int FAM, int P>
 __global__ void __launch_bounds__(kBlock) mc_fused_kernel(McArgs a) {
   __shared__ Family<T> fam;
   __shared__ T lo[kMaxDim], width[kMaxDim];
-  __shared__ T volume;
   const T* dom = (const T*)a.domain;
-  if (threadIdx.x == 0) {
-    load_family<T>(fam, a.family, a.dim, a.params);
-    T v = (T)1;
-    for (int k = 0; k < a.dim; ++k) {
-      lo[k] = dom[2 * k];
-      width[k] = dom[2 * k + 1] - dom[2 * k];
-      v = v * width[k];
-    }
-    volume = v;
+  load_family<T>(fam, a.family, a.dim, a.params);
+  if (threadIdx.x < a.dim) {
+    const int k = threadIdx.x;
+    lo[k] = dom[2 * k];
+    width[k] = dom[2 * k + 1] - dom[2 * k];
   }
   __syncthreads();
   constexpr int PB = Uniform<T>::per_block;
@@ -98,10 +93,10 @@ __global__ void __launch_bounds__(kBlock) mc_fused_kernel(McArgs a) {
   acc = block_reduce<kBlock>(acc);
   if (threadIdx.x == 0) a.partials[blockIdx.x] = acc;
   if (last_block_arrives(a.ticket)) {
-    Acc t{0.0, 0.0};
-    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) acc_merge(t, a.partials[i]);
-    t = block_reduce<kBlock>(t);
+    const Acc t = partials_reduce<kBlock>(a.partials, (int)gridDim.x);
     if (threadIdx.x == 0) {
+      T volume = (T)1;
+      for (int k = 0; k < dim; ++k) volume = volume * width[k];
       const double v = (double)volume * (t.s + t.c) / (double)a.n_points;
       if (a.out) *(T*)a.out = (T)v;
       if (a.out64) *a.out64 = v;

@@ -270,16 +270,19 @@ __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk) {
   const int64_t DB = d * B;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   Smem<T> sm = carve<T>(smem_raw, a);
-  if (threadIdx.x == 0) {
-    load_family<T>(fam, a.family, d, a.params);
+  load_family<T>(fam, a.family, d, a.params);
+  if (threadIdx.x < 32) {
     const T* dom = (const T*)st.domain;
-    T v = (T)1;
-    for (int k = 0; k < d; ++k) {
+    const int k = threadIdx.x;
+    T w = (T)1;
+    if (k < d) {
+      w = sub_rn(dom[2 * k + 1], dom[2 * k]);
       lo[k] = dom[2 * k];
-      wid[k] = sub_rn(dom[2 * k + 1], dom[2 * k]);
-      v = mul_rn(v, wid[k]);
+      wid[k] = w;
     }
-    volume = v;
+    T v = (T)1;  // the widths' product in dimension order
+    for (int i = 0; i < d; ++i) v = mul_rn(v, __shfl_sync(0xffffffffu, w, i));
+    if (k == 0) volume = v;
   }
   if (a.edges_smem) {
     for (int64_t i = threadIdx.x; i < d * (B + 1); i += blockDim.x) sm.xe[i] = ((const T*)st.x_edges)[i];
