@@ -3,10 +3,11 @@
 //
 // Each integral i is cut into tiles of `tile_pts` consecutive flat node
 // indices; tile_start[i] is the exclusive prefix of the tile counts.  CTAs
-// stride over the flat tile list, find a tile's integral by binary search in
+// stride over the flat tile list, find a tile's integral by a search in
 // tile_start, set the integral's geometry up in shared memory and sum the
 // tile's nodes with the same row-segment walk as the single fused rule
-// (strips of P nodes per thread, last dimension innermost).  Each tile's
+// (strips of P nodes per thread, last dimension innermost); an integral whose
+// rule factors safely is done by its 1-D sums in its first tile.  Each tile's
 // compensated partial goes to partials[tile]; a second kernel reduces every
 // integral's tiles in tile order (deterministic, no atomics).
 //
@@ -15,7 +16,7 @@
 
 #include <type_traits>
 
-#include "tq_grid_common.cuh"
+#include "tq_separable.cuh"
 
 namespace tq {
 
@@ -216,6 +217,19 @@ __device__ Acc grid_tile_sum(const BatchArgs& a, const BatchDesc& d, int64_t til
   return block_reduce<256>(acc);
 }
 
+// One integral by its 1-D sums (tq_separable.cuh), by one CTA; valid in
+// thread 0.
+template <typename T, int FAM>
+__device__ Acc sep_integral(const BatchArgs& a, const BatchDesc& d, const Geo<T>& g, const Family<T>& fam,
+                            Acc (*dsum)[kSepMaxM<false>], Acc* sp) {
+  Acc v{0.0, 0.0};
+  sep_sums<T, FAM, false>(g, fam, d.rule, d.dim, d.n, a.gl_nodes + d.gl_off, a.gl_weights + d.gl_off, 0u, 1u,
+                          nullptr, 0, nullptr, dsum, sp);
+  if (threadIdx.x < 32) v = dd_mul(sep_value<FAM>(dsum, d.dim), (double)fam.c);
+  __syncthreads();  // dsum and sp are rewritten by the next integral
+  return v;
+}
+
 // Persistent launch over the flat tile list.  The family of a tile's
 // integral is the launch's (a.family >= 0) or its descriptor's, so one
 // launch can mix families; the switch is uniform across a CTA.
@@ -236,46 +250,76 @@ __global__ void __launch_bounds__(256) batch_grid_kernel(BatchArgs a) {
     tab = &tab_s;
     rt = &rt_s;
   }
-  for (int64_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
-    if (threadIdx.x < 32) {
-      const int64_t i = warp_find_start(a.tile_start, a.n_int, tile);
-      if (threadIdx.x == 0) {
-        d = a.desc[i];
-        tile0 = a.tile_start[i];
-      }
-      __syncwarp();
-      geo_setup<T, T>(g, d.rule, d.dim, d.n, (const T*)a.domains + d.dom_off);
-      load_family<T>(fam, a.family >= 0 ? a.family : d.family, d.dim, a.params + d.par_off);
-      if constexpr (std::is_same<T, float>::value)
-        if (threadIdx.x < d.dim) wsf[threadIdx.x] = f2_from_double(g.wscale[threadIdx.x]);
-      if (threadIdx.x == 0) {
-        uint64_t st = 1;
-        for (int k = d.dim - 2; k >= 0; --k) {
-          rstride[k] = st;
-          st *= (uint64_t)d.n;
+  __shared__ int64_t ti[8], ts[8], te[8];  // a round's integrals and their tile ranges
+  __shared__ int tsep[8];
+  __shared__ Acc dsum[kMaxDim][kSepMaxM<false>];
+  __shared__ Acc sp[kSepSlots<false>];
+  const int nw = (int)(blockDim.x >> 5), warp = threadIdx.x >> 5;
+  // Rounds of one tile per warp: the warps look their tiles' integrals up and
+  // decide on the factored form in parallel (dependent loads), then the CTA
+  // does the tiles.  An integral in factored form is done whole at its first
+  // tile; its other tiles are zeros and cost the look-up only.
+  for (int64_t base = blockIdx.x; base < a.n_tiles; base += (int64_t)nw * gridDim.x) {
+    {
+      const int64_t tile = base + (int64_t)warp * gridDim.x;
+      if (tile < a.n_tiles) {
+        const int64_t i = warp_find_start(a.tile_start, a.n_int, tile);
+        const BatchDesc& di = a.desc[i];
+        // one dimension: the rows' recurrences take fewer FP64 operations a node
+        const bool sep = (di.dim > 1 || di.rule == TQ_RULE_GAUSS) &&
+                         sep_ok<T, T>(a.family >= 0 ? a.family : di.family, di.dim, di.n,
+                                      (const T*)a.domains + di.dom_off, a.params + di.par_off);
+        if ((threadIdx.x & 31) == 0) {
+          ti[warp] = i;
+          ts[warp] = a.tile_start[i];
+          te[warp] = a.tile_start[i + 1];
+          tsep[warp] = sep;
         }
       }
     }
     __syncthreads();
-    Acc acc{CUDART_NAN, 0.0};  // an unknown family (rejected on the host) gives NaN
-    switch (fam.id) {
-      case TQ_FN_EXP_SUM:
-        acc = grid_tile_sum<T, TQ_FN_EXP_SUM, P>(a, d, tile, tile0, g, fam, rstride, tab, rt, &fdn, wsf);
-        break;
-      case TQ_FN_GAUSSIAN:
-        acc = grid_tile_sum<T, TQ_FN_GAUSSIAN, P>(a, d, tile, tile0, g, fam, rstride, tab, rt, &fdn, wsf);
-        break;
-      case TQ_FN_OSCILLATORY:
-        acc = grid_tile_sum<T, TQ_FN_OSCILLATORY, P>(a, d, tile, tile0, g, fam, rstride, tab, rt, &fdn, wsf);
-        break;
-      case TQ_FN_SUM_SIN:
-        acc = grid_tile_sum<T, TQ_FN_SUM_SIN, P>(a, d, tile, tile0, g, fam, rstride, tab, rt, &fdn, wsf);
-        break;
-      default:
-        break;
+    for (int r = 0; r < nw; ++r) {
+      const int64_t tile = base + (int64_t)r * gridDim.x;
+      if (tile >= a.n_tiles) break;
+      const bool sep = tsep[r] != 0;
+      if (sep && tile != ts[r]) continue;
+      if (threadIdx.x < 32) {
+        if (threadIdx.x == 0) {
+          d = a.desc[ti[r]];
+          tile0 = ts[r];
+        }
+        __syncwarp();
+        geo_setup<T, T>(g, d.rule, d.dim, d.n, (const T*)a.domains + d.dom_off);
+        load_family<T>(fam, a.family >= 0 ? a.family : d.family, d.dim, a.params + d.par_off);
+        if constexpr (std::is_same<T, float>::value)
+          if (threadIdx.x < d.dim) wsf[threadIdx.x] = f2_from_double(g.wscale[threadIdx.x]);
+        if (threadIdx.x == 0) {
+          uint64_t st = 1;
+          for (int k = d.dim - 2; k >= 0; --k) {
+            rstride[k] = st;
+            st *= (uint64_t)d.n;
+          }
+        }
+      }
+      __syncthreads();
+      Acc acc{CUDART_NAN, 0.0};  // an unknown family (rejected on the host) gives NaN
+#define TQ_BATCH_TILE(FAMC)                                                                              \
+  acc = sep ? sep_integral<T, FAMC>(a, d, g, fam, dsum, sp)                                              \
+            : grid_tile_sum<T, FAMC, P>(a, d, tile, tile0, g, fam, rstride, tab, rt, &fdn, wsf)
+      switch (fam.id) {
+        case TQ_FN_EXP_SUM: TQ_BATCH_TILE(TQ_FN_EXP_SUM); break;
+        case TQ_FN_GAUSSIAN: TQ_BATCH_TILE(TQ_FN_GAUSSIAN); break;
+        case TQ_FN_OSCILLATORY: TQ_BATCH_TILE(TQ_FN_OSCILLATORY); break;
+        case TQ_FN_SUM_SIN: TQ_BATCH_TILE(TQ_FN_SUM_SIN); break;
+        default: break;
+      }
+#undef TQ_BATCH_TILE
+      if (threadIdx.x == 0) a.partials[tile] = acc;
+      if (sep)
+        for (int64_t t = tile + 1 + threadIdx.x; t < te[r]; t += blockDim.x) a.partials[t] = Acc{0.0, 0.0};
+      __syncthreads();
     }
-    if (threadIdx.x == 0) a.partials[tile] = acc;
-    __syncthreads();
+    __syncthreads();  // the round's tables are rewritten
   }
 }
 

@@ -27,7 +27,7 @@
 
 #include <type_traits>
 
-#include "tq_grid_common.cuh"
+#include "tq_separable.cuh"
 
 namespace tq {
 
@@ -434,27 +434,31 @@ __device__ void adj_accumulate(const AdjCtx<T, GL, DM>& c, int64_t first, int64_
 }
 
 // The integral and its gradients from the reduced accumulators tot[2+4*dim]
-// (one thread).
+// (one warp, lane k on dimension k).
 template <typename D>
 __device__ void adj_outputs(const double* tot, int family, double c, const D* dom, int dim,
                             double* out_value, double* out_gdom, double* out_gpar) {
+  const int k = threadIdx.x & 31;
   const double I = c * tot[0];
-  *out_value = I;
-  for (int k = 0; k < dim; ++k) {
+  if (k < dim) {
     const double L = (double)dom[2 * k + 1] - (double)dom[2 * k];
     const double sx = c * tot[2 + k], st = c * tot[2 + dim + k];
-    out_gdom[2 * k] = -I / L + (sx - st);
-    out_gdom[2 * k + 1] = I / L + st;
+    const double q = I / L;
+    out_gdom[2 * k] = -q + (sx - st);
+    out_gdom[2 * k + 1] = q + st;
     out_gpar[2 + k] = c * tot[2 + 2 * dim + k];
     out_gpar[2 + dim + k] = c * tot[2 + 3 * dim + k];
   }
-  out_gpar[0] = tot[0];
-  if (family == TQ_FN_EXP_SUM)
-    out_gpar[1] = c * tot[0];
-  else if (family == TQ_FN_OSCILLATORY)
-    out_gpar[1] = 2.0 * CUDART_PI * c * tot[1];
-  else
-    out_gpar[1] = 0.0;
+  if (k == 0) {
+    *out_value = I;
+    out_gpar[0] = tot[0];
+    if (family == TQ_FN_EXP_SUM)
+      out_gpar[1] = c * tot[0];
+    else if (family == TQ_FN_OSCILLATORY)
+      out_gpar[1] = 2.0 * CUDART_PI * c * tot[1];
+    else
+      out_gpar[1] = 0.0;
+  }
 }
 
 // ----------------------------------------------------------- one integral
@@ -466,6 +470,7 @@ struct GradArgs {
   const double* gl_weights;
   const double* params;
   double* partials;  // [blocks][nacc]
+  int64_t slots;     // 16-byte partials the workspace holds
   unsigned* ticket;
   double* out_value;
   double* out_gdom;  // [dim][2]
@@ -479,8 +484,27 @@ __global__ void __launch_bounds__(kBlock) grid_adjoint_kernel(GradArgs args) {
   __shared__ uint64_t rstride[kMaxDim];
   __shared__ double sh[kBlock / 32][2 + 4 * DM];
   __shared__ AdjTab tab;
+  __shared__ double tot[2 + 4 * kMaxDim];
+  // the factored form (tq_separable.cuh), by the first few CTAs
+  const bool sep = (args.dim > 1 || args.n <= kSepRow) &&
+                   sep_ok<T, D>(FAM, args.dim, args.n, (const D*)args.domain, args.params);
+  if (sep && blockIdx.x >= (unsigned)sep_ctas(args.dim, args.n)) return;
   geo_setup<T, D>(g, args.rule, args.dim, args.n, (const D*)args.domain);
   load_family<T>(fam, args.family, args.dim, args.params);
+  if (sep) {
+    __shared__ Acc dsum[kMaxDim][kSepMaxM<true>];
+    __shared__ Acc sp[kSepSlots<true>];
+    __syncthreads();
+    if (sep_sums<T, FAM, true>(g, fam, args.rule, args.dim, args.n, args.gl_nodes, args.gl_weights, blockIdx.x,
+                               gridDim.x, (Acc*)args.partials, args.slots, args.ticket, dsum, sp) &&
+        threadIdx.x < 32) {
+      sep_adjoint<FAM, T>(dsum, fam.a, args.dim, tot);
+      __syncwarp();
+      adj_outputs<D>(tot, FAM, (double)fam.c, (const D*)args.domain, args.dim, args.out_value, args.out_gdom,
+                     args.out_gpar);
+    }
+    return;
+  }
   if (threadIdx.x == 0) {
     uint64_t st = 1;
     for (int k = args.dim - 2; k >= 0; --k) {
@@ -510,7 +534,6 @@ __global__ void __launch_bounds__(kBlock) grid_adjoint_kernel(GradArgs args) {
   if (last_block_arrives(args.ticket)) {
     // each warp reduces accumulators over the CTAs (strided, compensated,
     // fixed merge order)
-    __shared__ double tot[2 + 4 * kMaxDim];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int i = warp; i < nacc; i += blockDim.x >> 5) {
       Acc a{0.0, 0.0};
@@ -519,11 +542,10 @@ __global__ void __launch_bounds__(kBlock) grid_adjoint_kernel(GradArgs args) {
       if (lane == 0) tot[i] = a.s + a.c;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32)
       adj_outputs<D>(tot, FAM, (double)fam.c, (const D*)args.domain, dim, args.out_value, args.out_gdom,
                      args.out_gpar);
-      *args.ticket = 0u;
-    }
+    if (threadIdx.x == 0) *args.ticket = 0u;
   }
 }
 
@@ -587,6 +609,27 @@ __device__ void batch_adj_dispatch(const BatchGradArgs& a, const tq_batch_desc& 
   }
 }
 
+// One integral by its 1-D sums (tq_separable.cuh), by one CTA, into the
+// partials' row `tile`.
+template <typename T, int FAM>
+__device__ void batch_adj_sep(const BatchGradArgs& a, const tq_batch_desc& d, int64_t tile, const Geo<T>& g,
+                              const Family<T>& fam, Acc (*dsum)[kSepMaxM<true>], Acc* sp) {
+  sep_sums<T, FAM, true>(g, fam, d.rule, d.dim, d.n, a.gl_nodes + d.gl_off, a.gl_weights + d.gl_off, 0u, 1u,
+                         nullptr, 0, nullptr, dsum, sp);
+  if (threadIdx.x < 32) sep_adjoint<FAM, T>(dsum, fam.a, d.dim, a.partials + tile * a.stride);
+}
+template <typename T>
+__device__ void batch_adj_sep_dispatch(const BatchGradArgs& a, const tq_batch_desc& d, int64_t tile,
+                                       const Geo<T>& g, const Family<T>& fam, Acc (*dsum)[kSepMaxM<true>],
+                                       Acc* sp) {
+  switch (fam.id) {
+    case TQ_FN_EXP_SUM: batch_adj_sep<T, TQ_FN_EXP_SUM>(a, d, tile, g, fam, dsum, sp); break;
+    case TQ_FN_GAUSSIAN: batch_adj_sep<T, TQ_FN_GAUSSIAN>(a, d, tile, g, fam, dsum, sp); break;
+    case TQ_FN_OSCILLATORY: batch_adj_sep<T, TQ_FN_OSCILLATORY>(a, d, tile, g, fam, dsum, sp); break;
+    default: batch_adj_sep<T, TQ_FN_SUM_SIN>(a, d, tile, g, fam, dsum, sp); break;
+  }
+}
+
 // Gauss integrals and fp64 batches work in fp64 (their table rows as
 // double-floats); fp32 Newton-Cotes integrals in fp32 (the node arithmetic
 // of tq_grid_adjoint).  Up to four dimensions the kernel is held to 128
@@ -604,39 +647,82 @@ __global__ void __launch_bounds__(kBlock, DM <= 4 ? 2 : 1) batch_adjoint_kernel(
   __shared__ tq_batch_desc d;
   __shared__ int64_t tile0;
   constexpr bool kF32 = std::is_same<D, float>::value;
-  for (int64_t tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x) {
-    if (threadIdx.x < 32) {
-      const int64_t i = warp_find_start(a.tile_start, a.n_int, tile);
-      if (threadIdx.x == 0) {
-        d = a.desc[i];
-        tile0 = a.tile_start[i];
-      }
-      __syncwarp();
-      const int fid = a.family >= 0 ? a.family : d.family;
-      const D* dom = (const D*)a.domains + d.dom_off;
-      if (kF32 && d.rule != TQ_RULE_GAUSS) {
-        geo_setup<float, D>(g32, d.rule, d.dim, d.n, dom);
-        load_family<float>(fam32, fid, d.dim, a.params + d.par_off);
-      } else {
-        geo_setup<double, D>(g64, d.rule, d.dim, d.n, dom);
-        load_family<double>(fam64, fid, d.dim, a.params + d.par_off);
-      }
-      if (threadIdx.x == 0) {
-        uint64_t st = 1;
-        for (int k = d.dim - 2; k >= 0; --k) {
-          rstride[k] = st;
-          st *= (uint64_t)d.n;
+  __shared__ int64_t ti[kBlock / 32], ts[kBlock / 32], te[kBlock / 32];
+  __shared__ int tsep[kBlock / 32];
+  __shared__ Acc dsum[kMaxDim][kSepMaxM<true>];
+  __shared__ Acc sp[kSepSlots<true>];
+  const int warp = threadIdx.x >> 5;
+  // Rounds of one tile per warp, as in batch_grid_kernel: the warps look
+  // their tiles' integrals up in parallel; an integral in factored form is
+  // done whole at its first tile, the rows of its other tiles are zeros.
+  for (int64_t base = blockIdx.x; base < a.n_tiles; base += (int64_t)(kBlock / 32) * gridDim.x) {
+    {
+      const int64_t tile = base + (int64_t)warp * gridDim.x;
+      if (tile < a.n_tiles) {
+        const int64_t i = warp_find_start(a.tile_start, a.n_int, tile);
+        const tq_batch_desc& di = a.desc[i];
+        const int fid = a.family >= 0 ? a.family : di.family;
+        const D* dom = (const D*)a.domains + di.dom_off;
+        const double* par = a.params + di.par_off;
+        // one dimension in several tiles: the tiles' nodes spread over CTAs
+        const bool sep = (di.dim > 1 || di.n <= a.tile_pts) &&
+                         (kF32 && di.rule != TQ_RULE_GAUSS ? sep_ok<float, D>(fid, di.dim, di.n, dom, par)
+                                                           : sep_ok<double, D>(fid, di.dim, di.n, dom, par));
+        if ((threadIdx.x & 31) == 0) {
+          ti[warp] = i;
+          ts[warp] = a.tile_start[i];
+          te[warp] = a.tile_start[i + 1];
+          tsep[warp] = sep;
         }
       }
     }
     __syncthreads();
-    if (d.rule == TQ_RULE_GAUSS)
-      batch_adj_dispatch<double, D, true, DM>(a, d, tile, tile0, g64, fam64, rstride, &tab, sh);
-    else if (kF32)
-      batch_adj_dispatch<float, D, false, DM>(a, d, tile, tile0, g32, fam32, rstride, &tab, sh);
-    else
-      batch_adj_dispatch<double, D, false, DM>(a, d, tile, tile0, g64, fam64, rstride, &tab, sh);
-    __syncthreads();
+    for (int r = 0; r < kBlock / 32; ++r) {
+      const int64_t tile = base + (int64_t)r * gridDim.x;
+      if (tile >= a.n_tiles) break;
+      const bool sep = tsep[r] != 0;
+      if (sep && tile != ts[r]) continue;
+      if (threadIdx.x < 32) {
+        if (threadIdx.x == 0) {
+          d = a.desc[ti[r]];
+          tile0 = ts[r];
+        }
+        __syncwarp();
+        const int fid = a.family >= 0 ? a.family : d.family;
+        const D* dom = (const D*)a.domains + d.dom_off;
+        if (kF32 && d.rule != TQ_RULE_GAUSS) {
+          geo_setup<float, D>(g32, d.rule, d.dim, d.n, dom);
+          load_family<float>(fam32, fid, d.dim, a.params + d.par_off);
+        } else {
+          geo_setup<double, D>(g64, d.rule, d.dim, d.n, dom);
+          load_family<double>(fam64, fid, d.dim, a.params + d.par_off);
+        }
+        if (threadIdx.x == 0) {
+          uint64_t st = 1;
+          for (int k = d.dim - 2; k >= 0; --k) {
+            rstride[k] = st;
+            st *= (uint64_t)d.n;
+          }
+        }
+      }
+      __syncthreads();
+      if (sep) {
+        if (kF32 && d.rule != TQ_RULE_GAUSS)
+          batch_adj_sep_dispatch<float>(a, d, tile, g32, fam32, dsum, sp);
+        else
+          batch_adj_sep_dispatch<double>(a, d, tile, g64, fam64, dsum, sp);
+        const int64_t cells = (te[r] - tile - 1) * a.stride;
+        for (int64_t e = threadIdx.x; e < cells; e += blockDim.x) a.partials[(tile + 1) * a.stride + e] = 0.0;
+      } else if (d.rule == TQ_RULE_GAUSS) {
+        batch_adj_dispatch<double, D, true, DM>(a, d, tile, tile0, g64, fam64, rstride, &tab, sh);
+      } else if (kF32) {
+        batch_adj_dispatch<float, D, false, DM>(a, d, tile, tile0, g32, fam32, rstride, &tab, sh);
+      } else {
+        batch_adj_dispatch<double, D, false, DM>(a, d, tile, tile0, g64, fam64, rstride, &tab, sh);
+      }
+      __syncthreads();
+    }
+    __syncthreads();  // the round's tables are rewritten
   }
 }
 
@@ -659,11 +745,9 @@ __global__ void batch_adjoint_finalize_kernel(BatchGradArgs a, double* out_value
     if (lane == 0) tot[wib][i] = s.s + s.c;
   }
   __syncwarp();
-  if (lane == 0) {
-    const int fid = a.family >= 0 ? a.family : d.family;
-    adj_outputs<D>(tot[wib], fid, a.params[d.par_off], (const D*)a.domains + d.dom_off, d.dim, out_value + w,
-                   out_gdom + d.dom_off, out_gpar + d.par_off);
-  }
+  const int fid = a.family >= 0 ? a.family : d.family;
+  adj_outputs<D>(tot[wib], fid, a.params[d.par_off], (const D*)a.domains + d.dom_off, d.dim, out_value + w,
+                 out_gdom + d.dom_off, out_gpar + d.par_off);
 }
 
 }  // namespace tq
@@ -683,8 +767,16 @@ static bool valid_nc(int rule, int64_t n) {
   return true;
 }
 
+static size_t adj_ws_least(int dim, int64_t blocks) {  // the node-by-node path's partials
+  return 256 + (size_t)blocks * (2 + 4 * (size_t)(dim > 0 ? dim : 1)) * 8;
+}
+
 extern "C" size_t tq_grid_adjoint_workspace_size(int dim, int64_t total_points) {
-  return 256 + (size_t)adj_blocks(total_points) * (2 + 4 * (size_t)(dim > 0 ? dim : 1)) * 8;
+  // room for every unit of the factored form too (a smaller workspace that
+  // holds the node-by-node partials is accepted: one CTA then sums all units)
+  const size_t sep = 256 + (size_t)(dim > 0 ? dim : 1) * 32 * kSepMaxM<true> * sizeof(Acc);
+  const size_t least = adj_ws_least(dim, adj_blocks(total_points));
+  return least > sep ? least : sep;
 }
 
 extern "C" int tq_grid_adjoint(int dtype, int rule, int dim, int64_t n_per_dim, const void* domain,
@@ -703,7 +795,11 @@ extern "C" int tq_grid_adjoint(int dtype, int rule, int dim, int64_t n_per_dim, 
     if (total > (int64_t(1) << 62) / n_per_dim) return TQ_ERR_TOO_LARGE;
     total *= n_per_dim;
   }
-  if (workspace_bytes < tq_grid_adjoint_workspace_size(dim, total)) return TQ_ERR_WORKSPACE;
+  int64_t blocks = adj_blocks(total);
+  if (workspace_bytes < adj_ws_least(dim, blocks)) return TQ_ERR_WORKSPACE;
+  // a small grid whose 1-D sums can use more CTAs than its nodes need
+  const int64_t sb = sep_ctas(dim, n_per_dim);
+  if (blocks < sb && (dim > 1 || n_per_dim <= kSepRow) && workspace_bytes >= adj_ws_least(dim, sb)) blocks = sb;
   GradArgs a;
   a.rule = rule;
   a.dim = dim;
@@ -716,10 +812,11 @@ extern "C" int tq_grid_adjoint(int dtype, int rule, int dim, int64_t n_per_dim, 
   a.params = params;
   a.ticket = (unsigned*)workspace;
   a.partials = (double*)((char*)workspace + 256);
+  a.slots = (int64_t)((workspace_bytes - 256) / sizeof(Acc));
   a.out_value = out_value;
   a.out_gdom = out_grad_domain;
   a.out_gpar = out_grad_params;
-  const dim3 grid((unsigned)adj_blocks(total));
+  const dim3 grid((unsigned)blocks);
   cudaStream_t s = (cudaStream_t)stream;
 #define TQ_ADJ(DMV)                                                                      \
   if (rule == TQ_RULE_GAUSS) {                                                           \

@@ -14,7 +14,7 @@
 
 #include <type_traits>
 
-#include "tq_grid_common.cuh"
+#include "tq_separable.cuh"
 
 namespace tq {
 
@@ -27,6 +27,7 @@ struct FusedArgs {
   const double* gl_weights;
   const double* params;
   Acc* partials;
+  int64_t slots;  // partials the workspace holds
   unsigned* ticket;
   void* out;
   int out_dtype;
@@ -104,8 +105,24 @@ __global__ void __launch_bounds__(kBlock, 2) grid_fused_kernel(FusedArgs args) {
   __shared__ Geo<T> g;
   __shared__ Family<T> fam;
   __shared__ uint64_t rstride[kMaxDim];
+  // the factored form, by the first few CTAs; the others have nothing to do
+  const bool sep = (args.dim > 1 || args.n <= kSepRow) &&
+                   sep_ok<T, D>(FAM, args.dim, args.n, (const D*)args.domain, args.params);
+  if (sep && blockIdx.x >= (unsigned)sep_ctas(args.dim, args.n)) return;
   geo_setup<T, D>(g, RULE, args.dim, args.n, (const D*)args.domain);
   load_family<T>(fam, args.family, args.dim, args.params);
+  if (sep) {
+    __shared__ Acc dsum[kMaxDim][kSepMaxM<false>];
+    __shared__ Acc sp[kSepSlots<false>];
+    __syncthreads();
+    if (sep_sums<T, FAM, false>(g, fam, RULE, args.dim, args.n, args.gl_nodes, args.gl_weights, blockIdx.x,
+                                gridDim.x, args.partials, args.slots, args.ticket, dsum, sp) &&
+        threadIdx.x < 32) {
+      const Acc v = dd_mul(sep_value<FAM>(dsum, args.dim), (double)fam.c);
+      if (threadIdx.x == 0) write_result(args.out, args.out_dtype, args.out64, v.s + v.c);
+    }
+    return;
+  }
   if (threadIdx.x == 0) {
     uint64_t st = 1;
     for (int k = args.dim - 2; k >= 0; --k) {
@@ -937,8 +954,11 @@ extern "C" int tq_grid_fused(int dtype, int rule, int dim, int64_t n_per_dim, co
   if (!grid_total(dim, n_per_dim, &total)) return TQ_ERR_TOO_LARGE;
   const bool gl = rule == TQ_RULE_GAUSS;
   const bool f64 = gl || dtype == TQ_F64;
-  const int64_t blocks = fused_blocks(total, f64 ? kStripD : kStripF);
+  int64_t blocks = fused_blocks(total, f64 ? kStripD : kStripF);
   if (workspace_bytes < reduce_ws_bytes(blocks)) return TQ_ERR_WORKSPACE;
+  // a small grid whose 1-D sums can use more CTAs than its nodes need
+  const int64_t sb = sep_ctas(dim, n_per_dim);
+  if (blocks < sb && (dim > 1 || n_per_dim <= kSepRow) && workspace_bytes >= reduce_ws_bytes(sb)) blocks = sb;
   FusedArgs a;
   a.rule = rule;
   a.dim = dim;
@@ -951,28 +971,23 @@ extern "C" int tq_grid_fused(int dtype, int rule, int dim, int64_t n_per_dim, co
   a.params = params;
   a.ticket = (unsigned*)workspace;
   a.partials = (Acc*)((char*)workspace + 256);
+  a.slots = (int64_t)((workspace_bytes - 256) / sizeof(Acc));
   a.out = out;
   a.out_dtype = out_dtype;
   a.out64 = out64;
   cudaStream_t s = (cudaStream_t)stream;
   const dim3 grid((unsigned)blocks);
 #define TQ_FUSED_RULE(RULEC)                                                              \
-  if (gl) {                                                                                \
-    if (dtype == TQ_F64)                                                                   \
-      grid_fused_kernel<double, double, RULEC, FAM, kStripD><<<grid, kBlock, 0, s>>>(a);   \
-    else                                                                                   \
-      grid_fused_kernel<double, float, RULEC, FAM, kStripD><<<grid, kBlock, 0, s>>>(a);    \
-  } else if (dtype == TQ_F64) {                                                            \
+  if (dtype == TQ_F64)                                                                     \
     grid_fused_kernel<double, double, RULEC, FAM, kStripD><<<grid, kBlock, 0, s>>>(a);     \
-  } else {                                                                                 \
-    grid_fused_kernel<float, float, RULEC, FAM, kStripF><<<grid, kBlock, 0, s>>>(a);       \
-  }
+  else                                                                                     \
+    grid_fused_kernel<float, float, RULEC, FAM, kStripF><<<grid, kBlock, 0, s>>>(a);
   TQ_DISPATCH_FAMILY(family, FAM, {
     switch (rule) {
       case TQ_RULE_TRAPEZOID: { TQ_FUSED_RULE(TQ_RULE_TRAPEZOID) } break;
       case TQ_RULE_SIMPSON: { TQ_FUSED_RULE(TQ_RULE_SIMPSON) } break;
       case TQ_RULE_BOOLE: { TQ_FUSED_RULE(TQ_RULE_BOOLE) } break;
-      default: {
+      default: {  // Gauss: fp64 nodes on the domain of either type
         if (dtype == TQ_F64)
           grid_fused_kernel<double, double, TQ_RULE_GAUSS, FAM, kStripD><<<grid, kBlock, 0, s>>>(a);
         else

@@ -1,0 +1,338 @@
+// Sum factorisation of the built-in families on tensor-product grids.
+//
+// A built-in integrand is a function of a separable sum, so its tensor-
+// product rule factors into 1-D sums over each dimension's nodes, with the
+// same nodes and weights (Orszag's sum factorisation):
+//   ExpSum   c prod_k sum_j w_kj exp(a_k x_kj)          (b joins dimension 0)
+//   Gaussian c prod_k sum_j w_kj exp(-a_k (x_kj - u_k)^2)
+//   Oscill.  c Re prod_k sum_j w_kj exp(i a_k x_kj)     (2 pi b joins dimension 0)
+//   SumSin   c sum_k (sum_j w_kj sin(a_k x_kj)) prod_{m != k} (sum_j w_mj)
+// and the sums of its adjoint factor likewise with a few more moments per
+// dimension.  That is dim * n terms instead of n^dim.  Terms are evaluated
+// in fp64 (from the working type's nodes and parameters), weighted exactly,
+// summed exactly (fixed-point warp sums) and multiplied as unevaluated
+// hi + lo pairs, so the result carries little more than its last rounding.
+//
+// It holds only where the factors stay inside the floating range although
+// the product does: sep_ok decides that from the bounds and the parameters
+// alone, equally in every warp; other integrals take the node-by-node path.
+#pragma once
+
+#include "tq_grid_common.cuh"
+
+namespace tq {
+
+// Largest one-dimensional grid the per-call kernels sum this way: up to four
+// terms a lane of 32 warps (1001 nodes fp64: SEP_1D_A us, strips SEP_1D_B us);
+// longer rows go to the strips, whose terms come by recurrence (fp64) or in
+// fp32, over the whole chip.
+constexpr int64_t kSepRow = 4096;
+
+template <int FAM, bool GRAD>
+struct SepM {  // 1-D moments per dimension
+  static constexpr int value = !GRAD ? (FAM == TQ_FN_EXP_SUM || FAM == TQ_FN_GAUSSIAN ? 1 : 2)
+                               : FAM == TQ_FN_EXP_SUM  ? 3
+                               : FAM == TQ_FN_GAUSSIAN ? 4
+                               : FAM == TQ_FN_OSCILLATORY ? 6
+                                                          : 5;
+};
+template <bool GRAD>
+constexpr int kSepMaxM = GRAD ? 6 : 2;  // the largest of the families
+template <bool GRAD>
+constexpr int kSepSlots = kMaxDim * kSepMaxM<GRAD>;  // partials of one CTA (at most kMaxDim units)
+
+// CTAs the factored form of one integral can use: dim * parts units of one
+// warp, four to a CTA.
+__host__ __device__ inline int sep_parts(int64_t n) { return (int)(n < 32 * 31 ? (n + 31) / 32 : 32); }
+__host__ __device__ inline int sep_ctas(int dim, int64_t n) { return (dim * sep_parts(n) + 3) / 4; }
+
+// Whether the factored form is safe (see above), by a whole warp, lane k on
+// dimension k; the same in every warp that asks.  D: type of the domain,
+// T: type the node-by-node path works in.  Its limits: exponents up to 300
+// (80 in fp32, where e^88 overflows in the node-by-node path), angles up to
+// 10^6, |c| and the weights' product within 2^+-200 (fp32: no node value
+// near overflow), everything finite, no empty dimension.  A Gaussian's
+// largest term in a dimension is at most two mean node gaps beyond the
+// distance of u to the interval.
+template <typename T, typename D>
+__device__ __forceinline__ bool sep_ok(int family, int dim, int64_t n, const D* __restrict__ dom,
+                                       const double* __restrict__ par) {
+  const int k = threadIdx.x & 31;
+  constexpr bool F32 = sizeof(T) == 4;
+  const double c = par[0];
+  const float b = (float)par[1];
+  const int ce = exp_field(c) - 1023;
+  float m = 0.f;  // the dimension's share of the exponent or angle
+  int we = 0;
+  bool ok = true;
+  if (k < dim) {
+    const float lo = (float)dom[2 * k], hi = (float)dom[2 * k + 1], a = (float)par[2 + k];
+    const float wid = fabsf(hi - lo);
+    we = ((int)(__float_as_uint(wid / (float)n) >> 23) & 0xff) - 127;
+    ok = isfinite(lo) && isfinite(hi) && isfinite(a) && wid > 0.f && abs(we) <= 100;
+    const float far = fmaxf(fabsf(lo), fabsf(hi));
+    if (family == TQ_FN_GAUSSIAN) {
+      const float u = (float)par[2 + dim + k];
+      ok = ok && isfinite(u) && a >= 0.f;
+      const float l = fminf(lo, hi), h = fmaxf(lo, hi);
+      const float dist = fmaxf(fmaxf(l - u, u - h), 0.f) + 2.f * wid / (float)n;
+      m = a * dist * dist;
+    } else {
+      m = fabsf(a) * far;
+    }
+  }
+  float sum = m;
+  int wsum = we;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    wsum += __shfl_xor_sync(0xffffffffu, wsum, o);
+  }
+  ok = ok && isfinite(b) && abs(wsum) <= 200;
+  if (family == TQ_FN_EXP_SUM || family == TQ_FN_GAUSSIAN) {
+    if (family == TQ_FN_EXP_SUM) sum += fabsf(b);
+    ok = ok && sum <= (F32 ? 80.f : 300.f);
+    if (F32) ok = ok && abs(ce) <= 120 && (float)ce + (family == TQ_FN_EXP_SUM ? 1.45f * sum : 0.f) <= 120.f;
+  } else {
+    ok = ok && sum + 7.f * fabsf(b) <= 1e6f;
+    if (F32) ok = ok && abs(ce) <= 100;
+  }
+  ok = ok && abs(ce) <= 200;
+  return __all_sync(0xffffffffu, ok);  // false with any NaN
+}
+
+// a + (p + e) for a compensated pair a (Knuth's TwoSum)
+__device__ __forceinline__ void sep_add(Acc& a, double p, double e) {
+  const double t = a.s + p, bb = t - a.s;
+  a.c += ((a.s - (t - bb)) + (p - bb)) + e;
+  a.s = t;
+}
+// products and sums of unevaluated pairs hi + lo
+__device__ __forceinline__ Acc dd_mul(Acc a, Acc b) {
+  const double p = a.s * b.s;
+  double e = fma(a.s, b.s, -p);
+  e = fma(a.s, b.c, e);
+  return Acc{p, fma(a.c, b.s, e)};
+}
+__device__ __forceinline__ Acc dd_mul(Acc a, double b) {
+  const double p = a.s * b;
+  return Acc{p, fma(a.c, b, fma(a.s, b, -p))};
+}
+__device__ __forceinline__ Acc dd_add(Acc a, Acc b) {
+  sep_add(a, b.s, b.c);
+  return a;
+}
+__device__ __forceinline__ Acc dd_neg(Acc a) { return Acc{-a.s, -a.c}; }
+__device__ __forceinline__ Acc dd_shfl_down(Acc a, int o) { return acc_shfl_down(a, o); }
+
+// One warp's share of dimension k: the moments over the nodes [j0, j1).
+// Result valid in lane 0.
+template <typename T, int FAM, bool GRAD>
+__device__ void sep_unit(const Geo<T>& g, const Family<T>& fam, int rule, int64_t n,
+                         const double* __restrict__ gln, const double* __restrict__ glw, int k, int64_t j0,
+                         int64_t j1, Acc* m) {
+  constexpr int M = SepM<FAM, GRAD>::value;
+  const bool gl = rule == TQ_RULE_GAUSS;
+  const double a = (double)fam.a[k], u = (double)fam.u[k];
+  const double phase = k != 0 ? 0.0
+                       : FAM == TQ_FN_EXP_SUM       ? (double)fam.b
+                       : FAM == TQ_FN_OSCILLATORY   ? (double)((T)(2.0 * CUDART_PI) * fam.b)
+                                                    : 0.0;
+#pragma unroll
+  for (int i = 0; i < M; ++i) m[i] = Acc{0.0, 0.0};
+  const T ustep = GRAD ? (T)1 / (T)(n - 1) : (T)0;
+  for (int64_t j = j0 + (threadIdx.x & 31); j < j1; j += 32) {
+    const double x = gl ? __dadd_rn(__dmul_rn(g.half[k], __ldg(gln + j)), g.mid[k])
+                        : (double)linspace_node<T>(g.a[k], g.b[k], g.step[k], n, j);
+    const double w = gl ? __ldg(glw + j) : (double)nc_coef_f(rule, (int)j, (int)n);
+    double t = 0.0;  // unit node
+    if (GRAD) t = gl ? (__ldg(gln + j) + 1.0) * 0.5 : (double)linspace_node<T>((T)0, (T)1, ustep, n, j);
+    auto add = [&](int i, double v) {  // w v, exactly
+      const double p = w * v;
+      sep_add(m[i], p, fma(w, v, -p));
+    };
+    if (FAM == TQ_FN_EXP_SUM) {
+      const double e = exp(fma(a, x, phase));
+      add(0, e);
+      if (GRAD) {
+        add(1, e * t);
+        add(2, e * x);
+      }
+    } else if (FAM == TQ_FN_GAUSSIAN) {
+      const double d = x - u;
+      const double e = exp(-(a * (d * d)));
+      add(0, e);
+      if (GRAD) {
+        const double eg = e * (2.0 * a * d);
+        add(1, eg);
+        add(2, eg * t);
+        add(3, e * (d * d));
+      }
+    } else if (FAM == TQ_FN_OSCILLATORY) {
+      double sn, cs;
+      sincos(fma(a, x, phase), &sn, &cs);
+      add(0, cs);
+      add(1, sn);
+      if (GRAD) {
+        add(2, cs * t);
+        add(3, sn * t);
+        add(4, cs * x);
+        add(5, sn * x);
+      }
+    } else {
+      double sn, cs = 0.0;
+      if (GRAD)
+        sincos(a * x, &sn, &cs);
+      else
+        sn = sin(a * x);
+      add(0, 1.0);
+      add(1, sn);
+      if (GRAD) {
+        add(2, a * cs);
+        add(3, a * cs * t);
+        add(4, x * cs);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < M; ++i) m[i] = warp_reduce(m[i]);
+}
+
+// The weighted moments dsum[k][i] (in shared memory) of every dimension.
+// CTA bid of nblk; up to dim * 32 units of at most a few terms per lane are
+// spread over CTAs, four to a CTA: one warp per sub-partition, since the
+// FP64 unit of a sub-partition is the limit.  gpart holds `slots` partials;
+// sp: kSepSlots<GRAD> partials in shared memory.  Returns true (in every thread)
+// in the one CTA that has the sums; the ticket is left at zero.
+template <typename T, int FAM, bool GRAD>
+__device__ bool sep_sums(const Geo<T>& g, const Family<T>& fam, int rule, int dim, int64_t n,
+                         const double* __restrict__ gln, const double* __restrict__ glw, unsigned bid,
+                         unsigned nblk, Acc* gpart, int64_t slots, unsigned* ticket,
+                         Acc (*dsum)[kSepMaxM<GRAD>], Acc* sp) {
+  constexpr int M = SepM<FAM, GRAD>::value;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+  int parts = sep_parts(n);
+  unsigned ctas = min(nblk, (unsigned)sep_ctas(dim, n));
+  if (ctas > 1 && (int64_t)dim * parts * M > slots) ctas = 1;
+  if (ctas == 1) parts = min(parts, max(1, nw / dim));
+  if (bid >= ctas) return false;
+  Acc* dst = ctas > 1 ? gpart : sp;
+  for (int v = (int)bid + warp * (int)ctas; v < dim * parts; v += (int)ctas * nw) {
+    const int k = v / parts, q = v - k * parts;
+    Acc m[M];
+    sep_unit<T, FAM, GRAD>(g, fam, rule, n, gln, glw, k, n * q / parts, n * (q + 1) / parts, m);
+    if (lane == 0) {
+#pragma unroll
+      for (int i = 0; i < M; ++i) dst[v * M + i] = m[i];
+    }
+  }
+  if (ctas > 1) {
+    if (!last_block_of(ticket, ctas)) return false;
+    if (threadIdx.x == 0) *ticket = 0u;
+  } else {
+    __syncthreads();
+  }
+  for (int q = warp; q < dim * M; q += nw) {
+    const int k = q / M, i = q - k * M;
+    Acc v{0.0, 0.0};
+    if (lane < parts) {
+      const double* e = &dst[(k * parts + lane) * M + i].s;
+      v = ctas > 1 ? Acc{__ldcg(e), __ldcg(e + 1)} : Acc{e[0], e[1]};
+    }
+    if (parts > 1) v = warp_reduce(v);
+    if (lane == 0) dsum[k][i] = dd_mul(v, g.wscale[k]);
+  }
+  __syncthreads();
+  return true;
+}
+
+// The integral without c from the dimensions' moments, by one warp (products
+// in a tree over the dimensions); valid in lane 0.
+template <int FAM>
+__device__ Acc sep_value(const Acc (*dsum)[kSepMaxM<false>], int dim) {
+  const int k = threadIdx.x & 31;
+  Acc p = k < dim ? dsum[k][0] : Acc{1.0, 0.0};
+  Acc q = (k < dim && (FAM == TQ_FN_OSCILLATORY || FAM == TQ_FN_SUM_SIN)) ? dsum[k][1] : Acc{0.0, 0.0};
+  for (int o = 8; o > 0; o >>= 1) {
+    if (o >= dim) continue;
+    const Acc p2 = dd_shfl_down(p, o);
+    if (FAM == TQ_FN_OSCILLATORY) {  // (p + i q) (p2 + i q2)
+      const Acc q2 = dd_shfl_down(q, o);
+      const Acc re = dd_add(dd_mul(p, p2), dd_neg(dd_mul(q, q2)));
+      q = dd_add(dd_mul(p, q2), dd_mul(q, p2));
+      p = re;
+    } else if (FAM == TQ_FN_SUM_SIN) {  // p: product of the weights, q: the sum
+      const Acc q2 = dd_shfl_down(q, o);
+      q = dd_add(dd_mul(q, p2), dd_mul(p, q2));
+      p = dd_mul(p, p2);
+    } else {
+      p = dd_mul(p, p2);
+    }
+  }
+  return FAM == TQ_FN_SUM_SIN ? q : p;
+}
+
+// The adjoint's accumulators out[0 .. 2 + 4 dim) (sum W F, sum W F', then by
+// dimension sum W F' g', W F' g' t, W F' dg/da, W F' dg/du; no factor c)
+// from the dimensions' moments, by one warp.
+template <int FAM, typename T>
+__device__ void sep_adjoint(const Acc (*dsum)[kSepMaxM<true>], const T* av, int dim, double* out) {
+  const int k = threadIdx.x & 31;
+  auto val = [](Acc v) { return v.s + v.c; };
+  if (k < dim) {
+    // product over the other dimensions (lane k), complex for oscillations
+    Acc pr{1.0, 0.0}, pi{0.0, 0.0};
+    Acc so{0.0, 0.0};  // sum of sines: sum over the others of S_m prod W
+    for (int m = 0; m < dim; ++m) {
+      if (m == k) continue;
+      if (FAM == TQ_FN_OSCILLATORY) {
+        const Acc zr = dsum[m][0], zi = dsum[m][1];
+        const Acc re = dd_add(dd_mul(pr, zr), dd_neg(dd_mul(pi, zi)));
+        pi = dd_add(dd_mul(pr, zi), dd_mul(pi, zr));
+        pr = re;
+      } else {
+        if (FAM == TQ_FN_SUM_SIN) so = dd_add(dd_mul(so, dsum[m][0]), dd_mul(pr, dsum[m][1]));
+        pr = dd_mul(pr, dsum[m][0]);
+      }
+    }
+    // imaginary part of (pr + i pi)(moment r + i moment i), negated
+    auto nim = [&](int r, int i) { return -val(dd_add(dd_mul(pr, dsum[k][i]), dd_mul(pi, dsum[k][r]))); };
+    const double a = (double)av[k];
+    double F, Fp, sx, st, pa, pu = 0.0;
+    if (FAM == TQ_FN_OSCILLATORY) {
+      F = val(dd_add(dd_mul(pr, dsum[k][0]), dd_neg(dd_mul(pi, dsum[k][1]))));
+      Fp = nim(0, 1);
+      sx = a * Fp;
+      st = a * nim(2, 3);
+      pa = nim(4, 5);
+    } else if (FAM == TQ_FN_EXP_SUM) {
+      F = Fp = val(dd_mul(pr, dsum[k][0]));
+      sx = a * F;
+      st = a * val(dd_mul(pr, dsum[k][1]));
+      pa = val(dd_mul(pr, dsum[k][2]));
+    } else if (FAM == TQ_FN_GAUSSIAN) {
+      F = val(dd_mul(pr, dsum[k][0]));
+      Fp = -F;
+      sx = -val(dd_mul(pr, dsum[k][1]));
+      st = -val(dd_mul(pr, dsum[k][2]));
+      pa = -val(dd_mul(pr, dsum[k][3]));
+      pu = -sx;
+    } else {
+      F = val(dd_add(dd_mul(so, dsum[k][0]), dd_mul(pr, dsum[k][1])));
+      Fp = val(dd_mul(pr, dsum[k][0]));
+      sx = val(dd_mul(pr, dsum[k][2]));
+      st = val(dd_mul(pr, dsum[k][3]));
+      pa = val(dd_mul(pr, dsum[k][4]));
+    }
+    if (k == 0) {
+      out[0] = F;
+      out[1] = Fp;
+    }
+    out[2 + k] = sx;
+    out[2 + dim + k] = st;
+    out[2 + 2 * dim + k] = pa;
+    out[2 + 3 * dim + k] = pu;
+  }
+}
+
+}  // namespace tq
