@@ -146,7 +146,7 @@ def test_gradients_match_oracle(fam, dtype, cuda):
 
 
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
-@pytest.mark.parametrize("tile", [64, 4096, 32768])
+@pytest.mark.parametrize("tile", [37, 64, 4096, 32768])
 def test_batch_values_match_oracle(dtype, tile, cuda):
     """Factored and node-by-node integrals of all families and rules in one
     launch, one tile and many an integral, both block sizes."""
@@ -156,8 +156,8 @@ def test_batch_values_match_oracle(dtype, tile, cuda):
     nd = np.float64 if dtype == torch.float64 else np.float32
     for rule in RULES:
         for fam in ("exp", "gauss", "osc", "sumsin"):
-            for dim, n in [(1, 9), (1, 129), (2, 9), (2, 65), (3, 33), (5, 9)]:
-                n = valid_n(rule, n)
+            for dim, n in [(1, 9), (1, 129), (1, 4093), (1, 40_001), (2, 9), (2, 65), (3, 33), (5, 9)]:
+                n = valid_n(rule, min(n, 200) if rule == "gausslegendre" else n)
                 fs.append(family(fam, dim))
                 rules.append(rule)
                 Ns.append(n ** dim)

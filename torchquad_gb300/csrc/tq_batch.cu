@@ -48,7 +48,7 @@ struct BatchArgs {
 template <typename T, int FAM, int P>
 __device__ Acc grid_tile_sum(const BatchArgs& a, const BatchDesc& d, int64_t tile, int64_t tile0,
                              const Geo<T>& g, const Family<T>& fam, const uint64_t* rstride,
-                             InnerTab* tab, RowTab* rt, FastDiv* fdn, const F2* wsf) {
+                             InnerTab* tab, RowTab* rt, ChainTab* ct, FastDiv* fdn, const F2* wsf) {
   const int dim = d.dim, rule = d.rule, last = dim - 1;
   const int64_t n = d.n;
   const int n32 = (int)n;
@@ -60,6 +60,18 @@ __device__ Acc grid_tile_sum(const BatchArgs& a, const BatchDesc& d, int64_t til
   const double wlast = g.wscale[last];
   const T a_l = g.a[last], b_l = g.b[last], st_l = g.step[last];
   const int half = n32 / 2;
+  if constexpr (std::is_same<T, double>::value) {
+    if (dim == 1 && !gl) {
+      // chains of as many nodes as the tile has for each thread
+      const int len = (int)min((int64_t)kChain, max((int64_t)kBlk, (a.tile_pts / blockDim.x) / kBlk * kBlk));
+      chain_table<FAM>(*ct, fam, rule, st_l, begin);
+      __syncthreads();
+      Acc v = chain_rows<FAM>(g, fam, *ct, rule, n, begin, end, len, threadIdx.x, blockDim.x);
+      v.s *= wlast;
+      v.c *= wlast;
+      return block_reduce<256>(v);
+    }
+  }
   // fp64: last-dimension tables of this tile's integral (one
   // outer-function evaluation per row)
   bool use_tab = false;
@@ -75,8 +87,7 @@ __device__ Acc grid_tile_sum(const BatchArgs& a, const BatchDesc& d, int64_t til
       acc = tab_rows_sum<FAM>(g, fam, *tab, *rt, dim, rule, gl, n, *fdn, gln, glw, begin, end);
       return block_reduce<256>(acc);
     }
-    // rows without a table (one dimension, or longer than a table): equally
-    // spaced nodes by recurrence along the row
+    // rows longer than a table: equally spaced nodes by recurrence along the row
     if (!gl) rc = recur_const<FAM>(fam, last, st_l);
   }
   // node indices of an integral below 2^32: 32-bit divisions
@@ -242,85 +253,99 @@ __global__ void __launch_bounds__(256) batch_grid_kernel(BatchArgs a) {
   __shared__ int64_t tile0;
   InnerTab* tab = nullptr;
   RowTab* rt = nullptr;
+  ChainTab* ct = nullptr;
   __shared__ FastDiv fdn;
   __shared__ F2 wsf[kMaxDim];  // fp32: the dimensions' weight scales as double-floats
   if constexpr (std::is_same<T, double>::value) {
     __shared__ InnerTab tab_s;
     __shared__ RowTab rt_s;
+    __shared__ ChainTab ct_s;
     tab = &tab_s;
     rt = &rt_s;
+    ct = &ct_s;
   }
   __shared__ int64_t ti[8], ts[8], te[8];  // a round's integrals and their tile ranges
   __shared__ int tsep[8];
   __shared__ Acc dsum[kMaxDim][kSepMaxM<false>];
   __shared__ Acc sp[kSepSlots<false>];
   const int nw = (int)(blockDim.x >> 5), warp = threadIdx.x >> 5;
-  // Rounds of one tile per warp: the warps look their tiles' integrals up and
-  // decide on the factored form in parallel (dependent loads), then the CTA
-  // does the tiles.  An integral in factored form is done whole at its first
-  // tile; its other tiles are zeros and cost the look-up only.
-  for (int64_t base = blockIdx.x; base < a.n_tiles; base += (int64_t)nw * gridDim.x) {
-    {
-      const int64_t tile = base + (int64_t)warp * gridDim.x;
-      if (tile < a.n_tiles) {
-        const int64_t i = warp_find_start(a.tile_start, a.n_int, tile);
-        const BatchDesc& di = a.desc[i];
-        // one dimension: the rows' recurrences take fewer FP64 operations a node
-        const bool sep = (di.dim > 1 || di.rule == TQ_RULE_GAUSS) &&
-                         sep_ok<T, T>(a.family >= 0 ? a.family : di.family, di.dim, di.n,
-                                      (const T*)a.domains + di.dom_off, a.params + di.par_off);
-        if ((threadIdx.x & 31) == 0) {
-          ti[warp] = i;
-          ts[warp] = a.tile_start[i];
-          te[warp] = a.tile_start[i + 1];
-          tsep[warp] = sep;
+  // Integrals in factored form, one per CTA and turn: the whole value at its
+  // first tile, zeros at the others.  Then the tiles of the rest.  The warps
+  // look a round of integrals or tiles up in parallel (dependent loads),
+  // before the CTA does them.
+  auto lookup = [&](int64_t i) {  // by a whole warp
+    const BatchDesc& di = a.desc[i];
+    // one dimension: a chain takes fewer FP64 operations a node
+    const bool sep = (di.dim > 1 || di.rule == TQ_RULE_GAUSS) &&
+                     sep_ok<T, T>(a.family >= 0 ? a.family : di.family, di.dim, di.n,
+                                  (const T*)a.domains + di.dom_off, a.params + di.par_off);
+    if ((threadIdx.x & 31) == 0) {
+      ti[warp] = i;
+      ts[warp] = a.tile_start[i];
+      te[warp] = a.tile_start[i + 1];
+      tsep[warp] = sep;
+    }
+  };
+  auto setup = [&](int r) {  // the r-th looked up; ends with a barrier
+    if (threadIdx.x < 32) {
+      if (threadIdx.x == 0) {
+        d = a.desc[ti[r]];
+        tile0 = ts[r];
+      }
+      __syncwarp();
+      geo_setup<T, T>(g, d.rule, d.dim, d.n, (const T*)a.domains + d.dom_off);
+      load_family<T>(fam, a.family >= 0 ? a.family : d.family, d.dim, a.params + d.par_off);
+      if constexpr (std::is_same<T, float>::value)
+        if (threadIdx.x < d.dim) wsf[threadIdx.x] = f2_from_double(g.wscale[threadIdx.x]);
+      if (threadIdx.x == 0) {
+        uint64_t st = 1;
+        for (int k = d.dim - 2; k >= 0; --k) {
+          rstride[k] = st;
+          st *= (uint64_t)d.n;
         }
       }
     }
     __syncthreads();
-    for (int r = 0; r < nw; ++r) {
-      const int64_t tile = base + (int64_t)r * gridDim.x;
-      if (tile >= a.n_tiles) break;
-      const bool sep = tsep[r] != 0;
-      if (sep && tile != ts[r]) continue;
-      if (threadIdx.x < 32) {
-        if (threadIdx.x == 0) {
-          d = a.desc[ti[r]];
-          tile0 = ts[r];
-        }
-        __syncwarp();
-        geo_setup<T, T>(g, d.rule, d.dim, d.n, (const T*)a.domains + d.dom_off);
-        load_family<T>(fam, a.family >= 0 ? a.family : d.family, d.dim, a.params + d.par_off);
-        if constexpr (std::is_same<T, float>::value)
-          if (threadIdx.x < d.dim) wsf[threadIdx.x] = f2_from_double(g.wscale[threadIdx.x]);
-        if (threadIdx.x == 0) {
-          uint64_t st = 1;
-          for (int k = d.dim - 2; k >= 0; --k) {
-            rstride[k] = st;
-            st *= (uint64_t)d.n;
-          }
-        }
-      }
-      __syncthreads();
+  };
+#define TQ_BATCH_FAMILY(CALL)                                             \
+  switch (fam.id) {                                                       \
+    case TQ_FN_EXP_SUM: { constexpr int FAMC = TQ_FN_EXP_SUM; CALL; } break;       \
+    case TQ_FN_GAUSSIAN: { constexpr int FAMC = TQ_FN_GAUSSIAN; CALL; } break;     \
+    case TQ_FN_OSCILLATORY: { constexpr int FAMC = TQ_FN_OSCILLATORY; CALL; } break; \
+    case TQ_FN_SUM_SIN: { constexpr int FAMC = TQ_FN_SUM_SIN; CALL; } break;       \
+    default: break;                                                       \
+  }
+  for (int64_t base = blockIdx.x; base < a.n_int; base += (int64_t)nw * gridDim.x) {
+    const int64_t mine = base + (int64_t)warp * gridDim.x;
+    if (mine < a.n_int) lookup(mine);
+    __syncthreads();
+    for (int r = 0; r < nw && base + (int64_t)r * gridDim.x < a.n_int; ++r) {
+      if (!tsep[r]) continue;
+      setup(r);
       Acc acc{CUDART_NAN, 0.0};  // an unknown family (rejected on the host) gives NaN
-#define TQ_BATCH_TILE(FAMC)                                                                              \
-  acc = sep ? sep_integral<T, FAMC>(a, d, g, fam, dsum, sp)                                              \
-            : grid_tile_sum<T, FAMC, P>(a, d, tile, tile0, g, fam, rstride, tab, rt, &fdn, wsf)
-      switch (fam.id) {
-        case TQ_FN_EXP_SUM: TQ_BATCH_TILE(TQ_FN_EXP_SUM); break;
-        case TQ_FN_GAUSSIAN: TQ_BATCH_TILE(TQ_FN_GAUSSIAN); break;
-        case TQ_FN_OSCILLATORY: TQ_BATCH_TILE(TQ_FN_OSCILLATORY); break;
-        case TQ_FN_SUM_SIN: TQ_BATCH_TILE(TQ_FN_SUM_SIN); break;
-        default: break;
-      }
-#undef TQ_BATCH_TILE
-      if (threadIdx.x == 0) a.partials[tile] = acc;
-      if (sep)
-        for (int64_t t = tile + 1 + threadIdx.x; t < te[r]; t += blockDim.x) a.partials[t] = Acc{0.0, 0.0};
+      TQ_BATCH_FAMILY((acc = sep_integral<T, FAMC>(a, d, g, fam, dsum, sp)))
+      for (int64_t t = ts[r] + threadIdx.x; t < te[r]; t += blockDim.x)
+        a.partials[t] = t == ts[r] ? acc : Acc{0.0, 0.0};
       __syncthreads();
     }
     __syncthreads();  // the round's tables are rewritten
   }
+  for (int64_t base = blockIdx.x; base < a.n_tiles; base += (int64_t)nw * gridDim.x) {
+    const int64_t mine = base + (int64_t)warp * gridDim.x;
+    if (mine < a.n_tiles) lookup(warp_find_start(a.tile_start, a.n_int, mine));
+    __syncthreads();
+    for (int r = 0; r < nw && base + (int64_t)r * gridDim.x < a.n_tiles; ++r) {
+      if (tsep[r]) continue;
+      const int64_t tile = base + (int64_t)r * gridDim.x;
+      setup(r);
+      Acc acc{CUDART_NAN, 0.0};
+      TQ_BATCH_FAMILY((acc = grid_tile_sum<T, FAMC, P>(a, d, tile, tile0, g, fam, rstride, tab, rt, ct, &fdn, wsf)))
+      if (threadIdx.x == 0) a.partials[tile] = acc;
+      __syncthreads();
+    }
+    __syncthreads();
+  }
+#undef TQ_BATCH_FAMILY
 }
 
 // One warp per integral: compensated sum of its tiles in tile order.

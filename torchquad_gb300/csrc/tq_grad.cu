@@ -652,77 +652,88 @@ __global__ void __launch_bounds__(kBlock, DM <= 4 ? 2 : 1) batch_adjoint_kernel(
   __shared__ Acc dsum[kMaxDim][kSepMaxM<true>];
   __shared__ Acc sp[kSepSlots<true>];
   const int warp = threadIdx.x >> 5;
-  // Rounds of one tile per warp, as in batch_grid_kernel: the warps look
-  // their tiles' integrals up in parallel; an integral in factored form is
-  // done whole at its first tile, the rows of its other tiles are zeros.
-  for (int64_t base = blockIdx.x; base < a.n_tiles; base += (int64_t)(kBlock / 32) * gridDim.x) {
-    {
-      const int64_t tile = base + (int64_t)warp * gridDim.x;
-      if (tile < a.n_tiles) {
-        const int64_t i = warp_find_start(a.tile_start, a.n_int, tile);
-        const tq_batch_desc& di = a.desc[i];
-        const int fid = a.family >= 0 ? a.family : di.family;
-        const D* dom = (const D*)a.domains + di.dom_off;
-        const double* par = a.params + di.par_off;
-        // one dimension in several tiles: the tiles' nodes spread over CTAs
-        const bool sep = (di.dim > 1 || di.n <= a.tile_pts) &&
-                         (kF32 && di.rule != TQ_RULE_GAUSS ? sep_ok<float, D>(fid, di.dim, di.n, dom, par)
-                                                           : sep_ok<double, D>(fid, di.dim, di.n, dom, par));
-        if ((threadIdx.x & 31) == 0) {
-          ti[warp] = i;
-          ts[warp] = a.tile_start[i];
-          te[warp] = a.tile_start[i + 1];
-          tsep[warp] = sep;
+  // As in batch_grid_kernel: first the integrals in factored form, one per
+  // CTA and turn (its sums in the row of its first tile, zeros in the
+  // others), then the tiles of the rest; a round is looked up by the warps
+  // in parallel.
+  auto lookup = [&](int64_t i) {  // by a whole warp
+    const tq_batch_desc& di = a.desc[i];
+    const int fid = a.family >= 0 ? a.family : di.family;
+    const D* dom = (const D*)a.domains + di.dom_off;
+    const double* par = a.params + di.par_off;
+    // one dimension in several tiles: the tiles' nodes spread over CTAs
+    const bool sep = (di.dim > 1 || di.n <= a.tile_pts) &&
+                     (kF32 && di.rule != TQ_RULE_GAUSS ? sep_ok<float, D>(fid, di.dim, di.n, dom, par)
+                                                       : sep_ok<double, D>(fid, di.dim, di.n, dom, par));
+    if ((threadIdx.x & 31) == 0) {
+      ti[warp] = i;
+      ts[warp] = a.tile_start[i];
+      te[warp] = a.tile_start[i + 1];
+      tsep[warp] = sep;
+    }
+  };
+  auto setup = [&](int r) {  // the r-th looked up; ends with a barrier
+    if (threadIdx.x < 32) {
+      if (threadIdx.x == 0) {
+        d = a.desc[ti[r]];
+        tile0 = ts[r];
+      }
+      __syncwarp();
+      const int fid = a.family >= 0 ? a.family : d.family;
+      const D* dom = (const D*)a.domains + d.dom_off;
+      if (kF32 && d.rule != TQ_RULE_GAUSS) {
+        geo_setup<float, D>(g32, d.rule, d.dim, d.n, dom);
+        load_family<float>(fam32, fid, d.dim, a.params + d.par_off);
+      } else {
+        geo_setup<double, D>(g64, d.rule, d.dim, d.n, dom);
+        load_family<double>(fam64, fid, d.dim, a.params + d.par_off);
+      }
+      if (threadIdx.x == 0) {
+        uint64_t st = 1;
+        for (int k = d.dim - 2; k >= 0; --k) {
+          rstride[k] = st;
+          st *= (uint64_t)d.n;
         }
       }
     }
     __syncthreads();
-    for (int r = 0; r < kBlock / 32; ++r) {
-      const int64_t tile = base + (int64_t)r * gridDim.x;
-      if (tile >= a.n_tiles) break;
-      const bool sep = tsep[r] != 0;
-      if (sep && tile != ts[r]) continue;
-      if (threadIdx.x < 32) {
-        if (threadIdx.x == 0) {
-          d = a.desc[ti[r]];
-          tile0 = ts[r];
-        }
-        __syncwarp();
-        const int fid = a.family >= 0 ? a.family : d.family;
-        const D* dom = (const D*)a.domains + d.dom_off;
-        if (kF32 && d.rule != TQ_RULE_GAUSS) {
-          geo_setup<float, D>(g32, d.rule, d.dim, d.n, dom);
-          load_family<float>(fam32, fid, d.dim, a.params + d.par_off);
-        } else {
-          geo_setup<double, D>(g64, d.rule, d.dim, d.n, dom);
-          load_family<double>(fam64, fid, d.dim, a.params + d.par_off);
-        }
-        if (threadIdx.x == 0) {
-          uint64_t st = 1;
-          for (int k = d.dim - 2; k >= 0; --k) {
-            rstride[k] = st;
-            st *= (uint64_t)d.n;
-          }
-        }
-      }
-      __syncthreads();
-      if (sep) {
-        if (kF32 && d.rule != TQ_RULE_GAUSS)
-          batch_adj_sep_dispatch<float>(a, d, tile, g32, fam32, dsum, sp);
-        else
-          batch_adj_sep_dispatch<double>(a, d, tile, g64, fam64, dsum, sp);
-        const int64_t cells = (te[r] - tile - 1) * a.stride;
-        for (int64_t e = threadIdx.x; e < cells; e += blockDim.x) a.partials[(tile + 1) * a.stride + e] = 0.0;
-      } else if (d.rule == TQ_RULE_GAUSS) {
-        batch_adj_dispatch<double, D, true, DM>(a, d, tile, tile0, g64, fam64, rstride, &tab, sh);
-      } else if (kF32) {
-        batch_adj_dispatch<float, D, false, DM>(a, d, tile, tile0, g32, fam32, rstride, &tab, sh);
-      } else {
-        batch_adj_dispatch<double, D, false, DM>(a, d, tile, tile0, g64, fam64, rstride, &tab, sh);
-      }
+  };
+  constexpr int nw = kBlock / 32;
+  for (int64_t base = blockIdx.x; base < a.n_int; base += (int64_t)nw * gridDim.x) {
+    const int64_t mine = base + (int64_t)warp * gridDim.x;
+    if (mine < a.n_int) lookup(mine);
+    __syncthreads();
+    for (int r = 0; r < nw && base + (int64_t)r * gridDim.x < a.n_int; ++r) {
+      if (!tsep[r]) continue;
+      setup(r);
+      const int64_t tile = ts[r];
+      if (kF32 && d.rule != TQ_RULE_GAUSS)
+        batch_adj_sep_dispatch<float>(a, d, tile, g32, fam32, dsum, sp);
+      else
+        batch_adj_sep_dispatch<double>(a, d, tile, g64, fam64, dsum, sp);
+      const int64_t cells = (te[r] - tile - 1) * a.stride;
+      for (int64_t e = threadIdx.x; e < cells; e += blockDim.x) a.partials[(tile + 1) * a.stride + e] = 0.0;
       __syncthreads();
     }
     __syncthreads();  // the round's tables are rewritten
+  }
+  for (int64_t base = blockIdx.x; base < a.n_tiles; base += (int64_t)nw * gridDim.x) {
+    const int64_t mine = base + (int64_t)warp * gridDim.x;
+    if (mine < a.n_tiles) lookup(warp_find_start(a.tile_start, a.n_int, mine));
+    __syncthreads();
+    for (int r = 0; r < nw && base + (int64_t)r * gridDim.x < a.n_tiles; ++r) {
+      if (tsep[r]) continue;
+      const int64_t tile = base + (int64_t)r * gridDim.x;
+      setup(r);
+      if (d.rule == TQ_RULE_GAUSS)
+        batch_adj_dispatch<double, D, true, DM>(a, d, tile, tile0, g64, fam64, rstride, &tab, sh);
+      else if (kF32)
+        batch_adj_dispatch<float, D, false, DM>(a, d, tile, tile0, g32, fam32, rstride, &tab, sh);
+      else
+        batch_adj_dispatch<double, D, false, DM>(a, d, tile, tile0, g64, fam64, rstride, &tab, sh);
+      __syncthreads();
+    }
+    __syncthreads();
   }
 }
 

@@ -28,6 +28,7 @@ struct FusedArgs {
   const double* params;
   Acc* partials;
   int64_t slots;  // partials the workspace holds
+  int sms;        // SMs of the device
   unsigned* ticket;
   void* out;
   int out_dtype;
@@ -164,6 +165,23 @@ __global__ void __launch_bounds__(kBlock, 2) grid_fused_kernel(FusedArgs args) {
       rows_done = true;
     }
   }
+  if constexpr (std::is_same<T, double>::value && !GL) {
+    if (dim == 1) {
+      // chains of a length that gives every sub-partition's FP64 unit one warp
+      // (a chain's start costs as much as 60 of its nodes), warps in turn
+      // over the CTAs
+      __shared__ ChainTab ct;
+      chain_table<FAM>(ct, fam, RULE, st_l, 0);
+      __syncthreads();
+      const int64_t blk = total / (kBlk * (int64_t)args.sms * 128) + 1;
+      const int64_t chain = ((int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+      acc = chain_rows<FAM>(g, fam, ct, RULE, n, 0, total, (int)min((int64_t)kChain, blk * kBlk), chain,
+                            (int64_t)gridDim.x * blockDim.x);
+      acc.s *= wlast;
+      acc.c *= wlast;
+      rows_done = true;
+    }
+  }
   RecurConst rc{1.0, 1.0, 0.0};
   if constexpr (std::is_same<T, double>::value) {
     if (!rows_done && !use_tab && !GL) rc = recur_const<FAM>(fam, last, st_l);
@@ -198,8 +216,7 @@ __global__ void __launch_bounds__(kBlock, 2) grid_fused_kernel(FusedArgs args) {
             tabbed = true;
           }
         } else if (!GL) {
-          // rows without a table (one dimension, or longer than a table):
-          // equally spaced nodes by recurrence along the row
+          // rows longer than a table: equally spaced nodes by recurrence
           double v;
           const double x0 = linspace_node<double>(a_l, b_l, st_l, n, jl);
           const double x1 = linspace_node<double>(a_l, b_l, st_l, n, seg_end - 1);
@@ -972,6 +989,7 @@ extern "C" int tq_grid_fused(int dtype, int rule, int dim, int64_t n_per_dim, co
   a.ticket = (unsigned*)workspace;
   a.partials = (Acc*)((char*)workspace + 256);
   a.slots = (int64_t)((workspace_bytes - 256) / sizeof(Acc));
+  a.sms = sm_count();
   a.out = out;
   a.out_dtype = out_dtype;
   a.out64 = out64;

@@ -23,7 +23,7 @@
 namespace tq {
 
 // Largest one-dimensional grid the per-call kernels sum this way: up to four
-// terms a lane of 32 warps (1001 nodes fp64: SEP_1D_A us, strips SEP_1D_B us);
+// terms a lane of 32 warps (1001 nodes fp64 10.3 us, 14.4 us by the strips);
 // longer rows go to the strips, whose terms come by recurrence (fp64) or in
 // fp32, over the whole chip.
 constexpr int64_t kSepRow = 4096;
@@ -333,6 +333,180 @@ __device__ void sep_adjoint(const Acc (*dsum)[kSepMaxM<true>], const T* av, int 
     out[2 + 2 * dim + k] = pa;
     out[2 + 3 * dim + k] = pu;
   }
+}
+
+// ------------------------------------------------ fp64 rows in one dimension
+// A one-dimensional Newton-Cotes rule of equally spaced nodes, a thread
+// walking a chain of up to kChain nodes in blocks of kBlk from one direct
+// evaluation (two or three exp or one sincos) at the chain's start:
+//   Gaussian  f(x + i h) = F R^i G_i with F = f(x), R = exp(-2 a h (x - u)),
+//             G_i = exp(-a h^2 i^2): a block is F times a polynomial in R
+//             whose coefficients (weight times G_i) are the same for every
+//             block, by Horner's rule; F and R step to the next block by
+//             two factors that are themselves geometric
+//   exp sum   f(x + i h) = f(x) exp(a h i): a block is f(x) times a constant
+//   cosines   by the addition theorem: a block is cos and sin of the first
+//             angle times two constants, the angle rotated block by block.
+// So a node costs about 1.2 (Gaussian) or 0.2-0.4 FP64 operations plus the
+// chain's start, where stepping node by node from strips of 16 took 3 and a
+// start (two exp and the guards, 70 operations) every 16 nodes; the FP64 unit
+// bounds both.  Rounding accumulates over at most kChain / kBlk steps of a
+// factor, fewer than the 16 of the strips.  4096 mixed integrals, a quarter
+// of them such rows: 2.0 ms by strips, 0.63 ms by chains (and the
+// factored integrals spread over the CTAs by integral).
+constexpr int kBlk = 16;    // nodes per block (a multiple of 4: the rules' weight period)
+constexpr int kChain = 128;  // nodes per chain at most
+
+struct ChainTab {
+  double t[kBlk], t2[kBlk];  // weight times G_i, exp(a h i), or cos / sin(a h i)
+  double A, B;               // their sums
+  double q[3];               // Gaussian: G_kBlk, steps of R and of the block factor; exp: exp(a h kBlk);
+                             // cosines: cos and sin of a h kBlk
+};
+
+// Builds the table for chains that start at nodes off + m * kBlk (warp 0 of
+// the CTA; the caller puts a barrier before the first use).
+template <int FAM>
+__device__ void chain_table(ChainTab& tb, const Family<double>& fam, int rule, double h, int64_t off) {
+  const int i = threadIdx.x;
+  if (i >= 32) return;
+  const double a = fam.a[0];
+  const int m = (int)((off + i) & 3);
+  const double w = i >= kBlk ? 1.0
+                   : rule == TQ_RULE_TRAPEZOID ? 2.0
+                   : rule == TQ_RULE_SIMPSON ? ((m & 1) ? 4.0 : 2.0)
+                                             : ((m & 1) ? 32.0 : (m == 2 ? 12.0 : 14.0));
+  double v, v2 = 0.0;
+  if (FAM == TQ_FN_GAUSSIAN) {
+    const int e = i <= kBlk ? i * i : (i == kBlk + 1 ? 2 * kBlk : 2 * kBlk * kBlk);
+    v = w * exp(-(a * h * h) * (double)e);
+  } else if (FAM == TQ_FN_EXP_SUM) {
+    v = w * exp(a * h * (double)min(i, kBlk));
+  } else {
+    double sn, cs;
+    sincos(a * h * (double)min(i, kBlk), &sn, &cs);
+    v = w * cs;
+    v2 = w * sn;
+  }
+  if (i < kBlk) {
+    tb.t[i] = v;
+    tb.t2[i] = v2;
+  } else if (FAM == TQ_FN_GAUSSIAN) {
+    if (i < kBlk + 3) tb.q[i - kBlk] = v;
+  } else if (i == kBlk) {
+    tb.q[0] = v;
+    tb.q[1] = v2;
+  }
+  const Acc A = warp_reduce(Acc{i < kBlk ? v : 0.0, 0.0}), B = warp_reduce(Acc{i < kBlk ? v2 : 0.0, 0.0});
+  if (i == 0) {
+    tb.A = A.s + A.c;
+    tb.B = B.s + B.c;
+  }
+}
+
+// Sum over the nodes j0 .. j0 + cnt - 1 (x0 the first, x1 the last one's
+// coordinate) of the weighted integrand into *out.  Returns false where the
+// factors could leave the range of doubles: the exponent has to stay within
+// [-600, 600] at both ends (that of a Gaussian, a >= 0, is at most 0) and
+// change by at most 300 over a block.  The rules' end weights are half of
+// the interior's at the same place.
+template <int FAM>
+__device__ __forceinline__ bool chain_sum(const Family<double>& fam, const ChainTab& tb, int rule, double x0,
+                                          double x1, double h, int64_t j0, int cnt, int64_t n, double* out) {
+  const double a = fam.a[0];
+  const double half = rule == TQ_RULE_BOOLE ? 7.0 : 1.0;
+  const bool first = j0 == 0, final = j0 + cnt == n;
+  double acc = 0.0;
+  if (FAM == TQ_FN_GAUSSIAN) {
+    const double d0 = x0 - fam.u[0], d1 = x1 - fam.u[0];
+    const double e0 = -(a * (d0 * d0)), e1 = -(a * (d1 * d1)), r0 = -(2.0 * a * h * d0);
+    if (!(a >= 0.0 && e0 >= -600.0 && e1 >= -600.0 && fabs(r0) <= 15.0 &&
+          2.0 * a * h * h * (kBlk * kBlk) <= 200.0 && fabs(2.0 * a * h * d1) <= 15.0))
+      return false;
+    double F = fam.c * exp(e0), R = exp(r0), P = exp(r0 * (double)kBlk) * tb.q[0];
+    if (first) acc = -half * F;
+    int left = cnt;
+    for (; left >= kBlk; left -= kBlk) {
+      double p = tb.t[kBlk - 1];
+#pragma unroll
+      for (int i = kBlk - 2; i >= 0; --i) p = fma(p, R, tb.t[i]);
+      acc = fma(F, p, acc);
+      F *= P;
+      P *= tb.q[2];
+      R *= tb.q[1];
+    }
+    if (left > 0) {
+      double p = tb.t[left - 1];
+      for (int i = left - 2; i >= 0; --i) p = fma(p, R, tb.t[i]);
+      acc = fma(F, p, acc);
+    }
+    if (final) acc = fma(-half * fam.c, exp(e1), acc);
+  } else if (FAM == TQ_FN_EXP_SUM) {
+    const double e0 = fma(a, x0, fam.b), e1 = fma(a, x1, fam.b);
+    if (!(fabs(e0) <= 600.0 && fabs(e1) <= 600.0 && fabs(a * h) <= 15.0)) return false;
+    double f = fam.c * exp(e0);
+    if (first) acc = -half * f;
+    int left = cnt;
+    for (; left >= kBlk; left -= kBlk) {
+      acc = fma(f, tb.A, acc);
+      f *= tb.q[0];
+    }
+    for (int i = 0; i < left; ++i) acc = fma(f, tb.t[i], acc);
+    if (final) acc = fma(-half * fam.c, exp(e1), acc);
+  } else {
+    // f = cos(angle) (oscillatory) or sin(angle) (sum of sines)
+    const double ph = FAM == TQ_FN_OSCILLATORY ? 2.0 * CUDART_PI * fam.b : 0.0;
+    double sn, cs;
+    sincos(fma(a, x0, ph), &sn, &cs);
+    const bool osc = FAM == TQ_FN_OSCILLATORY;
+    if (first) acc = -half * (osc ? cs : sn);
+    int left = cnt;
+    for (; left >= kBlk; left -= kBlk) {
+      acc = osc ? fma(cs, tb.A, fma(-sn, tb.B, acc)) : fma(sn, tb.A, fma(cs, tb.B, acc));
+      const double c2 = fma(cs, tb.q[0], -(sn * tb.q[1]));
+      sn = fma(sn, tb.q[0], cs * tb.q[1]);
+      cs = c2;
+    }
+    for (int i = 0; i < left; ++i)
+      acc = osc ? fma(cs, tb.t[i], fma(-sn, tb.t2[i], acc)) : fma(sn, tb.t[i], fma(cs, tb.t2[i], acc));
+    if (final) acc = fma(-half, osc ? cos(fma(a, x1, ph)) : sin(a * x1), acc);
+    acc *= fam.c;
+  }
+  *out = acc;
+  return true;
+}
+
+// The thread's part of the nodes [begin, end) of a one-dimensional fp64
+// Newton-Cotes grid, without the weight scale: chains of `len` nodes (a
+// multiple of kBlk) from begin + first * len, first + step, ...; nodes of a
+// chain that chain_sum refuses are evaluated one by one.
+template <int FAM>
+__device__ Acc chain_rows(const Geo<double>& g, const Family<double>& fam, const ChainTab& tb, int rule, int64_t n,
+                          int64_t begin, int64_t end, int len, int64_t first, int64_t step) {
+  Acc acc{0.0, 0.0};
+  const double h = g.step[0];
+  for (int64_t j0 = begin + first * len; j0 < end; j0 += step * len) {
+    const int cnt = (int)min((int64_t)len, end - j0);
+    const double x0 = linspace_node<double>(g.a[0], g.b[0], h, n, j0);
+    const double x1 = linspace_node<double>(g.a[0], g.b[0], h, n, j0 + cnt - 1);
+    double v;
+    if (chain_sum<FAM>(fam, tb, rule, x0, x1, h, j0, cnt, n, &v)) {
+      acc_add(acc, v);
+    } else {
+      double sum = 0.0, comp = 0.0;
+      for (int64_t j = j0; j < j0 + cnt; ++j) {
+        const double x = linspace_node<double>(g.a[0], g.b[0], h, n, j);
+        const double f = fam_outer<FAM, double>(fam, fam_term<FAM, double>(fam, 0, x));
+        const double y = (double)nc_int(rule, j, n) * f - comp;
+        const double t = sum + y;
+        comp = (t - sum) - y;
+        sum = t;
+      }
+      acc_add(acc, sum);
+      acc_add(acc, -comp);
+    }
+  }
+  return acc;
 }
 
 }  // namespace tq
