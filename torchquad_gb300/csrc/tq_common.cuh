@@ -74,7 +74,7 @@ __device__ __forceinline__ Acc acc_shfl_down(const Acc& a, int off) {
 // redux.sync and over the CTA as 64-bit integers, and one thread turns the
 // total into hi + lo doubles by bit moves.  Integer sums are exact and do
 // not depend on their order; a value loses only bits below 2^-95 of the
-// largest.  A 101^3 fused Simpson launch (252 CTAs): 25.5 us with the fp64
+// largest.  A 101^3 fused Simpson launch (252 CTAs): 26.4 us with the fp64
 // trees, 18.7 us with these sums and the
 // dimensions set up in parallel; a 10001-node rule over 200 components (50
 // reductions a component group): 969 and 431 us.
@@ -133,38 +133,65 @@ __device__ __forceinline__ Acc fix_value(const int64_t (&S)[4], int emax) {
   return r;
 }
 
-// Sum of one Acc per lane over a warp; result valid in lane 0.
-__device__ __forceinline__ Acc warp_reduce(Acc a) {
-  const int emax = max(1, __reduce_max_sync(0xffffffffu, max(exp_field(a.s), exp_field(a.c))));
+// Sum of get(0) .. get(n - 1) by a whole warp (get is called twice for each);
+// result valid in lane 0.
+template <typename Get>
+__device__ __forceinline__ Acc warp_sum(int n, Get get) {
+  const int lane = threadIdx.x & 31;
+  int e = 1;
+  for (int i = lane; i < n; i += 32) {
+    const Acc v = get(i);
+    e = max(e, max(exp_field(v.s), exp_field(v.c)));
+  }
+  const int emax = __reduce_max_sync(0xffffffffu, e);
   if (emax == 0x7ff) {  // infinities or NaN: in the floating format
+    Acc a{0.0, 0.0};
+    for (int i = lane; i < n; i += 32) acc_merge(a, get(i));
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) acc_merge(a, acc_shfl_down(a, off));
     return a;
   }
-  int L[4] = {0, 0, 0, 0};
-  fix_add(L, a.s, emax);
-  fix_add(L, a.c, emax);
-  int64_t S[4];
+  int64_t S[4] = {0, 0, 0, 0};
+  for (int base = 0; base < n; base += 32) {
+    int L[4] = {0, 0, 0, 0};
+    if (base + lane < n) {
+      const Acc v = get(base + lane);
+      fix_add(L, v.s, emax);
+      fix_add(L, v.c, emax);
+    }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) S[i] = __reduce_add_sync(0xffffffffu, L[i]);
+    for (int i = 0; i < 4; ++i) S[i] += __reduce_add_sync(0xffffffffu, L[i]);
+  }
   return fix_value(S, emax);
 }
+// Sum of one Acc per lane over a warp; result valid in lane 0.
+__device__ __forceinline__ Acc warp_reduce(Acc a) {
+  return warp_sum(32, [&](int) { return a; });
+}
 
-// Sum of one Acc per thread over the CTA (blockDim.x <= BLOCK, whole
-// warps); result valid in thread 0.
-template <int BLOCK>
-__device__ __forceinline__ Acc block_reduce(Acc a) {
+// Sum of get(0) .. get(n - 1) by the CTA (blockDim.x <= BLOCK, whole warps;
+// get(i) is called twice, by thread i mod blockDim.x); result valid in
+// thread 0.
+template <int BLOCK, typename Get>
+__device__ __forceinline__ Acc block_sum(int n, Get get) {
   constexpr int kW = BLOCK / 32;
   __shared__ int wexp[kW];
-  __shared__ int wlimb[kW][4];
+  __shared__ int64_t wlimb[kW][4];
+  __shared__ Acc part[kW];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
-  const int e = __reduce_max_sync(0xffffffffu, max(exp_field(a.s), exp_field(a.c)));
+  int e = 1;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const Acc v = get(i);
+    e = max(e, max(exp_field(v.s), exp_field(v.c)));
+  }
+  e = __reduce_max_sync(0xffffffffu, e);
   if (lane == 0) wexp[warp] = e;
   __syncthreads();
   int emax = 1;
   for (int i = 0; i < nw; ++i) emax = max(emax, wexp[i]);
+  Acc a{0.0, 0.0};
   if (emax == 0x7ff) {  // infinities or NaN: in the floating format
-    __shared__ Acc part[kW];
+    for (int i = threadIdx.x; i < n; i += blockDim.x) acc_merge(a, get(i));
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) acc_merge(a, acc_shfl_down(a, off));
     if (lane == 0) part[warp] = a;
@@ -174,19 +201,25 @@ __device__ __forceinline__ Acc block_reduce(Acc a) {
     __syncthreads();
     return a;
   }
-  int L[4] = {0, 0, 0, 0};
-  fix_add(L, a.s, emax);
-  fix_add(L, a.c, emax);
+  int64_t S[4] = {0, 0, 0, 0};
+  for (int base = 0; base < n; base += blockDim.x) {
+    int L[4] = {0, 0, 0, 0};
+    const int i = base + (int)threadIdx.x;
+    if (i < n) {
+      const Acc v = get(i);
+      fix_add(L, v.s, emax);
+      fix_add(L, v.c, emax);
+    }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) L[i] = __reduce_add_sync(0xffffffffu, L[i]);
+    for (int q = 0; q < 4; ++q) S[q] += __reduce_add_sync(0xffffffffu, L[q]);
+  }
   if (lane == 0) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) wlimb[warp][i] = L[i];
+    for (int i = 0; i < 4; ++i) wlimb[warp][i] = S[i];
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    int64_t S[4] = {0, 0, 0, 0};
-    for (int w = 0; w < nw; ++w) {
+    for (int w = 1; w < nw; ++w) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) S[i] += wlimb[w][i];
     }
@@ -195,16 +228,16 @@ __device__ __forceinline__ Acc block_reduce(Acc a) {
   __syncthreads();
   return a;
 }
-
-// Sum of the partials [0, n) of a launch's CTAs by the last of them; result
-// valid in thread 0.
+// Sum of one Acc per thread over the CTA; result valid in thread 0.
+template <int BLOCK>
+__device__ __forceinline__ Acc block_reduce(Acc a) {
+  return block_sum<BLOCK>((int)blockDim.x, [&](int) { return a; });
+}
+// Sum of the partials [0, n) of a launch's CTAs by the last of them (they
+// were written by other CTAs: read past L1); result valid in thread 0.
 template <int BLOCK>
 __device__ __forceinline__ Acc partials_reduce(const Acc* partials, int n) {
-  Acc t{0.0, 0.0};
-  int i = threadIdx.x;
-  if (i < n) t = partials[i];
-  for (i += blockDim.x; i < n; i += blockDim.x) acc_merge(t, partials[i]);
-  return block_reduce<BLOCK>(t);
+  return block_sum<BLOCK>(n, [&](int i) { return Acc{__ldcg(&partials[i].s), __ldcg(&partials[i].c)}; });
 }
 
 // fp32 compensated strip accumulator (cheap on the FP32 pipe).
@@ -278,41 +311,6 @@ __device__ __forceinline__ F2 f2_from_double(double x) {
 }
 // The double-float rounded to the nearest float.
 __device__ __forceinline__ float f2_round(F2 a) { return __fadd_rn(a.hi, a.lo); }
-
-// A double split into two floats by integer operations alone (no FP64
-// instruction; on GB300 conversions also occupy the FP64 unit): hi takes the
-// sign, the exponent and the leading 24 significant bits (truncated), lo the
-// remaining 29 bits rounded to 23, so |x - (hi + lo)| <= 2^-47 |x|, without
-// bias.  lo comes from a float whose exponent is known, 2^(e-1046) + q
-// 2^(e-1069) with q the rounded top 23 of the 29 bits, minus 2^(e-1046)
-// (exact).  Branch-free.  Only 2^-40 <= |x| < 2^40 is split, so that
-// weighted products and long sums of such values stay far inside the float
-// range; otherwise hi = lo = 0, and ok is false unless x is a zero: other
-// values (small, large, subnormal, infinite, NaN) are the caller's to
-// handle in fp64.
-struct F2Split {
-  F2 v;
-  bool ok;
-};
-__device__ __forceinline__ F2Split f2_split(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const uint32_t bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
-  const uint32_t em = bh & 0x7ff00000u;  // biased binary exponent e, << 20
-  const uint32_t sgn = bh & 0x80000000u;
-  F2Split r;
-  const bool in = em - (983u << 20) <= (79u << 20) + 0xfffffu;  // 983 <= e <= 1062
-  // bits 30..23: the low 8 bits of e, 22..0: fraction bits 51..29; the
-  // float exponent e - 896 is those 8 bits with the top one flipped
-  const uint32_t fs = __funnelshift_l(bl, bh, 3);
-  const float hi = __uint_as_float(((fs ^ 0x40000000u) & 0x7fffffffu) | sgn);
-  const uint32_t ex = em * 8u - (919u << 23);
-  const uint32_t q = ((bl & 0x1fffffffu) + 32u) >> 6;  // a carry into the exponent stays exact
-  const float lo = __fsub_rn(__uint_as_float(ex + q), __uint_as_float(ex));
-  r.v.hi = in ? hi : 0.f;
-  r.v.lo = in ? __uint_as_float(__float_as_uint(lo) | sgn) : 0.f;
-  r.ok = in || ((bh & 0x7fffffffu) | bl) == 0u;
-  return r;
-}
 
 // "Last CTA finishes" pattern: every CTA writes its partial, fences, takes a
 // ticket; the CTA that draws the last ticket reduces all partials in index
