@@ -244,7 +244,6 @@ __device__ __forceinline__ T vegas_outer(const Family<T>& f, T s) {
 
 // Philox blocks a point's D draws can touch: a point's first draw sits at
 // word (j*D) mod PB of its first block, at most PB - gcd(D, PB).
-__host__ __device__ constexpr int gcd_c(int a, int b) { return b == 0 ? a : gcd_c(b, a % b); }
 template <int D, int PB>
 struct DrawBlocks {
   static constexpr int step = gcd_c(D, PB);               // first-word offsets are multiples
