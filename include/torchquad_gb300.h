@@ -246,12 +246,29 @@ int tq_weighted_sum(int dtype, int rule, int dim, int64_t n_per_dim,
                     int64_t n_values, double* acc, void* workspace,
                     size_t workspace_bytes, void* stream);
 
+/* tq_weighted_sum of a whole range at once: out[s] (out_dtype) = the sum, for
+ * TQ_RULE_MC times prod_k(b_k - a_k) (in dtype, as monte_carlo.py:72-77) over
+ * count; no running sum, no second call (count >= 1). */
+int tq_weighted_result(int dtype, int rule, int dim, int64_t n_per_dim,
+                       const void* domain, const double* gl_weights,
+                       int64_t start, int64_t count, const void* f, int f_dtype,
+                       int64_t n_values, void* out, int out_dtype,
+                       void* workspace, size_t workspace_bytes, void* stream);
+
 /* out[s] = (out_dtype)(scale * (acc[2s] + acc[2s+1])) where scale is 1 for
  * grid rules and prod_k(b_k - a_k) / n_points (computed in dtype, as
  * monte_carlo.py:72-77) for TQ_RULE_MC. */
 int tq_finalize_sum(int dtype, int rule, int dim, const void* domain,
                     int64_t n_points, const double* acc, int64_t n_values,
                     void* out, int out_dtype, void* stream);
+
+/* Monte Carlo points (monte_carlo.py:84-106): points[count][dim] (dtype) =
+ * u * (b - a) + a, u the elements 0 .. count*dim-1 of tq_uniform's stream from
+ * block offset `offset`; the product and the sum rounded one after the other
+ * in dtype.  domain: device [dim][2] of dtype. */
+int tq_sample_points(int dtype, int dim, int64_t count, const void* domain,
+                     uint64_t seed, uint64_t stream_id, uint64_t offset,
+                     void* points, void* stream);
 
 /* ---- random numbers ------------------------------------------------------ */
 

@@ -178,6 +178,13 @@ SIGNATURES = {
         [c_int, c_int, c_int, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_int,
          c_int64, c_void_p, c_void_p, c_size_t, c_void_p],
     ),
+    "tq_weighted_result": (
+        c_int,
+        [c_int, c_int, c_int, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_int,
+         c_int64, c_void_p, c_int, c_void_p, c_size_t, c_void_p],
+    ),
+    "tq_sample_points": (
+        c_int, [c_int, c_int, c_int64, c_void_p, c_uint64, c_uint64, c_uint64, c_void_p, c_void_p]),
     "tq_finalize_sum": (
         c_int,
         [c_int, c_int, c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int, c_void_p],

@@ -28,6 +28,49 @@ __global__ void __launch_bounds__(kBlock)
   }
 }
 
+// Uniform points of a box, in one pass (tq_uniform and two torch operations
+// wrote and read the [count, dim] array three times: 10^6 x 3 fp64 35 us on
+// the device, 16.5 us here).  Two roundings per coordinate, as u * width + lo
+// has them in torch.
+template <typename T>
+__global__ void __launch_bounds__(kBlock)
+    sample_points_kernel(int dim, int64_t numel, const T* __restrict__ dom, uint64_t seed, uint64_t sid,
+                         uint64_t offset, T* __restrict__ out) {
+  constexpr int PB = Uniform<T>::per_block;
+  __shared__ T lo[kMaxDim], width[kMaxDim];
+  __shared__ FastDiv fd;
+  if (threadIdx.x < dim) {
+    lo[threadIdx.x] = dom[2 * threadIdx.x];
+    width[threadIdx.x] = dom[2 * threadIdx.x + 1] - dom[2 * threadIdx.x];
+  }
+  if (threadIdx.x == 0) fd = make_fastdiv((uint32_t)dim);
+  __syncthreads();
+  const int64_t nblk = (numel + PB - 1) / PB;
+  const bool small = numel <= (int64_t)0xffffffffll;
+  for (int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nblk; b += (int64_t)gridDim.x * blockDim.x) {
+    const uint4 r = philox_block(seed, sid, offset + (uint64_t)b);
+    const int64_t e0 = b * PB;
+    int k = small ? (int)((uint32_t)e0 - fdiv((uint32_t)e0, fd) * fd.d) : (int)(e0 % dim);
+    T v[PB];
+#pragma unroll
+    for (int l = 0; l < PB; ++l) {
+      const T u = Uniform<T>::from(r, l);
+      if constexpr (sizeof(T) == 4)
+        v[l] = __fadd_rn(__fmul_rn(u, width[k]), lo[k]);
+      else
+        v[l] = __dadd_rn(__dmul_rn(u, width[k]), lo[k]);
+      k = k + 1 == dim ? 0 : k + 1;
+    }
+    if (e0 + PB <= numel && ((uintptr_t)out & 15) == 0) {  // a block's values are 16 bytes
+      *(uint4*)(out + e0) = *(const uint4*)v;
+    } else {
+#pragma unroll
+      for (int l = 0; l < PB; ++l)
+        if (e0 + l < numel) out[e0 + l] = v[l];
+    }
+  }
+}
+
 struct McArgs {
   int dim, family;
   int64_t n_points;
@@ -211,6 +254,28 @@ extern "C" int tq_uniform(int dtype, uint64_t seed, uint64_t stream_id, uint64_t
   else
     uniform_kernel<float><<<(unsigned)grid, kBlock, 0, s>>>(seed, stream_id, offset, numel,
                                                             (float*)out);
+  return launch_status();
+}
+
+extern "C" int tq_sample_points(int dtype, int dim, int64_t count, const void* domain, uint64_t seed,
+                                uint64_t stream_id, uint64_t offset, void* points, void* stream) {
+  if (!valid_dtype(dtype)) return TQ_ERR_DTYPE;
+  if (dim < 1 || dim > kMaxDim) return TQ_ERR_DIM;
+  if (count < 0 || !domain || (!points && count > 0)) return TQ_ERR_ARG;
+  if (count > (int64_t(1) << 60) / dim) return TQ_ERR_TOO_LARGE;
+  if (count == 0) return TQ_OK;
+  const int64_t numel = count * dim;
+  const int64_t nblk = (numel + (dtype == TQ_F64 ? 1 : 3)) / (dtype == TQ_F64 ? 2 : 4);
+  int64_t grid = (nblk + kBlock - 1) / kBlock;
+  const int64_t cap = (int64_t)sm_count() * 16;
+  if (grid > cap) grid = cap;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (dtype == TQ_F64)
+    sample_points_kernel<double><<<(unsigned)grid, kBlock, 0, s>>>(dim, numel, (const double*)domain, seed, stream_id,
+                                                                   offset, (double*)points);
+  else
+    sample_points_kernel<float><<<(unsigned)grid, kBlock, 0, s>>>(dim, numel, (const float*)domain, seed, stream_id,
+                                                                  offset, (float*)points);
   return launch_status();
 }
 

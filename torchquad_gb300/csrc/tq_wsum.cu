@@ -55,10 +55,37 @@ struct WsumArgs {
   const void* domain;
   const double* gl_weights;
   const void* f;
-  double* acc;
+  double* acc;   // running sums [n_values][2] (out == nullptr)
+  void* out;     // or the results themselves, of out_dtype
+  int out_dtype;
   Acc* partials;
   unsigned* ticket;
 };
+
+// Sum t of component s into the running sum, or as the result: times the
+// domain's volume over the samples (monte_carlo.py:72-77, the volume in the
+// domain's type) for Monte Carlo.
+template <typename D>
+__device__ __forceinline__ void wsum_store(const WsumArgs& a, int64_t s, Acc t) {
+  if (!a.out) {
+    Acc run{a.acc[2 * s], a.acc[2 * s + 1]};
+    acc_merge(run, t);
+    a.acc[2 * s] = run.s;
+    a.acc[2 * s + 1] = run.c;
+    return;
+  }
+  double v = t.s + t.c;
+  if (a.rule == TQ_RULE_MC) {
+    const D* dom = (const D*)a.domain;
+    D vol = (D)1;
+    for (int k = 0; k < a.dim; ++k) vol = vol * (D)(dom[2 * k + 1] - dom[2 * k]);
+    v *= (double)vol / (double)a.count;
+  }
+  if (a.out_dtype == TQ_F64)
+    ((double*)a.out)[s] = v;
+  else
+    ((float*)a.out)[s] = (float)v;
+}
 
 // Inner weights.  One dimension: a lane's nodes keep their place modulo four
 // as it strides over a segment, so a Newton-Cotes lane has one interior and
@@ -86,11 +113,11 @@ __device__ void wsum_join_table(const WsumArgs& a, double* tab) {
     tab[j] = w;
   }
 }
-// Outer weight of a row: the remaining dimensions' weights and every
-// dimension's scale (scale: their product).
+// Outer weight of a row: the remaining dimensions' unscaled weights (whole
+// numbers for the Newton-Cotes rules, exact as double-floats too).
 template <bool GL>
-__device__ __forceinline__ double wsum_outer(const WsumArgs& a, double scale, const FastDiv& fd, int64_t row) {
-  double w = scale;
+__device__ __forceinline__ double wsum_outer(const WsumArgs& a, const FastDiv& fd, int64_t row) {
+  double w = 1.0;
   const int n32 = (int)a.n;
   if (row <= (int64_t)0xffffffffll) {
     uint32_t r = (uint32_t)row;
@@ -189,25 +216,24 @@ struct UnitSumP {
 };
 
 // A lane's sum over its units, each folded in with its outer weight w: in
-// fp64, or as double-floats in units of 2^e0, the binary exponent of the
-// weights' scale, with unit sums of 2^80 and more (and infinities and NaN) in
-// the fp64 side sum.
+// fp64, or as double-floats, with unit sums of 2^60 and more (and infinities
+// and NaN) in the fp64 side sum.
 struct LaneSumD {
   double s = 0.0;
   __device__ __forceinline__ void fold(const UnitSumD& u, double w, F2, double*) { s = fma(u.s, w, s); }
-  __device__ __forceinline__ Acc value(double) const { return Acc{s, 0.0}; }
+  __device__ __forceinline__ Acc value() const { return Acc{s, 0.0}; }
 };
 struct LaneSumF {
   F2 s{0.f, 0.f};
   __device__ __forceinline__ void fold(const UnitSumF& u, double w, F2 wf, double* side) {
-    const bool in = fabsf(u.s) < 0x1p80f;
+    const bool in = fabsf(u.s) < 0x1p60f;
     if (in) s = f2_add(s, f2_mul(two_sum(u.s, -u.c), wf));
     if (__any_sync(0xffffffffu, !in)) side_add(side, in ? 0.0 : w, in ? 0.0 : (double)u.s - (double)u.c);
   }
   __device__ __forceinline__ void fold(const UnitSumP& u, double, F2 wf, double*) {
     s = f2_add(s, f2_mul(two_sum(u.hi, u.lo), wf));
   }
-  __device__ __forceinline__ Acc value(double unit) const { return Acc{(double)s.hi * unit, (double)s.lo * unit}; }
+  __device__ __forceinline__ Acc value() const { return Acc{(double)s.hi, (double)s.lo}; }
 };
 
 // Exact running sums of a lane (Monte Carlo and vector integrands): FixAcc
@@ -228,15 +254,15 @@ struct F3Acc {
     b = u.hi;
     c = __fadd_rn(c, u.lo);
   }
-  __device__ __forceinline__ void value(Acc& r, double unit) const {
+  __device__ __forceinline__ void value(Acc& r, double unit) const {  // unit: a power of two
     acc_add(r, (double)a * unit);
     acc_add(r, ((double)b + (double)c) * unit);
   }
 };
 // A lane's exact sum of weight x value.  fp32: values below 2^-60 go into a
 // sum of their own, scaled up (products of theirs would lose their last bits
-// below the float range), values of 2^60 and more, infinities and NaN into an
-// fp64 sum; the weight is a double-float in units of 2^e0.
+// below the float range), values of 2^50 and more, infinities and NaN into an
+// fp64 sum; the weight is a double-float.
 template <typename F>
 struct ExactSum;
 template <>
@@ -244,20 +270,20 @@ struct ExactSum<double> {
   FixAcc s;
   __device__ __forceinline__ void add(double v) { s.add(v); }
   __device__ __forceinline__ void add(double w, F2, double v) { s.add(w * v); }
-  __device__ __forceinline__ Acc value(double) const { return s.value(); }
+  __device__ __forceinline__ Acc value() const { return s.value(); }
 };
 template <>
 struct ExactSum<float> {
   F3Acc s, small;
   Acc side{0.0, 0.0};
   __device__ __forceinline__ void add(float v) {
-    if (fabsf(v) < 0x1p60f)
+    if (fabsf(v) < 0x1p50f)
       s.add(v);  // sums of values themselves lose nothing below the float range
     else
       acc_add(side, (double)v);
   }
   __device__ __forceinline__ void add(double w, F2 wf, float v) {
-    if (fabsf(v) < 0x1p60f) {
+    if (fabsf(v) < 0x1p50f) {
       const bool tiny = fabsf(v) < 0x1p-60f;
       const float x = tiny ? v * 0x1p96f : v;
       const float p = __fmul_rn(wf.hi, x);
@@ -270,19 +296,20 @@ struct ExactSum<float> {
       acc_add(side, w * (double)v);
     }
   }
-  __device__ __forceinline__ Acc value(double unit) const {
+  __device__ __forceinline__ Acc value() const {
     Acc r = side;
-    s.value(r, unit);
-    if (small.a != 0.f || small.b != 0.f || small.c != 0.f) small.value(r, unit * 0x1p-96);
+    s.value(r, 1.0);
+    if (small.a != 0.f || small.b != 0.f || small.c != 0.f) small.value(r, 0x1p-96);
     return r;
   }
 };
 
-// Shared set-up of the kernels: the weights' scale, its binary exponent and
+// Shared set-up of the kernels: the product of the dimensions' weight scales
+// (a CTA's sums take it at the very end, in fp64: folded into the rows'
+// double-float weights it would be rounded to 2^-48 for all of them alike) and
 // the join table.
 struct WsumSetup {
-  double scale;  // product of the dimensions' weight scales
-  double unit, inv_unit;  // 2^e0 and 2^-e0 (1 outside 2^+-1000)
+  double scale;
   FastDiv fd;
 };
 template <typename T, typename D, bool GL, bool JOIN>
@@ -293,27 +320,26 @@ __device__ __forceinline__ void wsum_setup(const WsumArgs& a, Geo<T>& g, WsumSet
   if (threadIdx.x == 0) {
     double s = 1.0;
     for (int k = 0; k < a.dim; ++k) s *= g.wscale[k];
-    const int e = exp_field(s) - 1023;
-    const bool in = e >= -1000 && e <= 1000;
     su.scale = s;
-    su.unit = in ? __hiloint2double((e + 1023) << 20, 0) : 1.0;
-    su.inv_unit = in ? __hiloint2double((1023 - e) << 20, 0) : 1.0;
     su.fd = make_fastdiv((uint32_t)a.n);
   }
   __syncthreads();
 }
+// (hi + lo) times s, rounded once
+__device__ __forceinline__ Acc wsum_scaled(Acc v, double s) {
+  const double p = v.s * s;
+  return Acc{p, fma(v.c, s, fma(v.s, s, -p))};
+}
 
-// The CTAs' sums into the running sum acc[0..1], by the last of them.
-__device__ __forceinline__ void wsum_finish(const WsumArgs& a, Acc mine) {
+// The CTAs' sums into the running sum or the result, by the last of them.
+template <typename D>
+__device__ __forceinline__ void wsum_finish(const WsumArgs& a, Acc mine, double scale) {
   const Acc acc = block_reduce<kBlock>(mine);
-  if (threadIdx.x == 0) a.partials[blockIdx.x] = acc;
+  if (threadIdx.x == 0) a.partials[blockIdx.x] = wsum_scaled(acc, scale);
   if (last_block_arrives(a.ticket)) {
     const Acc t = partials_reduce<kBlock>(a.partials, (int)gridDim.x);
     if (threadIdx.x == 0) {
-      Acc run{a.acc[0], a.acc[1]};
-      acc_merge(run, t);
-      a.acc[0] = run.s;
-      a.acc[1] = run.c;
+      wsum_store<D>(a, 0, t);
       *a.ticket = 0u;
     }
   }
@@ -349,7 +375,7 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_kernel(WsumArgs a) {
     double w = 0.0;  // outer weight of unit u0 + lane
     if (lane < cnt) {
       const int64_t row = unit_row(a, u0 + lane);
-      w = wsum_outer<GL>(a, su.scale, su.fd, a.row0 + row);
+      w = wsum_outer<GL>(a, su.fd, a.row0 + row);
       if (ONE) {
         const int64_t j0 = (u0 + lane - row * a.segs) * a.seg, p0 = (a.row0 + row) * a.R, p1 = p0 + a.R - 1;
         double e = 0.0;
@@ -359,7 +385,7 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_kernel(WsumArgs a) {
       }
     }
     F2 wf{0.f, 0.f};
-    if (F32 || PAIR) wf = f2_from_double(w * su.inv_unit);
+    if (F32 || PAIR) wf = f2_from_double(w);
     for (int q = 0; q < cnt; ++q) {
       const int64_t u = u0 + q;
       const int64_t row = unit_row(a, u);
@@ -422,18 +448,18 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_kernel(WsumArgs a) {
       sum.fold(us, wq, wqf, &side);
     }
   }
-  Acc r = sum.value(su.unit);
+  Acc r = sum.value();
   if (side != 0.0) acc_add(r, side);
   if (ONE) {  // the lane's weight (a small integer), then the end nodes
     r.s *= wi;
     r.c *= wi;
     acc_add(r, ends);
   }
-  wsum_finish(a, r);
+  wsum_finish<D>(a, r, su.scale);
 }
 
 // Monte Carlo samples of one value: their plain sum.
-template <typename F>
+template <typename D, typename F>
 __global__ void __launch_bounds__(kBlock, 4) sample_sum_kernel(WsumArgs a) {
   const F* __restrict__ f = (const F*)a.f;
   const int64_t step = (int64_t)gridDim.x * kBlock;
@@ -447,7 +473,7 @@ __global__ void __launch_bounds__(kBlock, 4) sample_sum_kernel(WsumArgs a) {
     for (int p = 0; p < 8; ++p) sum.add(v[p]);
   }
   for (; i < a.count; i += step) sum.add(__ldg(f + i));
-  wsum_finish(a, sum.value(1.0));
+  wsum_finish<D>(a, sum.value(), 1.0);
 }
 
 // Several values per node: lane = component + chunk * node, partials[CTA of
@@ -479,7 +505,7 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_vec_kernel(WsumArgs a)
     const int64_t r0 = (a.row0 + row) * a.R;
     const int64_t b = max(j0, a.start - r0);
     const int64_t j1 = min(min(j0 + a.seg, a.R), end - r0);
-    const double wo = mc ? 1.0 : wsum_outer<GL>(a, su.scale, su.fd, a.row0 + row);
+    const double wo = mc ? 1.0 : wsum_outer<GL>(a, su.fd, a.row0 + row);
     for (int64_t jb = b; jb < j1; jb += batch) {
       const int nb = (int)min((int64_t)batch, j1 - jb);
       double w = 0.0;  // weight of the batch's node `lane`
@@ -488,7 +514,7 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_vec_kernel(WsumArgs a)
         const int64_t j = jb + min(lane, nb - 1);
         w = wo * (JOIN ? tab[j] : GL ? __ldg(a.gl_weights + j)
                                      : wsum_weight<double>(a.rule, (int)(j & 3), j == 0 || j == a.R - 1));
-        if (F32) wf = f2_from_double(w * su.inv_unit);
+        if (F32) wf = f2_from_double(w);
       }
       const F* fr = f + (r0 - a.start + jb) * S;
       for (int i = 0; i < nb; i += 8 * per) {
@@ -514,27 +540,22 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_vec_kernel(WsumArgs a)
       }
     }
   }
-  part[threadIdx.x] = sum.value(mc ? 1.0 : su.unit);
+  part[threadIdx.x] = sum.value();
   __syncthreads();
   const int entries = (kBlock / 32) * per;  // a component's lanes: warp e / per, node e % per
   for (int c = warp; c < ncomp; c += kBlock / 32) {
     const Acc t = warp_sum(entries, [&](int e) { return part[(e / per) * 32 + (e % per) * ncomp + c]; });
-    if (lane == 0) a.partials[(int64_t)blockIdx.x * S + s0 + c] = t;
+    if (lane == 0) a.partials[(int64_t)blockIdx.x * S + s0 + c] = mc ? t : wsum_scaled(t, su.scale);
   }
 }
 
-// acc[s] += the partials of component s, one warp per component.
-__global__ void __launch_bounds__(kBlock) weighted_sum_combine_kernel(const Acc* partials, int n, int64_t S,
-                                                                      double* acc) {
+// The partials of component s added up, one warp per component.
+template <typename D>
+__global__ void __launch_bounds__(kBlock) weighted_sum_combine_kernel(WsumArgs a, int n) {
   const int64_t s = ((int64_t)blockIdx.x * kBlock + threadIdx.x) >> 5;
-  if (s >= S) return;
-  const Acc t = warp_sum(n, [&](int e) { return partials[(int64_t)e * S + s]; });
-  if ((threadIdx.x & 31) == 0) {
-    Acc run{acc[2 * s], acc[2 * s + 1]};
-    acc_merge(run, t);
-    acc[2 * s] = run.s;
-    acc[2 * s + 1] = run.c;
-  }
+  if (s >= a.n_values) return;
+  const Acc t = warp_sum(n, [&](int e) { return a.partials[(int64_t)e * a.n_values + s]; });
+  if ((threadIdx.x & 31) == 0) wsum_store<D>(a, s, t);
 }
 
 template <typename D>
@@ -598,15 +619,14 @@ static bool wsum_valid_rule(int rule, int64_t n) {
   }
 }
 
-extern "C" int tq_weighted_sum(int dtype, int rule, int dim, int64_t n_per_dim,
-                               const void* domain, const double* gl_weights, int64_t start,
-                               int64_t count, const void* f, int f_dtype, int64_t n_values,
-                               double* acc, void* workspace, size_t workspace_bytes,
-                               void* stream) {
+static int wsum_launch(int dtype, int rule, int dim, int64_t n_per_dim, const void* domain,
+                       const double* gl_weights, int64_t start, int64_t count, const void* f, int f_dtype,
+                       int64_t n_values, double* acc, void* out, int out_dtype, void* workspace,
+                       size_t workspace_bytes, void* stream) {
   if (!valid_dtype(dtype) || !valid_dtype(f_dtype)) return TQ_ERR_DTYPE;
   if (dim < 1 || dim > kMaxDim) return TQ_ERR_DIM;
   if (rule != TQ_RULE_MC && !wsum_valid_rule(rule, n_per_dim)) return TQ_ERR_RULE;
-  if (!domain || !f || !acc || !workspace || start < 0 || count < 0 || n_values < 1)
+  if (!domain || !f || (!acc && !out) || !workspace || start < 0 || count < 0 || n_values < 1)
     return TQ_ERR_ARG;
   if (rule == TQ_RULE_GAUSS && !gl_weights) return TQ_ERR_ARG;
   if (rule != TQ_RULE_MC) {
@@ -632,6 +652,8 @@ extern "C" int tq_weighted_sum(int dtype, int rule, int dim, int64_t n_per_dim,
   a.gl_weights = gl_weights;
   a.f = f;
   a.acc = acc;
+  a.out = out;
+  a.out_dtype = out_dtype;
   a.ticket = (unsigned*)workspace;
   a.partials = (Acc*)((char*)workspace + 256);
   const bool gl = rule == TQ_RULE_GAUSS, mc = rule == TQ_RULE_MC;
@@ -667,10 +689,13 @@ extern "C" int tq_weighted_sum(int dtype, int rule, int dim, int64_t n_per_dim,
   a.chunk = (int)(n_values < kComps ? n_values : kComps);
   const dim3 grid((unsigned)gx, (unsigned)(n_values == 1 ? 1 : chunks));
   if (mc && n_values == 1) {
-    if (f_dtype == TQ_F64)
-      sample_sum_kernel<double><<<grid, kBlock, 0, s>>>(a);
-    else
-      sample_sum_kernel<float><<<grid, kBlock, 0, s>>>(a);
+    if (dtype == TQ_F64) {
+      if (f_dtype == TQ_F64) sample_sum_kernel<double, double><<<grid, kBlock, 0, s>>>(a);
+      else sample_sum_kernel<double, float><<<grid, kBlock, 0, s>>>(a);
+    } else {
+      if (f_dtype == TQ_F64) sample_sum_kernel<float, double><<<grid, kBlock, 0, s>>>(a);
+      else sample_sum_kernel<float, float><<<grid, kBlock, 0, s>>>(a);
+    }
     return launch_status();
   }
   if (pair) {
@@ -709,10 +734,33 @@ extern "C" int tq_weighted_sum(int dtype, int rule, int dim, int64_t n_per_dim,
   if (n_values > 1) {
     const int e = launch_status();
     if (e != TQ_OK) return e;
-    weighted_sum_combine_kernel<<<(unsigned)((n_values * 32 + kBlock - 1) / kBlock), kBlock, 0, s>>>(
-        a.partials, (int)gx, n_values, acc);
+    const unsigned cb = (unsigned)((n_values * 32 + kBlock - 1) / kBlock);
+    if (dtype == TQ_F64)
+      weighted_sum_combine_kernel<double><<<cb, kBlock, 0, s>>>(a, (int)gx);
+    else
+      weighted_sum_combine_kernel<float><<<cb, kBlock, 0, s>>>(a, (int)gx);
   }
   return launch_status();
+}
+
+extern "C" int tq_weighted_sum(int dtype, int rule, int dim, int64_t n_per_dim,
+                               const void* domain, const double* gl_weights, int64_t start,
+                               int64_t count, const void* f, int f_dtype, int64_t n_values,
+                               double* acc, void* workspace, size_t workspace_bytes,
+                               void* stream) {
+  if (!acc && count > 0) return TQ_ERR_ARG;
+  return wsum_launch(dtype, rule, dim, n_per_dim, domain, gl_weights, start, count, f, f_dtype, n_values, acc,
+                     nullptr, TQ_F64, workspace, workspace_bytes, stream);
+}
+
+extern "C" int tq_weighted_result(int dtype, int rule, int dim, int64_t n_per_dim, const void* domain,
+                                  const double* gl_weights, int64_t start, int64_t count, const void* f,
+                                  int f_dtype, int64_t n_values, void* out, int out_dtype, void* workspace,
+                                  size_t workspace_bytes, void* stream) {
+  if (!valid_dtype(out_dtype)) return TQ_ERR_DTYPE;
+  if (!out || count < 1) return TQ_ERR_ARG;
+  return wsum_launch(dtype, rule, dim, n_per_dim, domain, gl_weights, start, count, f, f_dtype, n_values, nullptr,
+                     out, out_dtype, workspace, workspace_bytes, stream);
 }
 
 extern "C" int tq_finalize_sum(int dtype, int rule, int dim, const void* domain, int64_t n_points,

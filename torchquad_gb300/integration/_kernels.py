@@ -8,6 +8,7 @@ from __future__ import annotations
 import os
 
 import torch
+import torch.autograd.forward_ad as fwAD
 
 from .. import _lib as L
 
@@ -83,6 +84,47 @@ def finalize(acc, rule, dim, domain, n_points, S, out_dtype):
     return out
 
 
+def weighted_result(rule, dim, n, domain, gl_weights, start, values2d, out_dtype):
+    """[S] results of one range: sum_i w_i values2d[i, :], for Monte Carlo
+    times the domain's volume over the samples; one call, no running sum."""
+    count, S = values2d.shape
+    lib = L.lib()
+    ws = L.workspace.get(lib.tq_weighted_sum_workspace_size(count, S), "wsum")
+    out = torch.empty((S,), dtype=out_dtype, device=domain.device)
+    L.check(
+        lib.tq_weighted_result(
+            L.dtype_code(domain.dtype), rule, dim, n, domain.data_ptr(), L.ptr(gl_weights),
+            start, count, values2d.data_ptr(), L.dtype_code(values2d.dtype), S,
+            out.data_ptr(), L.dtype_code(out_dtype), ws.data_ptr(), ws.numel(), L.stream_handle(),
+        ),
+        "tq_weighted_result",
+    )
+    L.count_launches(1 if S == 1 else 2)
+    return out
+
+
+def plain_tensor(t) -> bool:
+    """Whether t is an ordinary tensor outside every transform that follows
+    torch operations (tracing, vmap and other functorch levels, forward-mode
+    derivatives), so that a kernel may take the place of torch operations on
+    it.  Gradients are the caller's to look at."""
+    return (type(t) is torch.Tensor and not torch.jit.is_tracing() and fwAD._current_level < 0
+            and torch._C._functorch.peek_interpreter_stack() is None)
+
+
+def sample_points(seed, stream_id, offset, N, domain):
+    """[N, dim] uniform points of the domain from the Philox stream."""
+    dim = domain.shape[0]
+    out = torch.empty((N, dim), dtype=domain.dtype, device=domain.device)
+    L.check(
+        L.lib().tq_sample_points(L.dtype_code(domain.dtype), dim, N, domain.data_ptr(), seed, stream_id, offset,
+                                 out.data_ptr(), L.stream_handle()),
+        "tq_sample_points",
+    )
+    L.count_launches(1)
+    return out
+
+
 class WeightedSum(torch.autograd.Function):
     """sum_i w_i * values[i, :] over a node range, differentiable in values.
 
@@ -92,9 +134,12 @@ class WeightedSum(torch.autograd.Function):
     @staticmethod
     def forward(ctx, values2d, rule, dim, n, domain, gl_weights, start):
         S = values2d.shape[1]
-        acc = torch.zeros((2 * S,), dtype=torch.float64, device=values2d.device)
-        weighted_sum_into(acc, rule, dim, n, domain, gl_weights, start, values2d)
-        out = finalize(acc, L.TQ_RULE_TRAPEZOID, dim, domain, 1, S, values2d.dtype)
+        if rule != L.TQ_RULE_MC and values2d.shape[0] > 0:
+            out = weighted_result(rule, dim, n, domain, gl_weights, start, values2d, values2d.dtype)
+        else:  # plain sums: the Monte Carlo volume is the caller's
+            acc = torch.zeros((2 * S,), dtype=torch.float64, device=values2d.device)
+            weighted_sum_into(acc, rule, dim, n, domain, gl_weights, start, values2d)
+            out = finalize(acc, L.TQ_RULE_TRAPEZOID, dim, domain, 1, S, values2d.dtype)
         ctx.meta = (rule, dim, n, domain, gl_weights, start, values2d.shape[0], values2d.dtype)
         return out
 

@@ -222,6 +222,10 @@ class GridIntegrator(BaseIntegrator):
             if values.requires_grad and torch.is_grad_enabled():
                 outs.append(K.WeightedSum.apply(values, self._rule, dim, n, domain, gl_w, start))
                 continue
+            if count == total:
+                out_dtype = torch.promote_types(values.dtype, self._result_dtype(domain))
+                out = K.weighted_result(self._rule, dim, n, domain, gl_w, 0, values, out_dtype)
+                return _assemble_result(out, shape, is_complex)
             if acc is None:
                 acc = torch.zeros((2 * values.shape[1],), dtype=torch.float64, device=domain.device)
             K.weighted_sum_into(acc, self._rule, dim, n, domain, gl_w, start, values)

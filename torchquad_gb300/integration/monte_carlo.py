@@ -55,10 +55,8 @@ class MonteCarlo(BaseIntegrator):
             volume = torch.prod(domain[:, 1] - domain[:, 0])
             out = volume.to(s.dtype) * s / n
         else:
-            acc = torch.zeros((2 * values.shape[1],), dtype=torch.float64, device=values.device)
-            K.weighted_sum_into(acc, L.TQ_RULE_MC, dim, 1, domain, None, 0, values)
             out_dtype = torch.promote_types(values.dtype, domain.dtype)
-            out = K.finalize(acc, L.TQ_RULE_MC, dim, domain, n, values.shape[1], out_dtype)
+            out = K.weighted_result(L.TQ_RULE_MC, dim, 1, domain, None, 0, values, out_dtype)
         return _assemble_result(out, shape, is_complex)
 
     def calculate_sample_points(self, N, integration_domain, seed=None, rng=None):
@@ -68,6 +66,10 @@ class MonteCarlo(BaseIntegrator):
         elif seed is not None:
             raise ValueError("seed and rng cannot both be passed")
         dim = integration_domain.shape[0]
+        if self._can_fuse_points(integration_domain, rng):
+            N = int(N)
+            offset = rng.reserve(N * dim, integration_domain.dtype)
+            return K.sample_points(rng.seed, rng.stream_id, offset, N, integration_domain.contiguous())
         domain_starts = integration_domain[:, 0]
         domain_sizes = integration_domain[:, 1] - domain_starts
         u = rng.uniform(size=[N, dim], dtype=domain_sizes.dtype)
@@ -75,6 +77,22 @@ class MonteCarlo(BaseIntegrator):
             u = torch.as_tensor(u)
         u = u.to(domain_sizes.device)
         return u * domain_sizes + domain_starts
+
+    @staticmethod
+    def _can_fuse_points(domain, rng):
+        """Points by one kernel: this package's draws on a CUDA domain that
+        no derivative or transform follows."""
+        return (
+            type(rng) is RNG
+            and domain.dtype in (torch.float32, torch.float64)
+            and domain.is_cuda
+            and domain.device.index == torch.cuda.current_device()
+            and domain.dim() == 2
+            and domain.shape[1] == 2
+            and 1 <= domain.shape[0] <= L.TQ_MAX_DIM
+            and not (torch.is_grad_enabled() and domain.requires_grad)
+            and K.plain_tensor(domain)
+        )
 
     def get_jit_compiled_integrate(self, dim, N=1000, integration_domain=None, seed=None, backend=None):
         """integrate(fn, integration_domain) with dim, N and the RNG stream
