@@ -189,6 +189,25 @@ int tq_grid_adjoint(int dtype, int rule, int dim, int64_t n_per_dim, const void*
                     double* out_grad_params, void* workspace, size_t workspace_bytes,
                     void* stream);
 
+/* Backward of the fused rule for a result gradient grad_out[0] (device,
+ * grad_out_dtype): grad_out times the gradient of tq_grid_adjoint, with
+ * respect to the domain ([dim][2]), c, b, a ([dim]) and u ([dim]), into
+ * grads[0..4] (host array of device pointers, contiguous, NULL where no
+ * gradient is wanted) of types grad_dtypes[0..4].  Workspace as for
+ * tq_grid_adjoint. */
+int tq_grid_vjp(int dtype, int rule, int dim, int64_t n_per_dim, const void* domain,
+                const double* gl_nodes, const double* gl_weights, int family,
+                const double* params, const void* grad_out, int grad_out_dtype,
+                void* const* grads, const int* grad_dtypes, void* workspace,
+                size_t workspace_bytes, void* stream);
+
+/* The device parameter vector c, b, a[dim], u[dim] (fp64) from device tensors
+ * and host values: dev[0..3] (host array: c, b, a, u; NULL takes the values of
+ * host[2 + 2*dim] instead), their types and element strides. */
+int tq_pack_params(int dim, const void* const* dev, const int* dtypes,
+                   const int64_t* strides, const double* host, double* out,
+                   void* stream);
+
 /* Workspace bytes of tq_batch_grid_adjoint: n_tiles rows of 2 + 4*max_dim
  * fp64 partial sums. */
 size_t tq_batch_grid_adjoint_workspace_size(int64_t n_tiles, int max_dim);

@@ -179,3 +179,63 @@ def test_batch_values_match_oracle(dtype, tile, cuda):
         tol = 1e-12 if dtype == torch.float64 else 1e-6
         bad = np.abs(got - want) > tol * mag + 1e-300
         assert not bad.any(), [(fs[i], rules[i], Ns[i], got[i], want[i]) for i in np.nonzero(bad)[0][:5]]
+
+
+@pytest.mark.parametrize("where", ["device", "host", "mixed", "strided"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_backward_from_device_and_host_parameters(where, dtype, cuda):
+    """The parameter vector gathered on the device and the one-launch backward
+    against the gradient oracle; host parameters take the torch path."""
+    from oracle import grad as OGR
+
+    dim, n = 3, 21
+    dom_l = domain(dim)
+    a, u, c = [0.9, 1.7, 0.6], [0.2, 0.4, 0.1], 1.3
+    dev = {"device": cuda, "host": "cpu", "mixed": cuda, "strided": cuda}[where]
+    leaf = lambda x, d=dev, t=torch.float64: torch.tensor(x, dtype=t, device=d).requires_grad_()  # noqa: E731
+    if where == "strided":
+        base = leaf([[v, 0.0] for v in a])
+        a_t = base[:, 0]
+    else:
+        base = a_t = leaf(a)
+    u_t = leaf(u, "cpu" if where == "mixed" else dev)
+    c_t = leaf(c, dev, torch.float32)
+    dom = torch.tensor(dom_l, dtype=dtype, device=cuda).requires_grad_()
+    f = tq.GaussianPeak(dim, a=a_t, u=u_t, c=c_t)
+    val = tq.Simpson().integrate(f, dim, N=n**dim, integration_domain=dom)
+    want = OGR.value_and_grad(f.family, np.concatenate([[np.float32(c), 0.0], a, u]), OGR.SIMPSON, dim, n, dom_l)
+    tol = 1e-10 if dtype == torch.float64 else 4.0 * 2.0**-24 * n * dim
+    for scale in (1.0, -2.5):
+        g = torch.autograd.grad(val, [dom, c_t, base, u_t], grad_outputs=torch.tensor(scale, dtype=val.dtype, device=cuda),
+                                retain_graph=True)
+        ga = g[2][:, 0] if where == "strided" else g[2]
+        assert [x.dtype for x in g] == [dtype, torch.float32, torch.float64, torch.float64]
+        assert all(x.device == t.device for x, t in zip(g, (dom, c_t, base, u_t)))
+        c_tol = max(tol, 2.0**-23)
+        got_par = np.concatenate([[0.0, 0.0], ga.detach().cpu().numpy(), g[3].cpu().numpy()]) / scale
+        want_par = np.concatenate([[0.0, 0.0], want[2][2:]])
+        _assert_gradients((val.item(), g[0].cpu().numpy() / scale, got_par), (want[0], want[1], want_par),
+                          tol, (where, dtype))
+        assert abs(g[1].item() / scale - want[2][0]) <= c_tol * abs(want[2][0])
+
+
+def test_parameters_written_between_calls(cuda):
+    """Parameters on the device, written in place or replaced: every call sees
+    the values of its time, also from another stream."""
+    a = torch.tensor([1.0, 2.0], dtype=torch.float64, device=cuda)
+    f = tq.ExpSum(2, a=a)
+    dom = [[0.0, 1.0], [0.0, 1.0]]
+    exact = lambda v: np.prod([(np.exp(x) - 1.0) / x for x in v])  # noqa: E731
+    run = lambda: integrate("gausslegendre", f, 2, 24**2, dom, torch.float64, cuda).item()  # noqa: E731
+    for v in ([1.0, 2.0], [0.5, 2.0], [0.5, 2.0], [1.5, 0.25]):
+        a.copy_(torch.tensor(v, dtype=torch.float64))
+        for _ in range(3):
+            assert abs(run() - exact(v)) <= 1e-12 * exact(v)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        a.mul_(2.0)
+        assert abs(run() - exact([3.0, 0.5])) <= 1e-11
+    torch.cuda.current_stream().wait_stream(s)
+    f.a = torch.tensor([0.7, 0.9], dtype=torch.float64, device=cuda)
+    assert abs(run() - exact([0.7, 0.9])) <= 1e-11

@@ -10,6 +10,7 @@ import threading
 from ctypes import POINTER, c_double, c_int, c_int64, c_size_t, c_uint64, c_void_p, c_char_p
 
 import torch
+import torch.autograd.forward_ad as fwAD
 
 from .build import lib_path
 
@@ -148,6 +149,14 @@ SIGNATURES = {
         [c_int, c_int, c_int, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
          c_void_p, c_void_p, c_void_p, c_size_t, c_void_p],
     ),
+    "tq_grid_vjp": (
+        c_int,
+        [c_int, c_int, c_int, c_int64, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int,
+         POINTER(c_void_p), POINTER(c_int), c_void_p, c_size_t, c_void_p],
+    ),
+    "tq_pack_params": (
+        c_int,
+        [c_int, POINTER(c_void_p), POINTER(c_int), POINTER(c_int64), POINTER(c_double), c_void_p, c_void_p]),
     "tq_batch_grid_adjoint_workspace_size": (c_size_t, [c_int64, c_int]),
     "tq_batch_grid_adjoint": (
         c_int,
@@ -308,6 +317,17 @@ def body_stream(device, avoid=()) -> torch.cuda.Stream:
         if s.cuda_stream not in taken:
             return s
     raise RuntimeError("no CUDA stream distinct from the capturing stream")
+
+
+def plain_tensor(t) -> bool:
+    """Whether t is an ordinary tensor (or parameter) with memory of its own,
+    outside every transform that follows torch operations (tracing, vmap and
+    other functorch levels, forward-mode derivatives), so that a kernel may
+    take the place of torch operations on it.  Gradients are the caller's to
+    look at."""
+    return (type(t) in (torch.Tensor, torch.nn.Parameter) and torch._C._has_storage(t)
+            and not torch.jit.is_tracing() and fwAD._current_level < 0
+            and torch._C._functorch.peek_interpreter_stack() is None)
 
 
 def dtype_code(dtype: torch.dtype) -> int:

@@ -435,29 +435,57 @@ __device__ void adj_accumulate(const AdjCtx<T, GL, DM>& c, int64_t first, int64_
 
 // The integral and its gradients from the reduced accumulators tot[2+4*dim]
 // (one warp, lane k on dimension k).
-template <typename D>
-__device__ void adj_outputs(const double* tot, int family, double c, const D* dom, int dim,
-                            double* out_value, double* out_gdom, double* out_gpar) {
+struct AdjPlain {  // every gradient, fp64, in the layouts of tq_grid_adjoint
+  double *value, *gdom, *gpar;
+  __device__ __forceinline__ void v(double x) const { *value = x; }
+  __device__ __forceinline__ void domain(int i, double x) const { gdom[i] = x; }
+  __device__ __forceinline__ void param(int i, int, double x) const { gpar[i] = x; }
+};
+// The gradients times that of the result, each into the tensor that wants it
+// (its own type; null: not wanted).
+struct AdjVjp {
+  const void* gout;
+  void* out[5];  // domain, c, b, a, u
+  int gout_dtype, dtype[5];
+  __device__ __forceinline__ void put(int t, int i, double x) const {
+    if (!out[t]) return;
+    const double v = (gout_dtype == TQ_F64 ? *(const double*)gout : (double)*(const float*)gout) * x;
+    if (dtype[t] == TQ_F64)
+      ((double*)out[t])[i] = v;
+    else
+      ((float*)out[t])[i] = (float)v;
+  }
+  __device__ __forceinline__ void v(double) const {}
+  __device__ __forceinline__ void domain(int i, double x) const { put(0, i, x); }
+  __device__ __forceinline__ void param(int i, int dim, double x) const {
+    if (i < 2)
+      put(1 + i, 0, x);
+    else if (i < 2 + dim)
+      put(3, i - 2, x);
+    else
+      put(4, i - 2 - dim, x);
+  }
+};
+template <typename D, typename Out>
+__device__ void adj_outputs(const double* tot, int family, double c, const D* dom, int dim, const Out& out) {
   const int k = threadIdx.x & 31;
   const double I = c * tot[0];
   if (k < dim) {
     const double L = (double)dom[2 * k + 1] - (double)dom[2 * k];
     const double sx = c * tot[2 + k], st = c * tot[2 + dim + k];
     const double q = I / L;
-    out_gdom[2 * k] = -q + (sx - st);
-    out_gdom[2 * k + 1] = q + st;
-    out_gpar[2 + k] = c * tot[2 + 2 * dim + k];
-    out_gpar[2 + dim + k] = c * tot[2 + 3 * dim + k];
+    out.domain(2 * k, -q + (sx - st));
+    out.domain(2 * k + 1, q + st);
+    out.param(2 + k, dim, c * tot[2 + 2 * dim + k]);
+    out.param(2 + dim + k, dim, c * tot[2 + 3 * dim + k]);
   }
   if (k == 0) {
-    *out_value = I;
-    out_gpar[0] = tot[0];
-    if (family == TQ_FN_EXP_SUM)
-      out_gpar[1] = c * tot[0];
-    else if (family == TQ_FN_OSCILLATORY)
-      out_gpar[1] = 2.0 * CUDART_PI * c * tot[1];
-    else
-      out_gpar[1] = 0.0;
+    out.v(I);
+    out.param(0, dim, tot[0]);
+    out.param(1, dim,
+              family == TQ_FN_EXP_SUM       ? c * tot[0]
+              : family == TQ_FN_OSCILLATORY ? 2.0 * CUDART_PI * c * tot[1]
+                                            : 0.0);
   }
 }
 
@@ -472,9 +500,16 @@ struct GradArgs {
   double* partials;  // [blocks][nacc]
   int64_t slots;     // 16-byte partials the workspace holds
   unsigned* ticket;
-  double* out_value;
-  double* out_gdom;  // [dim][2]
-  double* out_gpar;  // [2 + 2*dim]
+  int vjp;         // write through `prod` instead of `plain`
+  AdjPlain plain;  // value, [dim][2], [2 + 2*dim]
+  AdjVjp prod;
+  template <typename D>
+  __device__ __forceinline__ void outputs(const double* tot, int fam, double c) const {
+    if (vjp)
+      adj_outputs<D>(tot, fam, c, (const D*)domain, dim, prod);
+    else
+      adj_outputs<D>(tot, fam, c, (const D*)domain, dim, plain);
+  }
 };
 
 template <typename T, typename D, bool GL, int FAM, int DM>
@@ -500,8 +535,7 @@ __global__ void __launch_bounds__(kBlock) grid_adjoint_kernel(GradArgs args) {
         threadIdx.x < 32) {
       sep_adjoint<FAM, T>(dsum, fam.a, args.dim, tot);
       __syncwarp();
-      adj_outputs<D>(tot, FAM, (double)fam.c, (const D*)args.domain, args.dim, args.out_value, args.out_gdom,
-                     args.out_gpar);
+      args.outputs<D>(tot, FAM, (double)fam.c);
     }
     return;
   }
@@ -542,9 +576,7 @@ __global__ void __launch_bounds__(kBlock) grid_adjoint_kernel(GradArgs args) {
       if (lane == 0) tot[i] = a.s + a.c;
     }
     __syncthreads();
-    if (threadIdx.x < 32)
-      adj_outputs<D>(tot, FAM, (double)fam.c, (const D*)args.domain, dim, args.out_value, args.out_gdom,
-                     args.out_gpar);
+    if (threadIdx.x < 32) args.outputs<D>(tot, FAM, (double)fam.c);
     if (threadIdx.x == 0) *args.ticket = 0u;
   }
 }
@@ -757,8 +789,8 @@ __global__ void batch_adjoint_finalize_kernel(BatchGradArgs a, double* out_value
   }
   __syncwarp();
   const int fid = a.family >= 0 ? a.family : d.family;
-  adj_outputs<D>(tot[wib], fid, a.params[d.par_off], (const D*)a.domains + d.dom_off, d.dim, out_value + w,
-                 out_gdom + d.dom_off, out_gpar + d.par_off);
+  adj_outputs<D>(tot[wib], fid, a.params[d.par_off], (const D*)a.domains + d.dom_off, d.dim,
+                 AdjPlain{out_value + w, out_gdom + d.dom_off, out_gpar + d.par_off});
 }
 
 }  // namespace tq
@@ -790,16 +822,15 @@ extern "C" size_t tq_grid_adjoint_workspace_size(int dim, int64_t total_points) 
   return least > sep ? least : sep;
 }
 
-extern "C" int tq_grid_adjoint(int dtype, int rule, int dim, int64_t n_per_dim, const void* domain,
-                               const double* gl_nodes, const double* gl_weights, int family,
-                               const double* params, double* out_value, double* out_grad_domain,
-                               double* out_grad_params, void* workspace, size_t workspace_bytes,
-                               void* stream) {
+// plain or prod: where the results go.
+static int adjoint_launch(int dtype, int rule, int dim, int64_t n_per_dim, const void* domain,
+                          const double* gl_nodes, const double* gl_weights, int family, const double* params,
+                          const AdjPlain* plain, const AdjVjp* prod, void* workspace, size_t workspace_bytes,
+                          void* stream) {
   if (!valid_dtype(dtype)) return TQ_ERR_DTYPE;
   if (dim < 1 || dim > 8) return TQ_ERR_DIM;
   if (!valid_nc(rule, n_per_dim)) return TQ_ERR_RULE;
-  if (!domain || !params || !out_value || !out_grad_domain || !out_grad_params || !workspace)
-    return TQ_ERR_ARG;
+  if (!domain || !params || !workspace) return TQ_ERR_ARG;
   if (rule == TQ_RULE_GAUSS && (!gl_nodes || !gl_weights)) return TQ_ERR_ARG;
   int64_t total = 1;
   for (int k = 0; k < dim; ++k) {
@@ -824,9 +855,9 @@ extern "C" int tq_grid_adjoint(int dtype, int rule, int dim, int64_t n_per_dim, 
   a.ticket = (unsigned*)workspace;
   a.partials = (double*)((char*)workspace + 256);
   a.slots = (int64_t)((workspace_bytes - 256) / sizeof(Acc));
-  a.out_value = out_value;
-  a.out_gdom = out_grad_domain;
-  a.out_gpar = out_grad_params;
+  a.vjp = prod != nullptr;
+  a.plain = plain ? *plain : AdjPlain{};
+  a.prod = prod ? *prod : AdjVjp{};
   const dim3 grid((unsigned)blocks);
   cudaStream_t s = (cudaStream_t)stream;
 #define TQ_ADJ(DMV)                                                                      \
@@ -848,6 +879,83 @@ extern "C" int tq_grid_adjoint(int dtype, int rule, int dim, int64_t n_per_dim, 
     }
   });
 #undef TQ_ADJ
+  return launch_status();
+}
+
+extern "C" int tq_grid_adjoint(int dtype, int rule, int dim, int64_t n_per_dim, const void* domain,
+                               const double* gl_nodes, const double* gl_weights, int family,
+                               const double* params, double* out_value, double* out_grad_domain,
+                               double* out_grad_params, void* workspace, size_t workspace_bytes,
+                               void* stream) {
+  if (!valid_dtype(dtype)) return TQ_ERR_DTYPE;
+  if (dim < 1 || dim > 8) return TQ_ERR_DIM;
+  if (!valid_nc(rule, n_per_dim)) return TQ_ERR_RULE;
+  if (!out_value || !out_grad_domain || !out_grad_params) return TQ_ERR_ARG;
+  const AdjPlain plain{out_value, out_grad_domain, out_grad_params};
+  return adjoint_launch(dtype, rule, dim, n_per_dim, domain, gl_nodes, gl_weights, family, params, &plain, nullptr,
+                        workspace, workspace_bytes, stream);
+}
+
+extern "C" int tq_grid_vjp(int dtype, int rule, int dim, int64_t n_per_dim, const void* domain,
+                           const double* gl_nodes, const double* gl_weights, int family, const double* params,
+                           const void* grad_out, int grad_out_dtype, void* const* grads, const int* grad_dtypes,
+                           void* workspace, size_t workspace_bytes, void* stream) {
+  if (!grad_out || !grads || !grad_dtypes) return TQ_ERR_ARG;
+  if (!valid_dtype(grad_out_dtype)) return TQ_ERR_DTYPE;
+  AdjVjp prod;
+  prod.gout = grad_out;
+  prod.gout_dtype = grad_out_dtype;
+  for (int t = 0; t < 5; ++t) {
+    prod.out[t] = grads[t];
+    prod.dtype[t] = grad_dtypes[t];
+    if (grads[t] && !valid_dtype(grad_dtypes[t])) return TQ_ERR_DTYPE;
+  }
+  return adjoint_launch(dtype, rule, dim, n_per_dim, domain, gl_nodes, gl_weights, family, params, nullptr, &prod,
+                        workspace, workspace_bytes, stream);
+}
+
+// ------------------------------------------------------ parameter vectors
+// The fp64 parameter vector c, b, a[dim], u[dim] from tensors on the device
+// and values on the host, in one launch (reading device tensors back to build
+// it on the host cost a synchronisation each).
+namespace tq {
+struct PackArgs {
+  int dim;
+  const void* dev[4];  // c, b, a, u on the device, or null: the host's values
+  int dtype[4];
+  int64_t stride[4];
+  double host[2 + 2 * kMaxDim];
+  double* out;
+};
+__global__ void pack_params_kernel(PackArgs p) {
+  const int i = threadIdx.x, n = 2 + 2 * p.dim;
+  if (i >= n) return;
+  const int t = i < 2 ? i : (i < 2 + p.dim ? 2 : 3);
+  const int64_t e = t == 2 ? i - 2 : t == 3 ? i - 2 - p.dim : 0;
+  double v = p.host[i];
+  if (p.dev[t]) {
+    v = p.dtype[t] == TQ_F64 ? ((const double*)p.dev[t])[e * p.stride[t]]
+                             : (double)((const float*)p.dev[t])[e * p.stride[t]];
+  }
+  p.out[i] = v;
+}
+}  // namespace tq
+
+extern "C" int tq_pack_params(int dim, const void* const* dev, const int* dtypes, const int64_t* strides,
+                              const double* host, double* out, void* stream) {
+  if (dim < 1 || dim > kMaxDim) return TQ_ERR_DIM;
+  if (!dev || !dtypes || !strides || !host || !out) return TQ_ERR_ARG;
+  PackArgs p;
+  p.dim = dim;
+  p.out = out;
+  for (int t = 0; t < 4; ++t) {
+    p.dev[t] = dev[t];
+    p.dtype[t] = dtypes[t];
+    p.stride[t] = strides[t];
+    if (dev[t] && !valid_dtype(dtypes[t])) return TQ_ERR_DTYPE;
+  }
+  for (int i = 0; i < 2 + 2 * dim; ++i) p.host[i] = host[i];
+  pack_params_kernel<<<1, 64, 0, (cudaStream_t)stream>>>(p);
   return launch_status();
 }
 

@@ -21,6 +21,7 @@ selects the fused kernel, where no point tensor is materialised.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 
 import numpy as np
@@ -64,6 +65,7 @@ class BuiltinIntegrand:
         self._dev_params = {}
         self._np_key = None
         self._np = None
+        self._packed_key = None
         if not any(isinstance(v, torch.Tensor) for v in (a, u, b, c)):
             # plain numbers: the host vector without torch operations
             self._np = np.concatenate([[float(c), float(b)], self.a.numpy(), self.u.numpy()])
@@ -111,6 +113,40 @@ class BuiltinIntegrand:
         dev = torch.from_numpy(host).to(device, non_blocking=False)
         self._dev_params[key] = (host, dev)
         return dev
+
+    def launch_params(self, device) -> torch.Tensor:
+        """The device parameter vector for launches on the current stream.
+        Parameters that live on the device are gathered there by one launch;
+        reading them back would wait for everything queued before.  The
+        second call with the same parameters keeps the vector (device_params)."""
+        ts = (self.c, self.b, self.a, self.u)
+        if not any(t.is_cuda for t in ts):
+            return self.device_params(device)
+        key = self._params_key()
+        if key == self._np_key or key == self._packed_key or not self._packable(ts, device):
+            return self.device_params(device)
+        self._packed_key = key
+        host = [0.0] * (2 + 2 * self.dim)
+        at = (slice(0, 1), slice(1, 2), slice(2, 2 + self.dim), slice(2 + self.dim, 2 + 2 * self.dim))
+        for t, sl in zip(ts, at):
+            if not t.is_cuda:
+                host[sl] = t.detach().to(torch.float64).reshape(-1).tolist()
+        out = torch.empty(2 + 2 * self.dim, dtype=torch.float64, device=device)
+        L.check(
+            L.lib().tq_pack_params(
+                self.dim,
+                (ctypes.c_void_p * 4)(*[t.data_ptr() if t.is_cuda else None for t in ts]),
+                (ctypes.c_int * 4)(*[L.dtype_code(t.dtype) if t.is_cuda else 0 for t in ts]),
+                (ctypes.c_int64 * 4)(*[t.stride(0) if t.dim() else 0 for t in ts]),
+                (ctypes.c_double * len(host))(*host), out.data_ptr(), L.stream_handle()),
+            "tq_pack_params")
+        L.count_launches(1)
+        return out
+
+    def _packable(self, ts, device):
+        return self.dim <= L.TQ_MAX_DIM and all(
+            L.plain_tensor(t) and t.dtype in (torch.float32, torch.float64) and (t.device == device or t.device.type == "cpu")
+            and (t.numel() == 1 if i < 2 else t.shape == (self.dim,)) for i, t in enumerate(ts))
 
     # ---- torch evaluation (same operation order as the device functions)
     def _term(self, k, xk, a, u):

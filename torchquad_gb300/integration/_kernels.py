@@ -6,9 +6,9 @@ synchronising.  Scratch memory comes from a per-stream torch-owned workspace.
 from __future__ import annotations
 
 import os
+from ctypes import c_int, c_void_p
 
 import torch
-import torch.autograd.forward_ad as fwAD
 
 from .. import _lib as L
 
@@ -103,15 +103,6 @@ def weighted_result(rule, dim, n, domain, gl_weights, start, values2d, out_dtype
     return out
 
 
-def plain_tensor(t) -> bool:
-    """Whether t is an ordinary tensor outside every transform that follows
-    torch operations (tracing, vmap and other functorch levels, forward-mode
-    derivatives), so that a kernel may take the place of torch operations on
-    it.  Gradients are the caller's to look at."""
-    return (type(t) is torch.Tensor and not torch.jit.is_tracing() and fwAD._current_level < 0
-            and torch._C._functorch.peek_interpreter_stack() is None)
-
-
 def sample_points(seed, stream_id, offset, N, domain):
     """[N, dim] uniform points of the domain from the Philox stream."""
     dim = domain.shape[0]
@@ -154,9 +145,10 @@ class WeightedSum(torch.autograd.Function):
         return g, None, None, None, None, None, None
 
 
-def grid_fused(rule, dim, n, domain, gl_nodes, gl_weights, integrand, out_dtype):
+def grid_fused(rule, dim, n, domain, gl_nodes, gl_weights, integrand, out_dtype, params=None):
     out = torch.empty((), dtype=out_dtype, device=domain.device)
-    params = integrand.device_params(domain.device)
+    if params is None:
+        params = integrand.launch_params(domain.device)
     ws = L.workspace.get(L.lib().tq_grid_fused_workspace_size(rule, dim, n), "fused")
     L.check(
         L.lib().tq_grid_fused(
@@ -185,7 +177,7 @@ def uniform(seed, stream_id, offset, size, dtype, device):
 
 def mc_fused(dim, n_points, domain, integrand, seed, stream_id, offset):
     out = torch.empty((), dtype=domain.dtype, device=domain.device)
-    params = integrand.device_params(domain.device)
+    params = integrand.launch_params(domain.device)
     ws = L.workspace.get(L.lib().tq_mc_fused_workspace_size(dim, n_points), "fused")
     L.check(
         L.lib().tq_mc_fused(
@@ -199,13 +191,33 @@ def mc_fused(dim, n_points, domain, integrand, seed, stream_id, offset):
     return out
 
 
-def grid_adjoint(rule, dim, n, domain, gl_nodes, gl_weights, integrand):
+def grid_vjp(rule, dim, n, domain, gl_nodes, gl_weights, family, params, gout, wanted):
+    """gout times the gradient with respect to each tensor of wanted (domain,
+    c, b, a, u; None: not wanted), in the tensors' own types: one launch."""
+    grads = [None if t is None else torch.empty(t.shape, dtype=t.dtype, device=t.device) for t in wanted]
+    ptrs = (c_void_p * 5)(*[None if g is None else g.data_ptr() for g in grads])
+    types = (c_int * 5)(*[0 if g is None else L.dtype_code(g.dtype) for g in grads])
+    ws = L.workspace.get(L.lib().tq_grid_adjoint_workspace_size(dim, n**dim), "adjoint")
+    L.check(
+        L.lib().tq_grid_vjp(
+            L.dtype_code(domain.dtype), rule, dim, n, domain.data_ptr(), L.ptr(gl_nodes), L.ptr(gl_weights),
+            family, params.data_ptr(), gout.data_ptr(), L.dtype_code(gout.dtype), ptrs, types, ws.data_ptr(),
+            ws.numel(), L.stream_handle(),
+        ),
+        "tq_grid_vjp",
+    )
+    L.count_launches(1)
+    return grads
+
+
+def grid_adjoint(rule, dim, n, domain, gl_nodes, gl_weights, integrand, params=None):
     """(value, d/d domain [dim, 2], d/d params [2+2dim]) in fp64."""
     dev = domain.device
     val = torch.empty((), dtype=torch.float64, device=dev)
     gdom = torch.empty((dim, 2), dtype=torch.float64, device=dev)
     gpar = torch.empty((2 + 2 * dim,), dtype=torch.float64, device=dev)
-    params = integrand.device_params(dev)
+    if params is None:
+        params = integrand.launch_params(dev)
     ws = L.workspace.get(L.lib().tq_grid_adjoint_workspace_size(dim, n**dim), "adjoint")
     L.check(
         L.lib().tq_grid_adjoint(

@@ -156,8 +156,8 @@ class Gaussian(GridIntegrator):
         # scale the result by prod 0.5 (b - a) afterwards.
         return domain if self._rescales_nodes else self._unit_domain(domain)
 
-    def _integrate_fused(self, fn, dim, n, domain):
-        out = super()._integrate_fused(fn, dim, n, self._kernel_domain(domain))
+    def _integrate_fused(self, fn, dim, n, domain, params=None):
+        out = super()._integrate_fused(fn, dim, n, self._kernel_domain(domain), params)
         return out if self._rescales_nodes else out * self._weight_scale(domain, dim).to(out.dtype)
 
     def _integrate_materialised(self, fn, dim, n, domain):

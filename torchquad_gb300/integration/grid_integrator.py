@@ -56,24 +56,30 @@ class _FusedGridFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, domain, c, b, a, u, integ, fn, dim, n):
         ctx.integ, ctx.fn, ctx.dim, ctx.n = integ, fn, dim, n
-        ctx.save_for_backward(domain, c, b, a, u)
-        return integ._integrate_fused(fn, dim, n, domain.detach())
+        params = fn.launch_params(domain.device)
+        ctx.save_for_backward(domain, c, b, a, u, params)
+        return integ._integrate_fused(fn, dim, n, domain.detach(), params)
 
     @staticmethod
     def backward(ctx, gout):
-        domain, c, b, a, u = ctx.saved_tensors
+        *inputs, params = ctx.saved_tensors
         integ, fn, dim, n = ctx.integ, ctx.fn, ctx.dim, ctx.n
+        domain = inputs[0]
         gl_nodes, gl_w = integ._gl_tables(n, domain.device)
-        _, gdom, gpar = K.grid_adjoint(integ._rule, dim, n, domain.detach(), gl_nodes, gl_w, fn)
+        wanted = [t if need else None for t, need in zip(inputs, ctx.needs_input_grad)]
+        if gout.device == domain.device and L.plain_tensor(gout) and all(
+                t is None or (t.device == domain.device and t.dtype in (torch.float32, torch.float64))
+                for t in wanted):
+            grads = K.grid_vjp(integ._rule, dim, n, domain.detach(), gl_nodes, gl_w, fn.family, params, gout, wanted)
+            return (*grads, None, None, None, None)
+        _, gdom, gpar = K.grid_adjoint(integ._rule, dim, n, domain.detach(), gl_nodes, gl_w, fn, params)
         g = gout.detach().to(torch.float64)
 
         def back(t, grad):
-            if t is None or not t.requires_grad:
-                return None
-            return (g * grad).reshape(t.shape).to(t.device, t.dtype)
+            return None if t is None else (g * grad).reshape(t.shape).to(t.device, t.dtype)
 
-        return (back(domain, gdom), back(c, gpar[0]), back(b, gpar[1]), back(a, gpar[2 : 2 + dim]),
-                back(u, gpar[2 + dim : 2 + 2 * dim]), None, None, None, None)
+        each = (gdom, gpar[0], gpar[1], gpar[2 : 2 + dim], gpar[2 + dim : 2 + 2 * dim])
+        return (*(back(t, x) for t, x in zip(wanted, each)), None, None, None, None)
 
 
 class GridIntegrator(BaseIntegrator):
@@ -186,9 +192,9 @@ class GridIntegrator(BaseIntegrator):
         return (isinstance(fn, BuiltinIntegrand) and fn.dim == dim and dim <= 8
                 and getattr(self, "_rescales_nodes", True))
 
-    def _integrate_fused(self, fn, dim, n, domain):
+    def _integrate_fused(self, fn, dim, n, domain, params=None):
         gl_nodes, gl_w = self._gl_tables(n, domain.device)
-        return K.grid_fused(self._rule, dim, n, domain, gl_nodes, gl_w, fn, self._result_dtype(domain))
+        return K.grid_fused(self._rule, dim, n, domain, gl_nodes, gl_w, fn, self._result_dtype(domain), params)
 
     def _integrate_materialised(self, fn, dim, n, domain):
         total = n**dim

@@ -91,7 +91,7 @@ class MonteCarlo(BaseIntegrator):
             and domain.shape[1] == 2
             and 1 <= domain.shape[0] <= L.TQ_MAX_DIM
             and not (torch.is_grad_enabled() and domain.requires_grad)
-            and K.plain_tensor(domain)
+            and L.plain_tensor(domain)
         )
 
     def get_jit_compiled_integrate(self, dim, N=1000, integration_domain=None, seed=None, backend=None):
