@@ -281,6 +281,10 @@ int tq_finalize_sum(int dtype, int rule, int dim, const void* domain,
                     int64_t n_points, const double* acc, int64_t n_values,
                     void* out, int out_dtype, void* stream);
 
+/* domain[dim][2] (device, dtype) from host values (2*dim doubles, rounded to
+ * dtype), as launch arguments. */
+int tq_write_domain(int dtype, int dim, const double* values, void* domain, void* stream);
+
 /* Monte Carlo points (monte_carlo.py:84-106): points[count][dim] (dtype) =
  * u * (b - a) + a, u the elements 0 .. count*dim-1 of tq_uniform's stream from
  * block offset `offset`; the product and the sum rounded one after the other

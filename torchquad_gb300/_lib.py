@@ -194,6 +194,7 @@ SIGNATURES = {
     ),
     "tq_sample_points": (
         c_int, [c_int, c_int, c_int64, c_void_p, c_uint64, c_uint64, c_uint64, c_void_p, c_void_p]),
+    "tq_write_domain": (c_int, [c_int, c_int, POINTER(c_double), c_void_p, c_void_p]),
     "tq_finalize_sum": (
         c_int,
         [c_int, c_int, c_int, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int, c_void_p],
@@ -291,18 +292,29 @@ def check(status: int, where: str) -> None:
         raise TorchquadGB300Error(status, where)
 
 
+# Devices found usable, by index (a device does not go away again).
+_devices = {}
+
+
 def require_cuda() -> torch.device:
-    if not torch.cuda.is_available():
+    """The current CUDA device; raises where there is none."""
+    if not _devices and not torch.cuda.is_available():
         raise RuntimeError(
             "torchquad_gb300 runs its integration kernels on a CUDA device only "
             "and no CUDA device is available (there is no CPU fallback)."
         )
     lib()
-    return torch.device("cuda", torch.cuda.current_device())
+    index = torch.cuda.current_device()
+    device = _devices.get(index)
+    if device is None:
+        device = _devices[index] = torch.device("cuda", index)
+    return device
 
 
 def stream_handle() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device as a cudaStream_t (the raw
+    handle: torch.cuda.current_stream() builds a Stream object, 4 us)."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def body_stream(device, avoid=()) -> torch.cuda.Stream:
@@ -350,7 +362,7 @@ class _Workspace:
 
     def get(self, nbytes: int, slot: str = "main") -> torch.Tensor:
         dev = torch.cuda.current_device()
-        key = (dev, torch.cuda.current_stream().cuda_stream, slot)
+        key = (dev, torch._C._cuda_getCurrentRawStream(dev), slot)
         buf = self._bufs.get(key)
         if buf is None or buf.numel() < nbytes:
             # tickets in the first 16 bytes must start at zero

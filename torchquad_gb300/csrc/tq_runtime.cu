@@ -64,3 +64,29 @@ extern "C" const char* tq_status_string(int status) {
 extern "C" int tq_last_cuda_error(void) { return tq::g_last_cuda_error; }
 
 extern "C" int tq_device_sm_count(void) { return tq::sm_count(); }
+
+// ------------------------------------------------- domains of host values
+namespace tq {
+struct DomainArgs {
+  double v[2 * kMaxDim];
+};
+template <typename T>
+__global__ void write_domain_kernel(DomainArgs a, int n, T* out) {
+  if (threadIdx.x < n) out[threadIdx.x] = (T)a.v[threadIdx.x];
+}
+}  // namespace tq
+
+extern "C" int tq_write_domain(int dtype, int dim, const double* values, void* domain, void* stream) {
+  using namespace tq;
+  if (!valid_dtype(dtype)) return TQ_ERR_DTYPE;
+  if (dim < 1 || dim > kMaxDim) return TQ_ERR_DIM;
+  if (!values || !domain) return TQ_ERR_ARG;
+  DomainArgs a;
+  for (int i = 0; i < 2 * dim; ++i) a.v[i] = values[i];
+  cudaStream_t s = (cudaStream_t)stream;
+  if (dtype == TQ_F64)
+    write_domain_kernel<double><<<1, 32, 0, s>>>(a, 2 * dim, (double*)domain);
+  else
+    write_domain_kernel<float><<<1, 32, 0, s>>>(a, 2 * dim, (float*)domain);
+  return launch_status();
+}

@@ -7,6 +7,7 @@ current CUDA device, where every kernel of this package runs.
 """
 from __future__ import annotations
 
+import ctypes
 import warnings
 import weakref
 
@@ -98,7 +99,17 @@ def _setup_integration_domain(dim, integration_domain, backend):
         if hasattr(integration_domain, "__array__") and not isinstance(integration_domain, (list, tuple)):
             integration_domain = integration_domain.tolist()
         values = [[float(b) for b in bounds] for bounds in integration_domain]
-        t = torch.tensor(values, dtype=torch.get_default_dtype())
+        dtype = torch.get_default_dtype()
+        if (dtype in (torch.float32, torch.float64) and len(values) == dim <= L.TQ_MAX_DIM
+                and all(len(v) == 2 for v in values)):
+            # as launch arguments: a copy from the host waits for its staging
+            t = torch.empty((dim, 2), dtype=dtype, device=device)
+            flat = (ctypes.c_double * (2 * dim))(*[b for v in values for b in v])
+            L.check(L.lib().tq_write_domain(L.dtype_code(dtype), dim, flat, t.data_ptr(), L.stream_handle()),
+                    "tq_write_domain")
+            L.count_launches(1)
+            return t
+        t = torch.tensor(values, dtype=dtype)
         if t.shape != (dim, 2):
             raise ValueError(
                 "The integration domain has an unexpected shape. "
@@ -171,5 +182,6 @@ def _assemble_result(flat, shape, is_complex):
     is_1d = len(shape) == 0 or (len(shape) == 1 and shape[0] == 1)
     if is_1d:
         _warn_1d_result()
-        out = out.squeeze()
+        if out.dim():
+            out = out.squeeze()
     return out

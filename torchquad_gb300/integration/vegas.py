@@ -259,7 +259,7 @@ class VEGAS(BaseIntegrator):
             plan = _FusedPlan.get(
                 lambda: VegasDevice(dim, self.dtype, N_intervals, n_strat, device, domain,
                                     stats_slots=max_iterations + 10),
-                (str(device), torch.cuda.current_stream().cuda_stream, dim, self.dtype,
+                (str(device), L.stream_handle(), dim, self.dtype,
                  N_intervals, n_strat), fn.family,
                 use_grid_improve, use_warmup, ns, self._N_increment, max_iterations, self)
             self._dev = plan.dev
