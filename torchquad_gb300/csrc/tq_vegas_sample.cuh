@@ -150,7 +150,7 @@ constexpr int kWarps = kTile / 32;
 __host__ __device__ inline size_t sample_smem_bytes(int d, int64_t B, size_t tsize, bool hist,
                                                     bool edges) {
   size_t off = 0;
-  if (edges) off += tsize * (d * (B + 1) + d * B);
+  if (edges) off += ((tsize * (d * (B + 1)) + 15) & ~size_t(15)) + tsize * (d * B);
   off = (off + 15) & ~size_t(15);
   if (hist) off += (size_t)kWarps * d * B * (tsize + sizeof(unsigned));  // HistT<T> weight, u32 count
   return off;
@@ -164,7 +164,7 @@ __device__ Smem<T> carve(unsigned char* base, const SampleArgs& a) {
   size_t off = 0;
   if (a.edges_smem) {
     s.xe = (T*)(base + off);
-    off += sizeof(T) * d * (B + 1);
+    off += (sizeof(T) * d * (B + 1) + 15) & ~size_t(15);
     s.dxe = (T*)(base + off);
     off += sizeof(T) * d * B;
   } else {
@@ -181,6 +181,32 @@ __device__ Smem<T> carve(unsigned char* base, const SampleArgs& a) {
     s.hc = nullptr;
   }
   return s;
+}
+
+// Static shared memory of the sampler, declared once per kernel (a kernel that
+// holds several instantiations of the body would otherwise hold one each).
+template <typename T>
+struct SampleStatic {
+  Family<T> fam;
+  T lo[kMaxDim], wid[kMaxDim];
+  T volume;
+};
+
+// n values from global to shared memory by the CTA, 16 bytes a load and
+// several loads in flight where both addresses allow (a batch's CTA takes
+// 512 points, and copying a map of 1000 intervals value by value took it
+// longer than the points).
+template <typename T>
+__device__ __forceinline__ void copy_in(T* __restrict__ dst, const T* __restrict__ src, int n) {
+  constexpr int V = 16 / sizeof(T);
+  int done = 0;
+  if (((uintptr_t)src & 15) == 0) {  // dst is 16-byte aligned
+    const int nv = n / V;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < nv; i += kTile) ((uint4*)dst)[i] = ((const uint4*)src)[i];
+    done = nv * V;
+  }
+  for (int i = done + threadIdx.x; i < n; i += kTile) dst[i] = src[i];
 }
 
 // Warp-private histogram update without atomics: lanes with the same key
@@ -256,12 +282,13 @@ struct DrawBlocks {
 // The sampler as a device body: CTA bid of nblk CTAs taking part (the
 // per-launch kernel below, or one state's share of a batched launch).
 template <typename T, int FAM, bool WARM, int D>
-__device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk) {
+__device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk, SampleStatic<T>& ss) {
   constexpr int KD = D > 0 ? D : kMaxDim;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ Family<T> fam;
-  __shared__ T lo[kMaxDim], wid[kMaxDim];
-  __shared__ T volume;
+  Family<T>& fam = ss.fam;
+  T* const lo = ss.lo;
+  T* const wid = ss.wid;
+  T& volume = ss.volume;
   using H = typename HistT<T>::type;  // fp32 on the fp32 path
   const tq_vegas_state& st = a.st;
   const int d = D > 0 ? D : st.dim;
@@ -284,14 +311,12 @@ __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk) {
     if (k == 0) volume = v;
   }
   if (a.edges_smem) {
-    for (int64_t i = threadIdx.x; i < d * (B + 1); i += blockDim.x) sm.xe[i] = ((const T*)st.x_edges)[i];
-    for (int64_t i = threadIdx.x; i < DB; i += blockDim.x) sm.dxe[i] = ((const T*)st.dx_edges)[i];
+    copy_in(sm.xe, (const T*)st.x_edges, (int)(d * (B + 1)));
+    copy_in(sm.dxe, (const T*)st.dx_edges, (int)DB);
   }
-  if (a.hist_smem) {
-    for (int64_t i = threadIdx.x; i < (int64_t)kWarps * DB; i += blockDim.x) {
-      sm.hw[i] = 0;
-      sm.hc[i] = 0u;
-    }
+  if (a.hist_smem) {  // weights and counts, contiguous from a 16-byte boundary
+    const int bytes = (int)(kWarps * DB) * (int)(sizeof(H) + sizeof(unsigned));
+    for (int i = threadIdx.x; i < bytes / 16; i += kTile) ((uint4*)sm.hw)[i] = make_uint4(0, 0, 0, 0);
   }
 
   const int64_t M = WARM ? a.n_samples : __ldcg(st.cube_start + st.n_cubes);
@@ -484,7 +509,8 @@ __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk) {
 
 template <typename T, int FAM, bool WARM, int D>
 __global__ void __launch_bounds__(kTile, TQ_SAMPLE_MIN_BLOCKS) vegas_sample_kernel(SampleArgs a) {
-  sample_body<T, FAM, WARM, D>(a, blockIdx.x, gridDim.x);
+  __shared__ SampleStatic<T> ss;
+  sample_body<T, FAM, WARM, D>(a, blockIdx.x, gridDim.x, ss);
 }
 
 // fp32 states with 1 <= dim <= 8: the dimension-specialised sampler
