@@ -33,6 +33,10 @@ constexpr int64_t kBatchInitCtas = 64;
 // fit an SM's 228 KB.
 constexpr size_t kBatchSampleSmem = 56 * 1024;
 constexpr size_t kBatchSampleSmemF64 = 72 * 1024;
+// Resident map-row CTAs per SM of the fp32 batched launches (40 registers, 48
+// bytes spilled; the row's body alone takes 68, three CTAs): 256 states, a
+// graph of 15 iterations 2427 us with five, 2401 with six, 2404 with eight.
+constexpr int kBatchRowCtas = 6;
 
 // One state of the batch: the arguments of every phase body, built on the
 // host by the same helpers the single-state launchers use.
@@ -123,7 +127,8 @@ __device__ __forceinline__ void batch_map_row(const BatchEntry& e, double alpha,
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kRowThreads) vegas_batch_map_kernel(BatchLaunch L) {
+__global__ void __launch_bounds__(kRowThreads, std::is_same<T, float>::value ? kBatchRowCtas : 1)
+    vegas_batch_map_kernel(BatchLaunch L) {
   const uint2 m = L.map[blockIdx.x];
   const BatchEntry& e = L.e[m.x];
   batch_map_row<T>(e, L.alpha, (int)m.y, (unsigned)e.ctas[TQ_VB_MAP]);
@@ -140,7 +145,8 @@ __global__ void __launch_bounds__(kBlock) vegas_batch_nh_kernel(BatchLaunch L) {
 // CTAs [0, map_rows) of a state update its map rows, the others end its
 // iteration (the two touch disjoint parts of the state).
 template <typename T>
-__global__ void __launch_bounds__(kBlock) vegas_batch_finish_kernel(BatchLaunch L) {
+__global__ void __launch_bounds__(kBlock, std::is_same<T, float>::value ? kBatchRowCtas : 1)
+    vegas_batch_finish_kernel(BatchLaunch L) {
   const uint2 m = L.map[blockIdx.x];
   const BatchEntry& e = L.e[m.x];
   if (batch_stopped(e)) return;

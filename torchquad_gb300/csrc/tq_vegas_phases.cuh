@@ -285,13 +285,24 @@ static __device__ void finish_f32_body(const FinishArgs& a, unsigned bid, unsign
   }
   if (last_block_of(a.ticket, nblk) && warp == 0) {
     F2 r{0.f, 0.f}, q{0.f, 0.f}, ds{0.f, 0.f};
-    for (unsigned i = lane; i < nblk; i += 32) {  // fixed assignment and tree: deterministic
-      const float2 pr = __ldcg((const float2*)&part[6 * i]);
-      const float2 pq = __ldcg((const float2*)&part[6 * i + 2]);
-      const float2 pd = __ldcg((const float2*)&part[6 * i + 4]);
-      r = f2_add(r, F2{pr.x, pr.y});
-      q = f2_add(q, F2{pq.x, pq.y});
-      ds = f2_add(ds, F2{pd.x, pd.y});
+    // fixed assignment and tree: deterministic; four blocks' loads in flight
+    for (unsigned i0 = lane; i0 < nblk; i0 += 128) {
+      float2 pr[4], pq[4], pd[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const unsigned i = min(i0 + 32u * j, nblk - 1u);
+        pr[j] = __ldcg((const float2*)&part[6 * i]);
+        pq[j] = __ldcg((const float2*)&part[6 * i + 2]);
+        pd[j] = __ldcg((const float2*)&part[6 * i + 4]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (i0 + 32u * j < nblk) {
+          r = f2_add(r, F2{pr[j].x, pr[j].y});
+          q = f2_add(q, F2{pq[j].x, pq[j].y});
+          ds = f2_add(ds, F2{pd[j].x, pd[j].y});
+        }
+      }
     }
     f2_warp_sum3(r, q, ds);
     if (lane == 0) {
@@ -371,19 +382,158 @@ static __device__ __forceinline__ double cta_exclusive_scan(double x, double* sh
 // map: the weights are sums of squares, so a row of averaged (and filled)
 // weights sums to zero exactly when each of its averages is zero.  Since
 // every CTA reads every row, the weights and counts are cleared by the last
-// CTA to finish (ticket), not by each CTA for its own row.
+// CTA to have read them (ticket), not by each CTA for its own row.
 constexpr int kRowThreads = 256;
 constexpr int kRowPer = kSmallMap / kRowThreads;  // consecutive intervals per thread in the scans
 
 inline size_t map_row_smem(int64_t B, size_t ts) {
-  return (((7 * B + 3) * ts + (2 * B + 1) * 4 + 2 * B) + 15) & ~size_t(15);
+  return (((5 * B + 3) * ts + (2 * B + 1) * 4 + 2 * B) + 15) & ~size_t(15);
 }
 
-// The last CTA to arrive resets the weights and counts of the whole map
-// (_reset_weight).  Every CTA read the whole map's weights and counts; the
-// fenced ticket (last_block_of) orders those reads before the reset.
-static __device__ void clear_map_by_last(const tq_vegas_state& st, unsigned* ticket, unsigned nrows) {
-  if (last_block_of(ticket, nrows)) {
+// What bounds a row's update is the latency of its serial parts, 256 threads
+// to a row and no bandwidth to speak of: the loads of a row go out together,
+// the helpers below replace loops that took one dependent load or barrier at
+// a time, and the ticket is drawn when the row has been read, so that its
+// round trip runs beside the update.  The 256 states of a batch
+// (d 1-10, 60 to 1000 intervals): 36.5 -> 29.5 us a warm-up's update, 40 -> 33.5
+// an iteration's end; what is left hardly changes with the resident CTAs
+// (kBatchRowCtas), so it is issue, the double-float trees and scans.  One
+// state of d = 6 with 50 intervals: as before (675-683 us a run of 1e7 points).
+
+// rownz[kk] = 1 for each row with a nonzero average; half a warp to a row, so
+// that the rows' loads are in flight together (16 intervals of a row decide
+// it as a rule, and going on row by row waited for each).
+template <typename T>
+static __device__ __forceinline__ void find_nonzero_rows(const tq_vegas_state& st, int* rownz) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int d = st.dim, B = (int)st.n_bins;
+  for (int kb = 2 * warp; kb < d; kb += 2 * (kRowThreads / 32)) {
+    const int kk = kb + (lane >> 4);
+    bool found = kk >= d;
+    for (int base = 0; base < B; base += 16) {
+      const int b = base + (lane & 15);
+      bool nz = false;
+      if (!found && b < B) {
+        const int64_t c = st.counts[(int64_t)kk * B + b];
+        const T wi = (T)st.weights[(int64_t)kk * B + b];
+        nz = (c == 0 ? wi : div_rn(wi, (T)c)) != (T)0;
+      }
+      found |= ((__ballot_sync(0xffffffffu, nz) >> (lane & 16)) & 0xffffu) != 0u;
+      if (__all_sync(0xffffffffu, found)) break;
+    }
+    if (kk < d && (lane & 15) == 0) rownz[kk] = found;
+  }
+}
+
+// ind[e] = #{b : mk[b] <= e} of the runs of equal multiples, and vv[q] = the
+// sequential sum of sw over the run of multiple q (:214-230).  A long span of
+// ind is written by the warp, a long run is read eight intervals at a time
+// (the sum itself stays in order).
+template <typename T>
+static __device__ __forceinline__ void map_runs(const int32_t* mk, const T* sw, int B, int32_t* ind, T* vv) {
+  const int lane = threadIdx.x & 31;
+  for (int base = 0; base < B; base += kRowThreads) {
+    const int b = base + threadIdx.x;
+    int from = 0, to = 0;
+    if (b < B) {
+      from = b == 0 ? 0 : mk[b - 1];
+      to = b == B - 1 ? B + 1 : mk[b];
+      const int first = min(to, from + 4);
+      for (int e = from; e < first; ++e) ind[e] = b;
+    }
+    from += 4;
+    for (unsigned m = __ballot_sync(0xffffffffu, from < to); m; m &= m - 1u) {
+      const int src = __ffs(m) - 1;
+      const int f = __shfl_sync(0xffffffffu, from, src), t = __shfl_sync(0xffffffffu, to, src);
+      for (int e = f + lane; e < t; e += 32) ind[e] = base + (threadIdx.x & ~31) + src;
+    }
+    if (b < B - 1 && (b == 0 || mk[b] != mk[b - 1])) {
+      const int q = mk[b];
+      T a = add_rn((T)0, sw[b]);
+      int e = b + 1;
+      bool in = e < B - 1 && mk[e] == q;
+      while (in) {
+        int32_t m[8];
+        T v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int i = min(e + j, B - 2);
+          m[j] = mk[i];
+          v[j] = sw[i];
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          in = in && e + j < B - 1 && m[j] == q;
+          if (in) a = add_rn(a, v[j]);
+        }
+        e += 8;
+      }
+      vv[q] = a;
+    }
+  }
+}
+
+// Ten sweeps of the filling of empty intervals (:118-145); anyz: this thread
+// holds an empty interval, odd: one whose average is not +0.  A sweep fills
+// the last empty interval of a run from its right neighbour, then the first
+// one from its left neighbour, so after ten the intervals up to ten places
+// from an end of a run hold the average beyond the nearer end (the right one
+// of two equally near) and the others are as they were, +0: written at once.
+// Averages other than +0 in empty intervals are moved about by the sweeps;
+// those are run as they stand.
+template <typename T>
+static __device__ __forceinline__ void fill_empty(T* w, T* wt, unsigned char* z, unsigned char* zt, int B, int anyz,
+                                                  int odd) {
+  if (!__syncthreads_or(anyz)) return;  // also publishes w and z
+  if (!__syncthreads_or(odd)) {
+    for (int b = threadIdx.x; b < B; b += blockDim.x) {
+      if (!z[b]) continue;
+      int l = 0, r = 0;
+#pragma unroll
+      for (int i = 10; i > 0; --i) {
+        if (b + i < B && !z[min(b + i, B - 1)]) r = i;
+        if (b - i >= 0 && !z[max(b - i, 0)]) l = i;
+      }
+      if (r && (!l || r <= l))
+        w[b] = w[b + r];
+      else if (l)
+        w[b] = w[b - l];
+    }
+    __syncthreads();
+    return;
+  }
+  for (int sweep = 0; sweep < 10; ++sweep) {
+    for (int b = threadIdx.x; b < B; b += blockDim.x) {
+      wt[b] = (b < B - 1 && z[b]) ? w[b + 1] : w[b];
+      zt[b] = (b < B - 1) ? (z[b] && z[b + 1]) : z[b];
+    }
+    __syncthreads();
+    int left = 0;
+    for (int b = threadIdx.x; b < B; b += blockDim.x) {
+      w[b] = (b > 0 && zt[b]) ? wt[b - 1] : wt[b];
+      z[b] = (b > 0) ? (zt[b] && zt[b - 1]) : zt[b];
+      left |= z[b];
+    }
+    if (!__syncthreads_or(left)) break;
+  }
+}
+
+// The last CTA that has read the map resets the weights and counts of the
+// whole map (_reset_weight).  Every CTA reads all of them: draw_clear after
+// the barrier that ends its reads (thread 0's ticket, fenced), clear_map_if
+// at its end.
+static __device__ __forceinline__ unsigned draw_clear(unsigned* ticket) {
+  unsigned t = 0;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    t = atomicAdd(ticket, 1u);
+  }
+  return t;
+}
+static __device__ __forceinline__ void clear_map_if(const tq_vegas_state& st, unsigned* ticket, unsigned nrows,
+                                                    unsigned t) {
+  if (threadIdx.x == 0 && t == nrows - 1) __threadfence();
+  if (__syncthreads_or(threadIdx.x == 0 && t == nrows - 1)) {
     const int64_t n = (int64_t)st.dim * st.n_bins;
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
       st.weights[i] = 0.0;
@@ -401,63 +551,39 @@ static __device__ void map_rows_body(const tq_vegas_state& st, double alpha, voi
   __shared__ int rownz[kMaxDim];
   const int d = st.dim;
   const int B = (int)st.n_bins;
-  T* w = (T*)row_smem;                                 // [B] averaged, filled weights
-  T* wt = w + B;                                       // [B]
-  T* sw = wt + B;                                      // [B] smoothed weights
+  T* sw = (T*)row_smem;                                // [B] smoothed weights
   T* vv = sw + B;                                      // [B+1] sums per delta multiple
   T* nx = vv + (B + 1);                                // [B+1] new edges
+  T* w = vv;                                           // [B] averaged, filled weights (until sw is taken)
+  T* wt = nx;                                          // [B]
   int32_t* mk = (int32_t*)(nx + (B + 1));              // [B] delta multiples
   int32_t* ind = mk + B;                               // [B+1] old interval per new edge
   unsigned char* z = (unsigned char*)(ind + (B + 1));  // [B] empty intervals
   unsigned char* zt = z + B;                           // [B]
-  // zero-row test over the whole map; a row's remaining averages are
-  // skipped once some thread has found a nonzero one (the flag only ever
-  // goes from 0 to 1, so the outcome is the same)
-  if (threadIdx.x < d) rownz[threadIdx.x] = 0;
-  __syncthreads();
-  volatile int* rnz = rownz;
-  for (int kk = 0; kk < d; ++kk) {
-    for (int b = threadIdx.x; b < B && !rnz[kk]; b += blockDim.x) {
-      const int64_t c = st.counts[(int64_t)kk * B + b];
-      const T wi = (T)st.weights[(int64_t)kk * B + b];
-      if ((c == 0 ? wi : div_rn(wi, (T)c)) != (T)0) rnz[kk] = 1;
-    }
-  }
-  __syncthreads();
-  int zero_row = 0;
-  for (int kk = 0; kk < d; ++kk) zero_row |= !rownz[kk];
-  if (zero_row) {  // the map cannot be updated (:187-196): only the reset
-    if (k == 0 && threadIdx.x == 0) atomicAdd(st.flags + 0, 1);
-    if (!smooth_out) clear_map_by_last(st, ticket, nrows);
-    return;
-  }
-  // EQ 17 and the filling of empty intervals (:118-145).  A sweep over a row
-  // without empty intervals changes nothing, so stopping per row gives the
-  // reference's map-wide stopping rule.
-  int anyz = 0;
+  // EQ 17, and the zero-row test over the whole map
+  int anyz = 0, odd = 0;
   for (int b = threadIdx.x; b < B; b += blockDim.x) {
     const int64_t c = st.counts[(int64_t)k * B + b];
     const T wi = (T)st.weights[(int64_t)k * B + b];
     z[b] = c == 0;
     anyz |= c == 0;
+    odd |= c == 0 && (wi != (T)0 || signbit(wi));
     w[b] = c == 0 ? wi : div_rn(wi, (T)c);
   }
-  if (__syncthreads_or(anyz)) {
-    for (int sweep = 0; sweep < 10; ++sweep) {
-      for (int b = threadIdx.x; b < B; b += blockDim.x) {
-        wt[b] = (b < B - 1 && z[b]) ? w[b + 1] : w[b];
-        zt[b] = (b < B - 1) ? (z[b] && z[b + 1]) : z[b];
-      }
-      __syncthreads();
-      int left = 0;
-      for (int b = threadIdx.x; b < B; b += blockDim.x) {
-        w[b] = (b > 0 && zt[b]) ? wt[b - 1] : wt[b];
-        z[b] = (b > 0) ? (zt[b] && zt[b - 1]) : zt[b];
-        left |= z[b];
-      }
-      if (!__syncthreads_or(left)) break;
-    }
+  find_nonzero_rows<T>(st, rownz);
+  __syncthreads();
+  const unsigned turn = smooth_out ? 0u : draw_clear(ticket);
+  int zero_row = 0;
+  for (int kk = 0; kk < d; ++kk) zero_row |= !rownz[kk];
+  if (zero_row) {  // the map cannot be updated (:187-196): only the reset
+    if (k == 0 && threadIdx.x == 0) atomicAdd(st.flags + 0, 1);
+    if (!smooth_out) clear_map_if(st, ticket, nrows, turn);
+    return;
   }
+  // The filling of empty intervals.  A sweep over a row without empty
+  // intervals changes nothing, so stopping per row gives the reference's
+  // map-wide stopping rule.
+  fill_empty<T>(w, wt, z, zt, B, anyz, odd);
   double acc = 0.0;
   for (int b = threadIdx.x; b < B; b += blockDim.x) acc += (double)w[b];
   const T sum = (T)block_sum_all(acc, red);  // :151
@@ -505,19 +631,7 @@ static __device__ void map_rows_body(const tq_vegas_state& st, double alpha, voi
     ind[e] = 0;
   }
   __syncthreads();
-  // :214-230 from the runs of equal multiples: ind[e] = #{b : mk[b] <= e},
-  // vv[q] = the sequential sum of sw over the run of multiple q
-  for (int b = threadIdx.x; b < B; b += blockDim.x) {
-    const int from = b == 0 ? 0 : mk[b - 1];
-    const int to = b == B - 1 ? B + 1 : mk[b];
-    for (int e = from; e < to; ++e) ind[e] = b;
-    if (b < B - 1 && (b == 0 || mk[b] != mk[b - 1])) {
-      const int q = mk[b];
-      T a = (T)0;
-      for (int e = b; e < B - 1 && mk[e] == q; ++e) a = add_rn(a, sw[e]);
-      vv[q] = a;
-    }
-  }
+  map_runs<T>(mk, sw, B, ind, vv);
   __syncthreads();
   // :233 d_accu (fp64 cumulative sum rounded to T per element) and EQ 22
   const T* xe = (const T*)st.x_edges + (int64_t)k * (B + 1);
@@ -565,7 +679,7 @@ static __device__ void map_rows_body(const tq_vegas_state& st, double alpha, voi
   T* dxo = (T*)st.dx_edges + (int64_t)k * B;
   for (int e = threadIdx.x; e <= B; e += blockDim.x) xo[e] = nx[e];
   for (int b = threadIdx.x; b < B; b += blockDim.x) dxo[b] = sub_rn(nx[b + 1], nx[b]);  // :259
-  clear_map_by_last(st, ticket, nrows);
+  clear_map_if(st, ticket, nrows, turn);
 }
 
 
@@ -577,7 +691,8 @@ static __device__ void map_rows_body(const tq_vegas_state& st, double alpha, voi
 // as a TwoProduct): multiples agree with the fp64 truncation except where
 // C / delta lies within about 2^-46 of an integer without being one.
 static __device__ F2 f2_block_sum_all(F2 v, F2* sh) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  constexpr int nw = kRowThreads / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = f2_add(v, f2_shfl_down(v, o));
   __syncthreads();
@@ -586,7 +701,7 @@ static __device__ F2 f2_block_sum_all(F2 v, F2* sh) {
   if (warp == 0) {  // the warp partials in a fixed tree
     F2 t = lane < nw ? sh[lane] : F2{0.f, 0.f};
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t = f2_add(t, f2_shfl_down(t, o));
+    for (int o = nw / 2; o > 0; o >>= 1) t = f2_add(t, f2_shfl_down(t, o));
     if (lane == 0) sh[32] = t;
   }
   __syncthreads();
@@ -594,7 +709,8 @@ static __device__ F2 f2_block_sum_all(F2 v, F2* sh) {
 }
 
 static __device__ F2 f2_cta_exclusive_scan(F2 x, F2* sh) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  constexpr int nw = kRowThreads / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   F2 xi = x;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -609,7 +725,7 @@ static __device__ F2 f2_cta_exclusive_scan(F2 x, F2* sh) {
   if (warp == 0) {
     F2 y = lane < nw ? sh[lane] : F2{0.f, 0.f};
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
+    for (int o = 1; o < nw; o <<= 1) {
       const F2 v = f2_shfl_up(y, o);
       if (lane >= o) y = f2_add(v, y);
     }
@@ -618,9 +734,7 @@ static __device__ F2 f2_cta_exclusive_scan(F2 x, F2* sh) {
     sh[lane] = yx;
   }
   __syncthreads();
-  const F2 r = f2_add(sh[warp], ex);
-  __syncthreads();
-  return r;
+  return f2_add(sh[warp], ex);  // the next user of sh begins with a barrier
 }
 
 // C = c.hi + c.lo >= k * delta, exactly up to the last two roundings.
@@ -640,67 +754,65 @@ static __device__ void map_rows_f32_body(const tq_vegas_state& st, double alpha,
   __shared__ int rownz[kMaxDim];
   const int d = st.dim;
   const int B = (int)st.n_bins;
-  T* w = (T*)row_smem;
-  T* wt = w + B;
-  T* sw = wt + B;
+  T* sw = (T*)row_smem;
   T* vv = sw + B;
   T* nx = vv + (B + 1);
+  T* w = vv;   // until sw is taken
+  T* wt = nx;
   T* xe = nx + (B + 1);  // [B+1] old edges
   T* dxe = xe + (B + 1);  // [B] old widths
   int32_t* mk = (int32_t*)(dxe + B);
   int32_t* ind = mk + B;
   unsigned char* z = (unsigned char*)(ind + (B + 1));
   unsigned char* zt = z + B;
-  // one pass over global memory: the zero-row test over every row (all
-  // elements of the map at once), this row's averages and empty intervals,
-  // and this row's edges
-  if (threadIdx.x < d) rownz[threadIdx.x] = 0;
-  __syncthreads();
+  // one pass over global memory: this row's weights, counts and edges (all
+  // loads before the first use) and the zero-row test over every row
+  int64_t rc[kRowPer];
+  double rw[kRowPer];
+  T rx[kRowPer], rd[kRowPer], rlast = (T)0;
   const T* xe_g = (const T*)st.x_edges + (int64_t)k * (B + 1);
   const T* dxe_g = (const T*)st.dx_edges + (int64_t)k * B;
-  if (!smooth_out) {
-    for (int e = threadIdx.x; e <= B; e += blockDim.x) xe[e] = xe_g[e];
-    for (int b = threadIdx.x; b < B; b += blockDim.x) dxe[b] = dxe_g[b];
-  }
-  int anyz = 0;
-  volatile int* rnz = rownz;  // other rows: skipped once found nonzero (0 -> 1 only)
-  for (int i = threadIdx.x; i < d * B; i += blockDim.x) {
-    const int kk = i / B, b = i - kk * B;
-    if (kk != k && rnz[kk]) continue;
-    const int64_t c = st.counts[i];
-    const T wi = (T)st.weights[i];
-    const T av = c == 0 ? wi : div_rn(wi, (T)c);
-    if (av != (T)0) rnz[kk] = 1;
-    if (kk == k) {
-      z[b] = c == 0;
-      anyz |= c == 0;
-      w[b] = av;
+#pragma unroll
+  for (int j = 0; j < kRowPer; ++j) {
+    const int b = threadIdx.x + j * kRowThreads;
+    if (b < B) {
+      rc[j] = st.counts[(int64_t)k * B + b];
+      rw[j] = st.weights[(int64_t)k * B + b];
+      if (!smooth_out) {
+        rx[j] = xe_g[b];
+        rd[j] = dxe_g[b];
+      }
     }
   }
+  if (!smooth_out && threadIdx.x == 0) rlast = xe_g[B];
+  find_nonzero_rows<T>(st, rownz);
+  int anyz = 0, odd = 0;
+#pragma unroll
+  for (int j = 0; j < kRowPer; ++j) {
+    const int b = threadIdx.x + j * kRowThreads;
+    if (b < B) {
+      const T wi = (T)rw[j];
+      z[b] = rc[j] == 0;
+      anyz |= rc[j] == 0;
+      odd |= rc[j] == 0 && (wi != (T)0 || signbit(wi));
+      w[b] = rc[j] == 0 ? wi : div_rn(wi, (T)rc[j]);
+      if (!smooth_out) {
+        xe[b] = rx[j];
+        dxe[b] = rd[j];
+      }
+    }
+  }
+  if (!smooth_out && threadIdx.x == 0) xe[B] = rlast;
   __syncthreads();
+  const unsigned turn = smooth_out ? 0u : draw_clear(ticket);
   int zero_row = 0;
   for (int kk = 0; kk < d; ++kk) zero_row |= !rownz[kk];
   if (zero_row) {
     if (k == 0 && threadIdx.x == 0) atomicAdd(st.flags + 0, 1);
-    if (!smooth_out) clear_map_by_last(st, ticket, nrows);
+    if (!smooth_out) clear_map_if(st, ticket, nrows, turn);
     return;
   }
-  if (__syncthreads_or(anyz)) {
-    for (int sweep = 0; sweep < 10; ++sweep) {
-      for (int b = threadIdx.x; b < B; b += blockDim.x) {
-        wt[b] = (b < B - 1 && z[b]) ? w[b + 1] : w[b];
-        zt[b] = (b < B - 1) ? (z[b] && z[b + 1]) : z[b];
-      }
-      __syncthreads();
-      int left = 0;
-      for (int b = threadIdx.x; b < B; b += blockDim.x) {
-        w[b] = (b > 0 && zt[b]) ? wt[b - 1] : wt[b];
-        z[b] = (b > 0) ? (zt[b] && zt[b - 1]) : zt[b];
-        left |= z[b];
-      }
-      if (!__syncthreads_or(left)) break;
-    }
-  }
+  fill_empty<T>(w, wt, z, zt, B, anyz, odd);
   F2 acc{0.f, 0.f};
   for (int b = threadIdx.x; b < B; b += blockDim.x) acc = f2_add(acc, w[b]);
   const T sum = f2_round(f2_block_sum_all(acc, red));  // :151
@@ -744,17 +856,7 @@ static __device__ void map_rows_f32_body(const tq_vegas_state& st, double alpha,
     ind[e] = 0;
   }
   __syncthreads();
-  for (int b = threadIdx.x; b < B; b += blockDim.x) {  // :214-230
-    const int from = b == 0 ? 0 : mk[b - 1];
-    const int to = b == B - 1 ? B + 1 : mk[b];
-    for (int e = from; e < to; ++e) ind[e] = b;
-    if (b < B - 1 && (b == 0 || mk[b] != mk[b - 1])) {
-      const int q = mk[b];
-      T a = (T)0;
-      for (int e = b; e < B - 1 && mk[e] == q; ++e) a = add_rn(a, sw[e]);
-      vv[q] = a;
-    }
-  }
+  map_runs<T>(mk, sw, B, ind, vv);
   __syncthreads();
   // :233 d_accu and EQ 22
   s = F2{0.f, 0.f};
@@ -791,7 +893,7 @@ static __device__ void map_rows_f32_body(const tq_vegas_state& st, double alpha,
   T* dxo = (T*)st.dx_edges + (int64_t)k * B;
   for (int e = threadIdx.x; e <= B; e += blockDim.x) xo[e] = nx[e];
   for (int b = threadIdx.x; b < B; b += blockDim.x) dxo[b] = sub_rn(nx[b + 1], nx[b]);  // :259
-  clear_map_by_last(st, ticket, nrows);
+  clear_map_if(st, ticket, nrows, turn);
 }
 
 
