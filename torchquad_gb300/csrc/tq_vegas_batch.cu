@@ -89,25 +89,6 @@ __global__ void __launch_bounds__(kBlock) vegas_batch_begin_kernel(BatchLaunch L
 }
 
 template <typename T, bool WARM>
-__device__ __forceinline__ void batch_sample(const SampleArgs& a, int family, unsigned bid, unsigned nblk,
-                                             SampleStatic<T>& ss) {
-  switch (family) {
-    case TQ_FN_EXP_SUM:
-      sample_body<T, TQ_FN_EXP_SUM, WARM, 0>(a, bid, nblk, ss);
-      break;
-    case TQ_FN_GAUSSIAN:
-      sample_body<T, TQ_FN_GAUSSIAN, WARM, 0>(a, bid, nblk, ss);
-      break;
-    case TQ_FN_OSCILLATORY:
-      sample_body<T, TQ_FN_OSCILLATORY, WARM, 0>(a, bid, nblk, ss);
-      break;
-    default:
-      sample_body<T, TQ_FN_SUM_SIN, WARM, 0>(a, bid, nblk, ss);
-      break;
-  }
-}
-
-template <typename T, bool WARM>
 __global__ void __launch_bounds__(kTile, std::is_same<T, double>::value ? 3 : TQ_SAMPLE_MIN_BLOCKS)
     vegas_batch_sample_kernel(BatchLaunch L) {
   const uint2 m = L.map[blockIdx.x];
@@ -115,7 +96,7 @@ __global__ void __launch_bounds__(kTile, std::is_same<T, double>::value ? 3 : TQ
   if (!WARM && batch_stopped(e)) return;
   __shared__ SampleStatic<T> ss;
   const SampleArgs a = WARM ? e.warm : e.iter;  // a private copy the compiler may keep in registers
-  batch_sample<T, WARM>(a, a.family, m.y, (unsigned)e.ctas[WARM ? TQ_VB_WARM : TQ_VB_SAMPLE], ss);
+  sample_body<T, kAnyFamily, WARM, 0>(a, m.y, (unsigned)e.ctas[WARM ? TQ_VB_WARM : TQ_VB_SAMPLE], ss);
 }
 
 template <typename T>

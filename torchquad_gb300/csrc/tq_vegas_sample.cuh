@@ -118,6 +118,7 @@ struct SampleArgs {
   int64_t n_samples;  // warm-up: points; iterations: read from cube_start
   int use_map;        // accumulate the map histogram
   int edges_smem, hist_smem;
+  int count_smem;     // without hist_smem: counts of the CTA in shared memory
   int small_cubes;    // n_cubes < 2^32: cube digits with 32-bit division
   FastDiv ns_div;     // division by n_strat
   unsigned* ticket;
@@ -137,22 +138,25 @@ struct HistT<float> {
 
 // Shared memory of the sampler: the map (edges) when it fits, and one
 // private histogram per warp (weights in HistT, counts in u32) when it fits.
+// Where it does not, the counts of the CTA (u16, two to a word) when they fit
+// beside the map.
 template <typename T>
 struct Smem {
   T* xe;
   T* dxe;
   typename HistT<T>::type* hw;  // [warps][d*B]
-  unsigned* hc;                 // [warps][d*B]
+  unsigned* hc;                 // [warps][d*B]; count_smem: [(d*B+1)/2]
 };
 
 constexpr int kWarps = kTile / 32;
 
 __host__ __device__ inline size_t sample_smem_bytes(int d, int64_t B, size_t tsize, bool hist,
-                                                    bool edges) {
+                                                    bool edges, bool counts = false) {
   size_t off = 0;
   if (edges) off += ((tsize * (d * (B + 1)) + 15) & ~size_t(15)) + tsize * (d * B);
   off = (off + 15) & ~size_t(15);
   if (hist) off += (size_t)kWarps * d * B * (tsize + sizeof(unsigned));  // HistT<T> weight, u32 count
+  if (counts) off += ((size_t)(d * B + 1) / 2 * sizeof(unsigned) + 15) & ~size_t(15);
   return off;
 }
 
@@ -178,7 +182,7 @@ __device__ Smem<T> carve(unsigned char* base, const SampleArgs& a) {
     s.hc = (unsigned*)(base + off);
   } else {
     s.hw = nullptr;
-    s.hc = nullptr;
+    s.hc = (unsigned*)(base + off);
   }
   return s;
 }
@@ -246,9 +250,17 @@ __device__ __forceinline__ void warp_hist_add(H* hw, unsigned* hc, int key, bool
 __device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 
+// The family read from the state at run time (a batch's sampler).
+constexpr int kAnyFamily = -1;
+
 // s + g_k(x) (g_0(x) for k = 0).
 template <int FAM, typename T>
 __device__ __forceinline__ T vegas_sum(const Family<T>& f, int k, T x, T s) {
+  if constexpr (FAM == kAnyFamily) {
+    if (f.id == TQ_FN_GAUSSIAN) return vegas_sum<TQ_FN_GAUSSIAN, T>(f, k, x, s);
+    if (f.id == TQ_FN_SUM_SIN) return vegas_sum<TQ_FN_SUM_SIN, T>(f, k, x, s);
+    return vegas_sum<TQ_FN_EXP_SUM, T>(f, k, x, s);  // and TQ_FN_OSCILLATORY
+  }
   if (FAM == TQ_FN_GAUSSIAN) {
     const T d = sub_rn(x, f.u[k]);
     const T dd = mul_rn(d, d);
@@ -262,6 +274,12 @@ __device__ __forceinline__ T vegas_sum(const Family<T>& f, int k, T x, T s) {
 }
 template <int FAM, typename T>
 __device__ __forceinline__ T vegas_outer(const Family<T>& f, T s) {
+  if constexpr (FAM == kAnyFamily) {
+    if (f.id == TQ_FN_EXP_SUM) return vegas_outer<TQ_FN_EXP_SUM, T>(f, s);
+    if (f.id == TQ_FN_GAUSSIAN) return vegas_outer<TQ_FN_GAUSSIAN, T>(f, s);
+    if (f.id == TQ_FN_OSCILLATORY) return vegas_outer<TQ_FN_OSCILLATORY, T>(f, s);
+    return vegas_outer<TQ_FN_SUM_SIN, T>(f, s);
+  }
   if (FAM == TQ_FN_EXP_SUM) return mul_rn(f.c, exp(add_rn(s, f.b)));
   if (FAM == TQ_FN_GAUSSIAN) return mul_rn(f.c, exp(-s));
   if (FAM == TQ_FN_OSCILLATORY) return mul_rn(f.c, cos(fma_rn((T)(2.0 * CUDART_PI), f.b, s)));
@@ -278,12 +296,18 @@ struct DrawBlocks {
 
 // D > 0: the dimension is known at compile time (fully unrolled point
 // loops, D interval indices in registers); D = 0: any dimension up to
-// kMaxDim from the state.
+// kMaxDim from the state, the point loops left rolled.  A warp of a batch
+// takes two tiles, so it runs its code about once: unrolled sixteen times,
+// with a body per family, that code is fetched far more than it is run (256
+// states: 93 us a sampling phase; rolled 82.6; with the Philox blocks computed
+// by all lanes at once 80.5, as with one body for all families, which is
+// kept for its size).
 // The sampler as a device body: CTA bid of nblk CTAs taking part (the
 // per-launch kernel below, or one state's share of a batched launch).
 template <typename T, int FAM, bool WARM, int D>
 __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk, SampleStatic<T>& ss) {
   constexpr int KD = D > 0 ? D : kMaxDim;
+  constexpr int KU = D > 0 ? D : 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Family<T>& fam = ss.fam;
   T* const lo = ss.lo;
@@ -317,6 +341,9 @@ __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk, Sa
   if (a.hist_smem) {  // weights and counts, contiguous from a 16-byte boundary
     const int bytes = (int)(kWarps * DB) * (int)(sizeof(H) + sizeof(unsigned));
     for (int i = threadIdx.x; i < bytes / 16; i += kTile) ((uint4*)sm.hw)[i] = make_uint4(0, 0, 0, 0);
+  } else if (a.count_smem) {
+    const int words = ((int)DB + 1) / 2;
+    for (int i = threadIdx.x; i < (words + 3) / 4; i += kTile) ((uint4*)sm.hc)[i] = make_uint4(0, 0, 0, 0);
   }
 
   const int64_t M = WARM ? a.n_samples : __ldcg(st.cube_start + st.n_cubes);
@@ -338,6 +365,8 @@ __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk, Sa
   const int64_t n_warps = (int64_t)nblk * kWarps;
   const int64_t gw = (int64_t)bid * kWarps + warp;
   const int64_t t_begin = gw * n_tiles / n_warps, t_end = (gw + 1) * n_tiles / n_warps;
+  // a count of the CTA stays below its points
+  const bool cta_counts = a.count_smem && n_tiles <= (int64_t)nblk * 2047;
   int64_t c0 = 0;  // cube of the tile's first point
   const int64_t* pre = (!WARM && st.control[kCtlSplit] != 0) ? a.block_pre : nullptr;
   if (!WARM && t_begin < t_end) c0 = warp_find_cube(st.cube_start, pre, st.n_cubes, t_begin * 32);
@@ -372,8 +401,7 @@ __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk, Sa
       const uint64_t e0 = (uint64_t)j * (uint64_t)d;
       const uint64_t blk0 = offset + e0 / PB;
       const int lane0 = (int)(e0 % PB);
-      int cur = -1;
-      uint4 r = make_uint4(0, 0, 0, 0);
+      uint4 r = make_uint4(0, 0, 0, 0), nxt = r;
       // fp32 with the dimension fixed: every lane computes the blocks its
       // draws can touch at once (no divergent per-draw block branch) and
       // picks its words by its first word's offset
@@ -393,7 +421,7 @@ __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk, Sa
       }
       T jac = (T)1;
       T s = T(0);
-#pragma unroll
+#pragma unroll KU
       for (int k = 0; k < KD; ++k) {
         if (k < d) {
           T u;
@@ -404,13 +432,19 @@ __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk, Sa
               if (k + o < 4 * NB) w = lane0 == o ? words[k + o] : w;
             u = (T)u32_to_unit_f(w);
           } else {
-            const int le = lane0 + k;
-            const int bi = le / PB;
-            if (bi != cur) {
-              r = philox_block(seed, sid, blk0 + (uint64_t)bi);
-              cur = bi;
+            // the words from this point's offset in the block on, taken
+            // from two blocks every PB draws, by all lanes at once (lanes
+            // cross into their next block at different draws)
+            if (k % PB == 0) {
+              const uint4 b0 = k == 0 ? philox_block(seed, sid, blk0) : nxt;
+              nxt = philox_block(seed, sid, blk0 + (uint64_t)(k / PB + 1));
+              r = b0;
+              const int o = lane0 * (4 / PB);
+              if (o & 2) r = make_uint4(r.z, r.w, nxt.x, nxt.y);
+              if (o & 1) r = make_uint4(r.y, r.z, r.w, (o & 2) ? nxt.z : nxt.x);
             }
-            u = Uniform<T>::from(r, le - bi * PB);
+            u = Uniform<T>::from(r, 0);
+            r = PB == 4 ? make_uint4(r.y, r.z, r.w, 0u) : make_uint4(r.z, r.w, 0u, 0u);
           }
           T y;
           if (WARM) {
@@ -442,7 +476,7 @@ __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk, Sa
       jf2 = jfd * jfd;
     }
     if (a.use_map) {
-#pragma unroll
+#pragma unroll KU
       for (int k = 0; k < KD; ++k) {
         if (k < d) {
           if (a.hist_smem) {
@@ -450,7 +484,12 @@ __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk, Sa
             warp_hist_add<H>(whw, whc, key, valid, jf2);
           } else if (valid) {
             atomicAdd(st.weights + k * B + ids[k], (double)jf2);
-            atomicAdd((unsigned long long*)(st.counts + k * B + ids[k]), 1ull);
+            if (cta_counts) {
+              const int key = (int)(k * B) + ids[k];
+              atomicAdd(sm.hc + (key >> 1), 1u << ((key & 1) * 16));
+            } else {
+              atomicAdd((unsigned long long*)(st.counts + k * B + ids[k]), 1ull);
+            }
           }
         }
       }
@@ -496,6 +535,13 @@ __device__ void sample_body(const SampleArgs& a, unsigned bid, unsigned nblk, Sa
         atomicAdd(st.weights + i, (double)w);
         atomicAdd((unsigned long long*)(st.counts + i), (unsigned long long)cnt);
       }
+    }
+  }
+  if (cta_counts && a.use_map) {
+    __syncthreads();
+    for (int i = threadIdx.x; i < (int)DB; i += kTile) {
+      const unsigned cnt = (sm.hc[i >> 1] >> ((i & 1) * 16)) & 0xffffu;
+      if (cnt) atomicAdd((unsigned long long*)(st.counts + i), (unsigned long long)cnt);
     }
   }
   // The last CTA advances the RNG offset.  It reads nothing the other CTAs
