@@ -42,3 +42,43 @@ def test_counts_at_the_width_of_a_count(n, cuda):
     # equal intervals: a count is binomial, nine standard deviations
     mean = n / 1001
     assert float((dev.counts.double() - mean).abs().max()) <= 9.0 * mean**0.5
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("strat", [1, 2, 3, 7, 10, 41, 255, 4_093, 65_537, 1_048_575, 3_000_017])
+def test_stratified_draws_are_those_of_the_division(strat, dtype, cuda):
+    """The quotient by n_strat to its last bits: 2^24 intervals, so that a
+    count gives 24 bits of the y of its draw."""
+    from torchquad_gb300 import _lib as L
+
+    bins, f = 1 << 24, tq.ExpSum(1)
+    dev = VegasDevice(1, dtype, bins, strat, cuda)
+    dev.set_control(L.TQ_VC_NEVALS | L.TQ_VC_SEED | L.TQ_VC_STREAM, nevals=max(100_000, 2 * strat), seed=9, sid=0)
+    dev.get_nh()
+    dev.iterate_fused(f.family, f.device_params(cuda), True)
+    pos = torch.repeat_interleave(torch.arange(strat, device=cuda), dev.neval)
+    u = RNG(seed=9).uniform([pos.numel(), 1], dtype)[:, 0]
+    y = (pos.to(dtype) + u) / torch.full((1,), strat, dtype=dtype, device=cuda)
+    y = torch.where(y >= 1.0, torch.full_like(y, 0.999999), y)
+    want = torch.bincount(torch.floor(y * bins).long(), minlength=bins)
+    assert torch.equal(dev.counts[0], want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("bins", [2, 3, 5, 9, 17, 33])
+def test_groups_of_every_size_in_warp_histograms(bins, dtype, cuda):
+    """Few intervals: groups of up to 32 lanes share one, on both sides of the
+    steps that are taken without a loop."""
+    for n in (1, 31, 32, 33, 1_000, 70_001):
+        dev = warmed(3, bins, n, dtype, cuda)
+        y = RNG(seed=5).uniform([n, 3], dtype) * 0.999999
+        ids = torch.floor(y * bins).long()
+        x = y.double()
+        f2 = torch.exp(x.sum(1)) ** 2
+        for k in range(3):
+            assert torch.equal(dev.counts[k], torch.bincount(ids[:, k], minlength=bins))
+            want = torch.zeros(bins, dtype=torch.float64, device=cuda).index_add_(0, ids[:, k], f2)
+            # fp32: squares rounded three times and more, warp sums of at most
+            # n values in fp32 trees and one add a tile (70001/32/4864 tiles a warp)
+            tol = 1e-5 if dtype == torch.float32 else 1e-12
+            assert torch.allclose(dev.weights[k], want, rtol=tol, atol=0)
