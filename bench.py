@@ -261,7 +261,7 @@ def measure_batched(tq, dev, L, peaks, reps=5):
         vp = np.array([float(x) for x in plain])
         rel = np.abs(vb - exact) / np.abs(exact)
         d = plan.desc_np
-        rows = int(np.sum(d["total"] // d["n"]))
+        terms = int(np.sum(d["n"] * d["dim"]))
         rec = {
             "batched_integrals_per_s": len(specs) / t_batch,
             "batched_ms": t_batch * 1000.0,
@@ -278,13 +278,15 @@ def measure_batched(tq, dev, L, peaks, reps=5):
             "max_rel_diff_e2e_vs_resident": float(np.max(np.abs(v_e2e.double().numpy() - vb) / np.abs(vb))),
         }
         if dtype == torch.float64:
-            # fp64 grids: the outer function once per grid row, every node a
-            # multiply by its row factor and a compensated add (3 FP64 ops)
-            rec["outer_evals_per_s"] = rows / t_batch
-            ach = 3.0 * plan.total_points / t_batch / 1e12
-            rec["roofline"] = {"bound": "fp64", "achieved": ach, "peak": peaks["fp64"], "unit": "TFLOP/s",
-                               "frac": ach / peaks["fp64"], "ops_per_node": 3,
-                               "peak_source": "FP64 FMA probe measured in this run"}
+            # the sums factor into dim * n one-dimensional terms an integral:
+            # the argument's multiply, the weight's multiply and the add of
+            # each (the term's exp, cos or sin and long rows' Horner steps
+            # are not counted)
+            rec["terms_per_s"] = terms / t_batch
+            ach = 3.0 * terms / t_batch / 1e12
+            rec["roofline"] = {"bound": "fp64 and latency", "achieved": ach, "peak": peaks["fp64"],
+                               "unit": "TFLOP/s", "frac": ach / peaks["fp64"], "ops_per_term": 3,
+                               "terms": terms, "peak_source": "FP64 FMA probe measured in this run"}
         out[name] = rec
     out["cpu_baseline"] = c3_cpu_baseline(specs)
     return out
@@ -331,16 +333,16 @@ def measure_grid_cases(tq, dev, L, peaks, flush, reps=20):
                                   L.stream_handle()), "tq_grid_fused")
 
     t_k = timed_launches(torch, fused, 200)
-    ach = 3.0 * nodes / t_k / 1e12
-    c1 = {"api_ms": ms, "kernel_us": t_k * 1e6, "nodes_per_s": nodes / t_k, "outer_evals_per_s": n**2 / t_k,
+    ach = 3.0 * 3 * n / t_k / 1e12
+    c1 = {"api_ms": ms, "kernel_us": t_k * 1e6, "nodes_per_s": nodes / t_k, "terms_per_s": 3 * n / t_k,
           "e2e_ms": t_e2e * 1000.0, "rel_err_vs_analytic": abs(v.item() - exact) / exact,
           "e2e_value_matches": v_e2e == v.item(),
-          "roofline": {"kernel": "grid_fused_kernel<double,double,SIMPSON,EXP_SUM>", "bound": "fp64",
+          "roofline": {"kernel": "grid_fused_kernel<double,double,SIMPSON,EXP_SUM>", "bound": "latency",
                        "achieved": ach, "peak": peaks["fp64"], "unit": "TFLOP/s", "frac": ach / peaks["fp64"],
-                       "ops_per_node": 3, "peak_source": "FP64 FMA probe measured in this run",
-                       "note": "fp64 rows: exp once per grid row; per node a multiply by the row factor, "
-                               "a weight multiply and an add (3 FP64 ops); 1.03M nodes is a few microseconds "
-                               "of work, so launch and reduction latency weigh in"}}
+                       "ops_per_term": 3, "peak_source": "FP64 FMA probe measured in this run",
+                       "note": "the sum factors into 3 x 101 one-dimensional terms (argument and weight "
+                               "multiply and an add each): a few warps, so the launch and its reductions "
+                               "are latency"}}
     # materialised path: an arbitrary torch callable
     fn = lambda x: torch.exp(x.sum(1))  # noqa: E731
     c1["materialised_api_ms"] = timed(lambda: tq.Simpson().integrate(fn, 3, N=nodes, integration_domain=dom))
@@ -371,8 +373,8 @@ def measure_grid_cases(tq, dev, L, peaks, flush, reps=20):
                             "frac": bp / t_p / 1e9 / hbm, "bytes_per_node": 24},
             "weighted_sum": {"us": t_w * 1e6, "bytes": bw, "achieved_gbs": bw / t_w / 1e9, "peak_gbs": hbm,
                              "frac": bw / t_w / 1e9 / hbm, "bytes_per_node": 8,
-                             "arithmetic": "double-float products and sums on the FP32 pipe, each fp64 value "
-                                           "split into two floats by integer operations (no FP64 per node)"},
+                             "arithmetic": "pairs of values added in fp64, the pairs split into two floats "
+                                           "by integer operations and summed as double-floats"},
         }
         del pts, fv
     mat["peak_source"] = hbm_src
@@ -479,22 +481,19 @@ def measure_c4_batch(tq, dev, peaks, m=1024):
         OGR.value_and_grad(3, np.concatenate([[1.0, us[j]], a[j], np.zeros(4)]), OGR.GAUSS, 4, 32, [[0.0, 1.0]] * 4)
         j += 1
     t_cpu = (time.perf_counter() - t0) / j
-    nodes = m * 32**4
-    ach = 10.0 * nodes / t_dev / 1e12
+    terms = m * 4 * 32
+    ach = 12.0 * terms / t_dev / 1e12
     return {
         "batched_device_ms": t_dev * 1e3, "batched_fwd_bwd_integrals_per_s": m / t_dev,
         "batched_e2e_ms": t_e2e * 1e3, "batched_e2e_integrals_per_s": m / t_e2e,
         "plain_fwd_bwd_integrals_per_s": 1.0 / t_plain,
         "speedup_batched_vs_plain": t_plain * m / t_dev, "speedup_batched_e2e_vs_plain": t_plain * m / t_e2e,
         "max_rel_diff_batched_vs_plain_sample": float(max(diffs)),
-        "roofline": {"kernel": "batch_adjoint_kernel<double,4>", "bound": "issue (double-float on the FP32 pipe)",
+        "roofline": {"kernel": "batch_adjoint_kernel", "bound": "latency",
                      "achieved": ach, "peak": peaks["fp64"], "unit": "TFLOP/s", "frac": ach / peaks["fp64"],
-                     "ops_per_node": 10,
-                     "peak_source": "FP64 FMA probe measured in this run",
-                     "note": "10 fp64-equivalent operations per node (cos/sin of the angle sum from row factor "
-                             "and table, two weight products, four gradient accumulations), executed as "
-                             "double-floats on the FP32 pipe; the fraction compares them with the FP64 unit's "
-                             "peak rate, which the fp64 form of the loop was bound by"},
+                     "ops_per_term": 12, "peak_source": "FP64 FMA probe measured in this run",
+                     "note": "value and gradient factor into six weighted moments of each dimension's 32 "
+                             "nodes (a multiply and an add each; the cos and sin are not counted)"},
         "cpu_baseline": {"integrals_per_s": 1.0 / t_cpu, "unit": "integrals/s (value + gradient)",
                          "cores": cpu_cores_used(), "kind": "port",
                          "sample": f"{j} of the integrals, numpy gradient of the discrete rule "

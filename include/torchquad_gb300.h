@@ -96,7 +96,13 @@ size_t tq_grid_fused_workspace_size(int rule, int dim, int64_t n_per_dim);
  * + calculate_result/_apply_composite_rule (grid_integrator.py:57-91).
  * domain: device [dim][2] of dtype; gl_nodes/gl_weights: device fp64 [n]
  * Gauss-Legendre roots/weights on [-1,1] (only for TQ_RULE_GAUSS, whose
- * nodes are computed in fp64 as in gaussian.py:159-162). */
+ * nodes are computed in fp64 as in gaussian.py:159-162).
+ * The families are functions of a separable sum, so the rule is formed from
+ * dim * n_per_dim one-dimensional terms (fp64, weighted and summed exactly)
+ * where the factors stay in range: everything finite, no empty dimension,
+ * exponents up to 300 (80 for fp32), angles up to 10^6, c and the weights
+ * within 2^+-200 (fp32: no node value near overflow).  Other integrals, and
+ * one-dimensional rows of more than 4096 nodes, are evaluated node by node. */
 int tq_grid_fused(int dtype, int rule, int dim, int64_t n_per_dim,
                   const void* domain, const double* gl_nodes,
                   const double* gl_weights, int family, const double* params,
@@ -134,7 +140,9 @@ typedef struct tq_batch_desc {
  * launch (no counterpart in the reference, whose batch is a loop of
  * GridIntegrator.integrate, grid_integrator.py:32-55).  family is one
  * TQ_FN_* for every integral, or TQ_FN_PER_DESC to take each descriptor's
- * (families mixed in one launch).  Integral i is cut
+ * (families mixed in one launch).  Integrals that factor (see tq_grid_fused)
+ * are summed dimension by dimension, one to a CTA at a time; the others are
+ * worked on in tiles.  Integral i is cut
  * into ceil(total_i / tile_points) tiles; tile_start[n_integrals+1] is the
  * exclusive prefix of the tile counts (tile_start[n_integrals] = n_tiles).
  * block (128|256), strip (4|16 nodes per thread) and grid_blocks (0: 8 per

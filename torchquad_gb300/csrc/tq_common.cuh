@@ -74,10 +74,10 @@ __device__ __forceinline__ Acc acc_shfl_down(const Acc& a, int off) {
 // redux.sync and over the CTA as 64-bit integers, and one thread turns the
 // total into hi + lo doubles by bit moves.  Integer sums are exact and do
 // not depend on their order; a value loses only bits below 2^-95 of the
-// largest.  A 101^3 fused Simpson launch (252 CTAs): 26.4 us with the fp64
-// trees, 18.7 us with these sums and the
-// dimensions set up in parallel; a 10001-node rule over 200 components (50
-// reductions a component group): 969 and 431 us.
+// largest.  A 101^3 fused Simpson launch by nodes (252 CTAs): 26.4 us with the
+// fp64 trees, 18.7 us with these sums and the dimensions set up in parallel; a
+// 10001-node rule over 200 components (50 reductions a component group): 969
+// and 431 us.
 __device__ __forceinline__ int exp_field(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
 
 // L += v in units of 2^(emax - 1118) (limb i has weight 2^(24 i)); v finite,
@@ -431,7 +431,8 @@ __device__ __forceinline__ float u32_to_unit_f(uint32_t r) {
 }
 // x 2^-53 for the leading 53 bits x, put together by bit moves: a conversion
 // and a multiply would each hold the FP64 unit for 64 cycles a warp (fused
-// fp64 Monte Carlo, 10^7 points, d = 6: 1296 and, with the values summed as integers too, 913 us).
+// fp64 Monte Carlo, 10^7 points, d = 6: 1296 us, and 913 us this way with the
+// values summed as integers too).
 __device__ __forceinline__ double u64_to_unit_d(uint32_t lo, uint32_t hi) {
   const uint64_t x = (((uint64_t)hi << 32) | lo) >> 11;
   const int lz = __clzll((long long)x);
