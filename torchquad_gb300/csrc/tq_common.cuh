@@ -532,8 +532,7 @@ struct Family {
 // FP64 unit as long for one lane as for a warp.
 template <typename T>
 __device__ __forceinline__ void load_family(Family<T>& f, int id, int dim,
-                                            const double* __restrict__ p) {
-  const int k = threadIdx.x;
+                                            const double* __restrict__ p, int k = threadIdx.x) {
   if (k < kMaxDim) {
     f.a[k] = k < dim ? (T)p[2 + k] : T(0);
     f.u[k] = (k < dim && id == TQ_FN_GAUSSIAN) ? (T)p[2 + dim + k] : T(0);

@@ -595,6 +595,7 @@ struct BatchGradArgs {
   const double* gl_weights;
   int family;
   int stride;        // partial sums per tile row: 2 + 4 * DM
+  int64_t fact;      // CTAs that take the factored integrals
   double* partials;  // [n_tiles][stride]
 };
 
@@ -641,25 +642,61 @@ __device__ void batch_adj_dispatch(const BatchGradArgs& a, const tq_batch_desc& 
   }
 }
 
-// One integral by its 1-D sums (tq_separable.cuh), by one CTA, into the
-// partials' row `tile`.
-template <typename T, int FAM>
-__device__ void batch_adj_sep(const BatchGradArgs& a, const tq_batch_desc& d, int64_t tile, const Geo<T>& g,
-                              const Family<T>& fam, Acc (*dsum)[kSepMaxM<true>], Acc* sp) {
-  sep_sums<T, FAM, true>(g, fam, d.rule, d.dim, d.n, a.gl_nodes + d.gl_off, a.gl_weights + d.gl_off, 0u, 1u,
-                         nullptr, 0, nullptr, dsum, sp);
-  if (threadIdx.x < 32) sep_adjoint<FAM, T>(dsum, fam.a, d.dim, a.partials + tile * a.stride);
-}
+// A round of factored integrals (tq_separable.cuh), one to a warp: each warp
+// sets its integral up, the CTA takes their 1-D sums one integral after the
+// other, each warp forms its integral's products.  The products are a chain of
+// some 200 FP64 operations in one warp, 64 cycles each; side by side they
+// spread over the sub-partitions' FP64 units (1024 integrals of d = 4, 32
+// nodes: 154 us a call with set-up and products integral by integral in warp 0,
+// 139 this way, 121 with the finalize reading one row of such an integral, 107
+// on the CTAs resident at once).
+constexpr int kAdjWarps = kBlock / 32;
+template <int DM>
+struct AdjRound {
+  Geo<double> g64[kAdjWarps];
+  Family<double> fam64[kAdjWarps];
+  Geo<float> g32[kAdjWarps];
+  Family<float> fam32[kAdjWarps];
+  tq_batch_desc d[kAdjWarps];
+  Acc dsum[kAdjWarps][DM][kSepMaxM<true>];
+  double a[kAdjWarps][DM];
+  Acc sp[kAdjWarps * kSepMaxM<true>];  // at most a unit a warp (DM <= 8)
+};
 template <typename T>
-__device__ void batch_adj_sep_dispatch(const BatchGradArgs& a, const tq_batch_desc& d, int64_t tile,
-                                       const Geo<T>& g, const Family<T>& fam, Acc (*dsum)[kSepMaxM<true>],
-                                       Acc* sp) {
+__device__ void batch_adj_sums(const BatchGradArgs& a, const tq_batch_desc& d, const Geo<T>& g,
+                               const Family<T>& fam, Acc (*dsum)[kSepMaxM<true>], Acc* sp) {
+#define TQ_ADJ_SUMS(FAM)                                                                                         \
+  sep_sums<T, FAM, true>(g, fam, d.rule, d.dim, d.n, a.gl_nodes + d.gl_off, a.gl_weights + d.gl_off, 0u, 1u,     \
+                         nullptr, 0, nullptr, dsum, sp)
   switch (fam.id) {
-    case TQ_FN_EXP_SUM: batch_adj_sep<T, TQ_FN_EXP_SUM>(a, d, tile, g, fam, dsum, sp); break;
-    case TQ_FN_GAUSSIAN: batch_adj_sep<T, TQ_FN_GAUSSIAN>(a, d, tile, g, fam, dsum, sp); break;
-    case TQ_FN_OSCILLATORY: batch_adj_sep<T, TQ_FN_OSCILLATORY>(a, d, tile, g, fam, dsum, sp); break;
-    default: batch_adj_sep<T, TQ_FN_SUM_SIN>(a, d, tile, g, fam, dsum, sp); break;
+    case TQ_FN_EXP_SUM: TQ_ADJ_SUMS(TQ_FN_EXP_SUM); break;
+    case TQ_FN_GAUSSIAN: TQ_ADJ_SUMS(TQ_FN_GAUSSIAN); break;
+    case TQ_FN_OSCILLATORY: TQ_ADJ_SUMS(TQ_FN_OSCILLATORY); break;
+    default: TQ_ADJ_SUMS(TQ_FN_SUM_SIN); break;
   }
+#undef TQ_ADJ_SUMS
+}
+__device__ __forceinline__ void batch_adj_products(int family, const Acc (*dsum)[kSepMaxM<true>], const double* av,
+                                                   int dim, double* out) {
+  switch (family) {
+    case TQ_FN_EXP_SUM: sep_adjoint<TQ_FN_EXP_SUM, double>(dsum, av, dim, out); break;
+    case TQ_FN_GAUSSIAN: sep_adjoint<TQ_FN_GAUSSIAN, double>(dsum, av, dim, out); break;
+    case TQ_FN_OSCILLATORY: sep_adjoint<TQ_FN_OSCILLATORY, double>(dsum, av, dim, out); break;
+    default: sep_adjoint<TQ_FN_SUM_SIN, double>(dsum, av, dim, out); break;
+  }
+}
+
+// Whether an integral is taken in factored form (by a whole warp).
+template <typename D>
+__device__ __forceinline__ bool batch_adj_factors(const BatchGradArgs& a, const tq_batch_desc& d) {
+  constexpr bool kF32 = std::is_same<D, float>::value;
+  const int fid = a.family >= 0 ? a.family : d.family;
+  const D* dom = (const D*)a.domains + d.dom_off;
+  const double* par = a.params + d.par_off;
+  // one dimension in several tiles: the tiles' nodes spread over CTAs
+  return (d.dim > 1 || d.n <= a.tile_pts) &&
+         (kF32 && d.rule != TQ_RULE_GAUSS ? sep_ok<float, D>(fid, d.dim, d.n, dom, par)
+                                          : sep_ok<double, D>(fid, d.dim, d.n, dom, par));
 }
 
 // Gauss integrals and fp64 batches work in fp64 (their table rows as
@@ -675,32 +712,26 @@ __global__ void __launch_bounds__(kBlock, DM <= 4 ? 2 : 1) batch_adjoint_kernel(
   __shared__ Family<float> fam32;
   __shared__ uint64_t rstride[kMaxDim];
   __shared__ double sh[kBlock / 32][2 + 4 * DM];
-  __shared__ AdjTab tab;
+  __shared__ union {
+    AdjTab tab;        // tiles
+    AdjRound<DM> rnd;  // factored integrals
+  } u;
+  AdjTab& tab = u.tab;
   __shared__ tq_batch_desc d;
   __shared__ int64_t tile0;
   constexpr bool kF32 = std::is_same<D, float>::value;
-  __shared__ int64_t ti[kBlock / 32], ts[kBlock / 32], te[kBlock / 32];
+  __shared__ int64_t ti[kBlock / 32], ts[kBlock / 32];
   __shared__ int tsep[kBlock / 32];
-  __shared__ Acc dsum[kMaxDim][kSepMaxM<true>];
-  __shared__ Acc sp[kSepSlots<true>];
   const int warp = threadIdx.x >> 5;
-  // As in batch_grid_kernel: first the integrals in factored form, one per
-  // CTA and turn (its sums in the row of its first tile, zeros in the
-  // others), then the tiles of the rest; a round is looked up by the warps
-  // in parallel.
+  // As in batch_grid_kernel: first the integrals in factored form, in rounds
+  // of one a warp (an integral's sums in the row of its first tile), then the
+  // tiles of the rest; a round is looked up by the
+  // warps in parallel.
   auto lookup = [&](int64_t i) {  // by a whole warp
-    const tq_batch_desc& di = a.desc[i];
-    const int fid = a.family >= 0 ? a.family : di.family;
-    const D* dom = (const D*)a.domains + di.dom_off;
-    const double* par = a.params + di.par_off;
-    // one dimension in several tiles: the tiles' nodes spread over CTAs
-    const bool sep = (di.dim > 1 || di.n <= a.tile_pts) &&
-                     (kF32 && di.rule != TQ_RULE_GAUSS ? sep_ok<float, D>(fid, di.dim, di.n, dom, par)
-                                                       : sep_ok<double, D>(fid, di.dim, di.n, dom, par));
+    const bool sep = batch_adj_factors<D>(a, a.desc[i]);
     if ((threadIdx.x & 31) == 0) {
       ti[warp] = i;
       ts[warp] = a.tile_start[i];
-      te[warp] = a.tile_start[i + 1];
       tsep[warp] = sep;
     }
   };
@@ -731,21 +762,39 @@ __global__ void __launch_bounds__(kBlock, DM <= 4 ? 2 : 1) batch_adjoint_kernel(
     __syncthreads();
   };
   constexpr int nw = kBlock / 32;
-  for (int64_t base = blockIdx.x; base < a.n_int; base += (int64_t)nw * gridDim.x) {
-    const int64_t mine = base + (int64_t)warp * gridDim.x;
-    if (mine < a.n_int) lookup(mine);
+  for (int64_t base = blockIdx.x; blockIdx.x < a.fact && base < a.n_int; base += nw * a.fact) {
+    const int64_t mine = base + warp * a.fact;
+    const int lane = threadIdx.x & 31;
+    if (mine < a.n_int) {
+      lookup(mine);
+      const tq_batch_desc& di = a.desc[mine];
+      const int fid = a.family >= 0 ? a.family : di.family;
+      const D* dom = (const D*)a.domains + di.dom_off;
+      if (lane == 0) u.rnd.d[warp] = di;
+      if (kF32 && di.rule != TQ_RULE_GAUSS) {
+        geo_setup<float, D>(u.rnd.g32[warp], di.rule, di.dim, di.n, dom, lane);
+        load_family<float>(u.rnd.fam32[warp], fid, di.dim, a.params + di.par_off, lane);
+        if (lane < di.dim) u.rnd.a[warp][lane] = (double)(float)a.params[di.par_off + 2 + lane];
+      } else {
+        geo_setup<double, D>(u.rnd.g64[warp], di.rule, di.dim, di.n, dom, lane);
+        load_family<double>(u.rnd.fam64[warp], fid, di.dim, a.params + di.par_off, lane);
+        if (lane < di.dim) u.rnd.a[warp][lane] = a.params[di.par_off + 2 + lane];
+      }
+    }
     __syncthreads();
-    for (int r = 0; r < nw && base + (int64_t)r * gridDim.x < a.n_int; ++r) {
+    for (int r = 0; r < nw && base + r * a.fact < a.n_int; ++r) {
       if (!tsep[r]) continue;
-      setup(r);
-      const int64_t tile = ts[r];
-      if (kF32 && d.rule != TQ_RULE_GAUSS)
-        batch_adj_sep_dispatch<float>(a, d, tile, g32, fam32, dsum, sp);
+      const tq_batch_desc& dr = u.rnd.d[r];
+      if (kF32 && dr.rule != TQ_RULE_GAUSS)
+        batch_adj_sums<float>(a, dr, u.rnd.g32[r], u.rnd.fam32[r], u.rnd.dsum[r], u.rnd.sp);
       else
-        batch_adj_sep_dispatch<double>(a, d, tile, g64, fam64, dsum, sp);
-      const int64_t cells = (te[r] - tile - 1) * a.stride;
-      for (int64_t e = threadIdx.x; e < cells; e += blockDim.x) a.partials[(tile + 1) * a.stride + e] = 0.0;
-      __syncthreads();
+        batch_adj_sums<double>(a, dr, u.rnd.g64[r], u.rnd.fam64[r], u.rnd.dsum[r], u.rnd.sp);
+      // sep_sums ends with a barrier: sp may be rewritten, dsum[r] be read
+    }
+    if (mine < a.n_int && tsep[warp]) {
+      const tq_batch_desc& dr = u.rnd.d[warp];
+      batch_adj_products(a.family >= 0 ? a.family : dr.family, u.rnd.dsum[warp], u.rnd.a[warp], dr.dim,
+                         a.partials + ts[warp] * a.stride);
     }
     __syncthreads();  // the round's tables are rewritten
   }
@@ -779,8 +828,12 @@ __global__ void batch_adjoint_finalize_kernel(BatchGradArgs a, double* out_value
   __shared__ double tot[kBlock / 32][2 + 4 * 8];
   if (w >= a.n_int) return;
   const tq_batch_desc d = a.desc[w];
-  const int nacc = 2 + 4 * d.dim;
+  int nacc = 2 + 4 * d.dim;
   const int64_t t0 = a.tile_start[w], t1 = a.tile_start[w + 1];
+  if (batch_adj_factors<D>(a, d)) {  // the sums stand in the first tile's row
+    for (int i = lane; i < nacc; i += 32) tot[wib][i] = a.partials[t0 * a.stride + i];
+    nacc = 0;
+  }
   for (int i = 0; i < nacc; ++i) {
     Acc s{0.0, 0.0};
     for (int64_t t = t0 + lane; t < t1; t += 32) acc_add(s, a.partials[t * a.stride + i]);
@@ -994,6 +1047,12 @@ extern "C" int tq_batch_grid_adjoint(int dtype, int64_t n_integrals, const void*
   a.partials = (double*)workspace;
   int64_t grid = (int64_t)sm_count() * 4;
   if (grid > n_tiles) grid = n_tiles;
+  // The factored integrals go to the CTAs resident at once, so that each has
+  // several of them and no second wave sets itself up for one or two: 1024
+  // integrals of d = 4, 32 nodes, 121 us over all CTAs, 107 this way (tiles
+  // are better spread over all: 3464 against 3597 us for 256 by nodes).
+  const int64_t resident = (int64_t)sm_count() * (max_dim <= 4 ? 2 : 1);
+  a.fact = grid < resident ? grid : resident;
   cudaStream_t s = (cudaStream_t)stream;
   const unsigned g = (unsigned)grid;
   if (dtype == TQ_F64) {

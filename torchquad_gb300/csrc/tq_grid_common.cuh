@@ -49,8 +49,7 @@ __host__ __device__ __forceinline__ double nc_den(int rule) {
 // first use): the two fp64 divisions of a dimension cost thousands of cycles
 // when one thread does the dimensions in turn.
 template <typename T, typename D>
-__device__ void geo_setup(Geo<T>& g, int rule, int dim, int64_t n, const D* __restrict__ dom) {
-  const int k = threadIdx.x;
+__device__ void geo_setup(Geo<T>& g, int rule, int dim, int64_t n, const D* __restrict__ dom, int k = threadIdx.x) {
   if (k < dim) {
     const D a = dom[2 * k], b = dom[2 * k + 1];
     g.a[k] = (T)a;
