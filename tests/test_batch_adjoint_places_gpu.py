@@ -1,4 +1,4 @@
-"""Batched adjoint over several rounds of factored integrals: an integral's
+"""Batched adjoint with more factored integrals than warps: an integral's
 value and gradients do not depend on where in a batch it stands, beside
 factored and node-by-node integrals of other families and dimensions."""
 import numpy as np
