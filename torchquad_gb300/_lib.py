@@ -332,12 +332,15 @@ def body_stream(device, avoid=()) -> torch.cuda.Stream:
 
 
 def plain_tensor(t) -> bool:
-    """Whether t is an ordinary tensor (or parameter) with memory of its own,
-    outside every transform that follows torch operations (tracing, vmap and
-    other functorch levels, forward-mode derivatives), so that a kernel may
-    take the place of torch operations on it.  Gradients are the caller's to
-    look at."""
+    """Whether t is an ordinary tensor (or parameter) whose memory holds its
+    values, outside every transform that follows torch operations (tracing,
+    vmap and other functorch levels, forward-mode derivatives), so that a
+    kernel may take the place of torch operations on it.  Lazily negated or
+    conjugated views do not qualify (the gradient of a conjugated number's
+    imaginary part is one), nor do zero tensors without memory.  Gradients are
+    the caller's to look at."""
     return (type(t) in (torch.Tensor, torch.nn.Parameter) and torch._C._has_storage(t)
+            and not t.is_neg() and not t.is_conj() and not t._is_zerotensor()
             and not torch.jit.is_tracing() and fwAD._current_level < 0
             and torch._C._functorch.peek_interpreter_stack() is None)
 
