@@ -118,12 +118,15 @@ class BuiltinIntegrand:
         """The device parameter vector for launches on the current stream.
         Parameters that live on the device are gathered there by one launch;
         reading them back would wait for everything queued before.  The
-        second call with the same parameters keeps the vector (device_params)."""
+        second call with the same parameters keeps the vector (device_params),
+        unless it is captured into a CUDA graph, where nothing can be read
+        back."""
         ts = (self.c, self.b, self.a, self.u)
         if not any(t.is_cuda for t in ts):
             return self.device_params(device)
         key = self._params_key()
-        if key == self._np_key or key == self._packed_key or not self._packable(ts, device):
+        again = key == self._packed_key and not torch.cuda.is_current_stream_capturing()
+        if key == self._np_key or again or not self._packable(ts, device):
             return self.device_params(device)
         self._packed_key = key
         host = [0.0] * (2 + 2 * self.dim)
