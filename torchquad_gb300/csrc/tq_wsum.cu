@@ -37,6 +37,7 @@
 #include <type_traits>
 
 #include "tq_grid_common.cuh"
+#include "tq_ranges.cuh"
 
 namespace tq {
 
@@ -47,10 +48,8 @@ constexpr int kComps = 32;    // components per warp of the vector kernel
 struct WsumArgs {
   int rule, dim;
   int m;                  // joined inner dimensions
-  int64_t n, start, count, n_values;
-  int64_t R;              // nodes per row, n^m (Monte Carlo: count)
-  int64_t row0, rows;     // rows the range touches
-  int64_t seg, segs;      // nodes per segment, segments per row
+  int64_t n, n_values;
+  RowWalk w;              // the range; a row has n^m nodes (Monte Carlo: all of them)
   int chunk;              // components per CTA (vector kernel)
   const void* domain;
   const double* gl_weights;
@@ -79,7 +78,7 @@ __device__ __forceinline__ void wsum_store(const WsumArgs& a, int64_t s, Acc t) 
     const D* dom = (const D*)a.domain;
     D vol = (D)1;
     for (int k = 0; k < a.dim; ++k) vol = vol * (D)(dom[2 * k + 1] - dom[2 * k]);
-    v *= (double)vol / (double)a.count;
+    v *= (double)vol / (double)a.w.count;
   }
   if (a.out_dtype == TQ_F64)
     ((double*)a.out)[s] = v;
@@ -101,7 +100,7 @@ __device__ __forceinline__ F wsum_weight(int rule, int j, bool end) {
 template <bool GL>
 __device__ void wsum_join_table(const WsumArgs& a, double* tab) {
   const uint32_t n = (uint32_t)a.n;
-  for (int j = threadIdx.x; j < (int)a.R; j += blockDim.x) {
+  for (int j = threadIdx.x; j < (int)a.w.R; j += blockDim.x) {
     uint32_t r = (uint32_t)j;
     double w = 1.0;
     for (int k = 0; k < a.m; ++k) {
@@ -137,10 +136,6 @@ __device__ __forceinline__ double wsum_outer(const WsumArgs& a, const FastDiv& f
     }
   }
   return w;
-}
-
-__device__ __forceinline__ int64_t unit_row(const WsumArgs& a, int64_t u) {
-  return a.rows == 1 ? 0 : (a.segs == 1 ? u : u / a.segs);
 }
 
 // A double split into two floats by integer operations alone (no FP64
@@ -367,33 +362,31 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_kernel(WsumArgs a) {
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = (int64_t)gridDim.x * (kBlock / 32);
   const int64_t gw = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  const int64_t units = a.rows * a.segs, end = a.start + a.count;
+  const int64_t units = row_units(a.w), start = a.w.start, end = start + a.w.count;
   const int64_t ub = gw * units / nwarps, ue = (gw + 1) * units / nwarps;
   const double wi = wsum_weight<double>(a.rule, lane, false);
   for (int64_t u0 = ub; u0 < ue; u0 += 32) {
     const int cnt = (int)min((int64_t)32, ue - u0);
     double w = 0.0;  // outer weight of unit u0 + lane
     if (lane < cnt) {
-      const int64_t row = unit_row(a, u0 + lane);
-      w = wsum_outer<GL>(a, su.fd, a.row0 + row);
+      const RowPart pt = row_part(a.w, u0 + lane);
+      w = wsum_outer<GL>(a, su.fd, a.w.row0 + pt.row);
       if (ONE) {
-        const int64_t j0 = (u0 + lane - row * a.segs) * a.seg, p0 = (a.row0 + row) * a.R, p1 = p0 + a.R - 1;
+        const int64_t p0 = pt.r0, p1 = p0 + a.w.R - 1;
         double e = 0.0;
-        if (j0 == 0 && p0 >= a.start && p0 < end) e = (double)__ldg(f + (p0 - a.start));
-        if (j0 + a.seg >= a.R && p1 >= a.start && p1 < end) e += (double)__ldg(f + (p1 - a.start));
+        if (pt.j0 == 0 && p0 >= start && p0 < end) e = (double)__ldg(f + (p0 - start));
+        if (pt.j0 + a.w.seg >= a.w.R && p1 >= start && p1 < end) e += (double)__ldg(f + (p1 - start));
         ends = fma(-0.5 * wsum_weight<double>(a.rule, 0, false) * e, w, ends);
       }
     }
     F2 wf{0.f, 0.f};
     if (F32 || PAIR) wf = f2_from_double(w);
     for (int q = 0; q < cnt; ++q) {
-      const int64_t u = u0 + q;
-      const int64_t row = unit_row(a, u);
-      const int64_t j0 = (u - row * a.segs) * a.seg;            // segment [j0, j1) of its row
-      const int64_t r0 = (a.row0 + row) * a.R;                  // the row's first node
-      const int lo = (int)max(a.start - r0 - j0, (int64_t)0);   // the part inside the range: [lo, len)
-      const int len = (int)(min(min(j0 + a.seg, a.R), end - r0) - j0);
-      const F* fr = f + (r0 - a.start) + j0 + lane;
+      const RowPart pt = row_part(a.w, u0 + q);
+      const int64_t j0 = pt.j0;
+      const int lo = pt.lo, len = pt.len;
+      if (lo >= len) continue;
+      const F* fr = f + (pt.r0 - start) + j0 + lane;
       const double wq = __shfl_sync(0xffffffffu, w, q);
       Unit us;
       // N values a lane from offset i
@@ -465,14 +458,14 @@ __global__ void __launch_bounds__(kBlock, 4) sample_sum_kernel(WsumArgs a) {
   const int64_t step = (int64_t)gridDim.x * kBlock;
   ExactSum<F> sum;
   int64_t i = (int64_t)blockIdx.x * kBlock + threadIdx.x;
-  for (; i + 7 * step < a.count; i += 8 * step) {
+  for (; i + 7 * step < a.w.count; i += 8 * step) {
     F v[8];
 #pragma unroll
     for (int p = 0; p < 8; ++p) v[p] = __ldg(f + i + p * step);
 #pragma unroll
     for (int p = 0; p < 8; ++p) sum.add(v[p]);
   }
-  for (; i < a.count; i += step) sum.add(__ldg(f + i));
+  for (; i < a.w.count; i += step) sum.add(__ldg(f + i));
   wsum_finish<D>(a, sum.value(), 1.0);
 }
 
@@ -497,26 +490,23 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_vec_kernel(WsumArgs a)
   const int sub = lane / ncomp, comp = lane - sub * ncomp;
   const F* __restrict__ f = (const F*)a.f + s0 + comp;
   const int64_t nwarps = (int64_t)gridDim.x * (kBlock / 32);
-  const int64_t units = a.rows * a.segs, end = a.start + a.count;
+  const int64_t units = row_units(a.w);
   ExactSum<F> sum;
   for (int64_t u = (int64_t)warp * gridDim.x + blockIdx.x; u < units; u += nwarps) {
-    const int64_t row = unit_row(a, u);
-    const int64_t j0 = (u - row * a.segs) * a.seg;
-    const int64_t r0 = (a.row0 + row) * a.R;
-    const int64_t b = max(j0, a.start - r0);
-    const int64_t j1 = min(min(j0 + a.seg, a.R), end - r0);
-    const double wo = mc ? 1.0 : wsum_outer<GL>(a, su.fd, a.row0 + row);
-    for (int64_t jb = b; jb < j1; jb += batch) {
+    const RowPart pt = row_part(a.w, u);
+    const int64_t j1 = pt.j0 + pt.len;
+    const double wo = mc ? 1.0 : wsum_outer<GL>(a, su.fd, a.w.row0 + pt.row);
+    for (int64_t jb = pt.j0 + pt.lo; jb < j1; jb += batch) {
       const int nb = (int)min((int64_t)batch, j1 - jb);
       double w = 0.0;  // weight of the batch's node `lane`
       F2 wf{0.f, 0.f};
       if (!mc) {
         const int64_t j = jb + min(lane, nb - 1);
         w = wo * (JOIN ? tab[j] : GL ? __ldg(a.gl_weights + j)
-                                     : wsum_weight<double>(a.rule, (int)(j & 3), j == 0 || j == a.R - 1));
+                                     : wsum_weight<double>(a.rule, (int)(j & 3), j == 0 || j == a.w.R - 1));
         if (F32) wf = f2_from_double(w);
       }
-      const F* fr = f + (r0 - a.start + jb) * S;
+      const F* fr = f + (pt.r0 - a.w.start + jb) * S;
       for (int i = 0; i < nb; i += 8 * per) {
         F v[8];
 #pragma unroll
@@ -645,8 +635,6 @@ static int wsum_launch(int dtype, int rule, int dim, int64_t n_per_dim, const vo
   a.rule = rule;
   a.dim = dim;
   a.n = n_per_dim;
-  a.start = start;
-  a.count = count;
   a.n_values = n_values;
   a.domain = domain;
   a.gl_weights = gl_weights;
@@ -660,18 +648,16 @@ static int wsum_launch(int dtype, int rule, int dim, int64_t n_per_dim, const vo
   // rows of at least 32 nodes: join the inner dimensions of short ones (a
   // lane would otherwise fold an outer weight in, in FP64, every few values)
   a.m = mc ? dim : 1;
-  a.R = mc ? count : n_per_dim;
+  int64_t R = mc ? count : n_per_dim;
   if (mc) {  // one row of all the samples
-    a.start = 0;
+    start = 0;
   } else {
-    while (a.R < 32 && a.m < dim && a.R * n_per_dim <= kJoin) {
-      a.R *= n_per_dim;
+    while (R < 32 && a.m < dim && R * n_per_dim <= kJoin) {
+      R *= n_per_dim;
       ++a.m;
     }
   }
   const bool join = !mc && a.m > 1;
-  a.row0 = a.start / a.R;
-  a.rows = (a.start + count - 1) / a.R - a.row0 + 1;
   // double-float sums where enough nodes share them that their 2^-47 of a term
   // is below the sum's own last bit; few nodes, and long rows, in fp64
   const bool pair = f_dtype == TQ_F64 && n_values == 1 && !mc && !gl && !join && n_per_dim >= 32 &&
@@ -681,9 +667,9 @@ static int wsum_launch(int dtype, int rule, int dim, int64_t n_per_dim, const vo
   // segments: long, unless that leaves warps without work
   const int64_t warps = gx * (kBlock / 32);
   const int64_t least = n_values == 1 ? 128 : 32;
-  a.seg = 2048;
-  while (a.seg / 2 >= least && a.rows * ((a.R + a.seg - 1) / a.seg) < warps) a.seg /= 2;
-  a.segs = (a.R + a.seg - 1) / a.seg;
+  int64_t seg = 2048;
+  while (seg / 2 >= least && row_units(make_walk(start, count, R, seg)) < warps) seg /= 2;
+  a.w = make_walk(start, count, R, seg);
   cudaStream_t s = (cudaStream_t)stream;
   const int64_t chunks = (n_values + kComps - 1) / kComps;
   a.chunk = (int)(n_values < kComps ? n_values : kComps);
