@@ -1,6 +1,6 @@
 """The rows and segments that the weighted sums walk for a range of nodes
 (csrc/tq_ranges.cuh, compiled for the host): every unit's reads lie inside the
-range's values and the units cover the range once and in order, also where
+range's values, no unit is empty and they cover the range once and in order, also where
 the distances between a segment and the range leave 32 bits."""
 import ctypes
 import random
@@ -16,10 +16,10 @@ SHIM = """
 extern "C" int64_t check_walk(int64_t start, int64_t count, int64_t R, int64_t seg) {
   const tq::RowWalk w = tq::make_walk(start, count, R, seg);
   int64_t next = 0, u = 0;
-  for (const int64_t n = tq::row_units(w); u < n; ++u) {
+  for (; u < w.units; ++u) {
     const tq::RowPart p = tq::row_part(w, u);
     if (p.lo < 0 || p.len < 0 || p.len > w.seg || p.j0 + p.len > R) return u + 1;
-    if (p.lo >= p.len) continue;
+    if (p.lo >= p.len) return u + 1;  // a unit without nodes leaves a warp idle
     const int64_t first = p.r0 - w.start + p.j0 + p.lo;  // the value read first
     if (first != next || p.r0 != (w.row0 + p.row) * R) return u + 1;
     next += p.len - p.lo;

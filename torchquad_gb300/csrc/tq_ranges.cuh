@@ -18,10 +18,11 @@ struct RowWalk {
   int64_t R;             // nodes per row
   int64_t row0, rows;    // rows the range touches
   int64_t seg, segs;     // nodes per segment, segments per row
+  int64_t unit0, units;  // the segments that meet the range, counted from row0's first
 };
 
-// Unit u of the walk: the segment from node j0 of its row, of whose nodes
-// [lo, len) are in the range (none where lo >= len).
+// Unit u < units of the walk: the segment from node j0 of its row, of whose
+// nodes [lo, len) are in the range.
 struct RowPart {
   int64_t row;  // counted from row0
   int64_t r0;   // flat index of the row's first node
@@ -29,15 +30,12 @@ struct RowPart {
   int lo, len;
 };
 
-TQ_HD int64_t row_units(const RowWalk& w) { return w.rows * w.segs; }
-
-TQ_HD int64_t unit_row(const RowWalk& w, int64_t u) { return w.rows == 1 ? 0 : (w.segs == 1 ? u : u / w.segs); }
-
 // A row can be the whole grid, so the distances between a segment and the
 // range are clipped to the segment before they become ints.
 TQ_HD RowPart row_part(const RowWalk& w, int64_t u) {
   RowPart p;
-  p.row = unit_row(w, u);
+  u += w.unit0;
+  p.row = w.rows == 1 ? 0 : (w.segs == 1 ? u : u / w.segs);
   p.r0 = (w.row0 + p.row) * w.R;
   p.j0 = (u - p.row * w.segs) * w.seg;
   const int64_t lo = w.start - p.r0 - p.j0;
@@ -58,6 +56,11 @@ TQ_HD RowWalk make_walk(int64_t start, int64_t count, int64_t R, int64_t seg) {
   w.rows = (start + count - 1) / R - w.row0 + 1;
   w.seg = seg;
   w.segs = (R + seg - 1) / seg;
+  // A one-dimensional grid is one row: a range of it is a part of the row's
+  // segments, and its units alone are shared out over the warps.  (With the
+  // units of the whole row, a range of 1/8 left 7/8 of the warps idle.)
+  w.unit0 = (start - w.row0 * R) / seg;
+  w.units = (w.rows - 1) * w.segs + (start + count - 1 - (w.row0 + w.rows - 1) * R) / seg + 1 - w.unit0;
   return w;
 }
 

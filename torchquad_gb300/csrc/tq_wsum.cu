@@ -362,7 +362,7 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_kernel(WsumArgs a) {
   const int lane = threadIdx.x & 31;
   const int64_t nwarps = (int64_t)gridDim.x * (kBlock / 32);
   const int64_t gw = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-  const int64_t units = row_units(a.w), start = a.w.start, end = start + a.w.count;
+  const int64_t units = a.w.units, start = a.w.start, end = start + a.w.count;
   const int64_t ub = gw * units / nwarps, ue = (gw + 1) * units / nwarps;
   const double wi = wsum_weight<double>(a.rule, lane, false);
   for (int64_t u0 = ub; u0 < ue; u0 += 32) {
@@ -385,7 +385,6 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_kernel(WsumArgs a) {
       const RowPart pt = row_part(a.w, u0 + q);
       const int64_t j0 = pt.j0;
       const int lo = pt.lo, len = pt.len;
-      if (lo >= len) continue;
       const F* fr = f + (pt.r0 - start) + j0 + lane;
       const double wq = __shfl_sync(0xffffffffu, w, q);
       Unit us;
@@ -490,7 +489,7 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_vec_kernel(WsumArgs a)
   const int sub = lane / ncomp, comp = lane - sub * ncomp;
   const F* __restrict__ f = (const F*)a.f + s0 + comp;
   const int64_t nwarps = (int64_t)gridDim.x * (kBlock / 32);
-  const int64_t units = row_units(a.w);
+  const int64_t units = a.w.units;
   ExactSum<F> sum;
   for (int64_t u = (int64_t)warp * gridDim.x + blockIdx.x; u < units; u += nwarps) {
     const RowPart pt = row_part(a.w, u);
@@ -668,7 +667,7 @@ static int wsum_launch(int dtype, int rule, int dim, int64_t n_per_dim, const vo
   const int64_t warps = gx * (kBlock / 32);
   const int64_t least = n_values == 1 ? 128 : 32;
   int64_t seg = 2048;
-  while (seg / 2 >= least && row_units(make_walk(start, count, R, seg)) < warps) seg /= 2;
+  while (seg / 2 >= least && make_walk(start, count, R, seg).units < warps) seg /= 2;
   a.w = make_walk(start, count, R, seg);
   cudaStream_t s = (cudaStream_t)stream;
   const int64_t chunks = (n_values + kComps - 1) / kComps;
