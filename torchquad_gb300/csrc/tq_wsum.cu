@@ -13,7 +13,8 @@
 // longer than the loads and all other work of a value, so:
 //   fp64 values   pairs of a lane's values added in fp64, the sums of pairs as
 //                 double-floats (one weight a lane), or one FP64 fused
-//                 multiply-add a value (Gauss weights, joined rows)
+//                 multiply-add a value (Gauss weights, joined rows), groups of
+//                 up to 32 values of a lane then added exactly
 //   fp32 values   a compensated fp32 sum per segment and a double-float sum
 //                 of the segments, no FP64 instruction per value
 // Monte Carlo, and several values per node (vector integrands): sums that
@@ -29,7 +30,7 @@
 //
 // Measured (GB300), before and after: 301^3 fp64 values 96 us (double-floats
 // split from each value, 75 instructions a value) and 58 us (3.7 TB/s); 301^3
-// fp32 77 and 43 us; 15^6 fp64 475 and 39 us (outer weights per value strip);
+// fp32 77 and 43 us; 15^6 fp64 475 and 45 us (outer weights per value strip);
 // 10001 nodes x 200 components fp32 969 and 26 us (one component per thread
 // and node group: uncoalesced, eight FP64 operations a value); 10^6 Monte
 // Carlo values fp64 96 and 14 us.
@@ -212,20 +213,39 @@ struct UnitSumP {
 
 // A lane's sum over its units, each folded in with its outer weight w: in
 // fp64, or as double-floats, with unit sums of 2^60 and more (and infinities
-// and NaN) in the fp64 side sum.
+// and NaN) in the fp64 side sum.  In fp64, groups of up to 32 values of a lane
+// are added plainly and the groups' sums exactly, by integers (a Neumaier
+// pair's seven FP64 operations a group: 8e7 nodes 211 us, plain sums 177).
 struct LaneSumD {
   double s = 0.0;
-  __device__ __forceinline__ void fold(const UnitSumD& u, double w, F2, double*) { s = fma(u.s, w, s); }
-  __device__ __forceinline__ Acc value() const { return Acc{s, 0.0}; }
+  FixAcc t;
+  int k = 0;          // values in s; the same in the whole warp
+  bool many = false;  // t holds groups
+  __device__ __forceinline__ void fold(const UnitSumD& u, int n, double w, F2, double*) {
+    if (k + n > 32) {
+      t.add(s);
+      many = true;
+      s = 0.0;
+      k = 0;
+    }
+    s = fma(u.s, w, s);
+    k += n;
+  }
+  __device__ __forceinline__ Acc value() const {
+    if (!many) return Acc{s, 0.0};
+    Acc r = t.value();
+    acc_add(r, s);
+    return r;
+  }
 };
 struct LaneSumF {
   F2 s{0.f, 0.f};
-  __device__ __forceinline__ void fold(const UnitSumF& u, double w, F2 wf, double* side) {
+  __device__ __forceinline__ void fold(const UnitSumF& u, int, double w, F2 wf, double* side) {
     const bool in = fabsf(u.s) < 0x1p60f;
     if (in) s = f2_add(s, f2_mul(two_sum(u.s, -u.c), wf));
     if (__any_sync(0xffffffffu, !in)) side_add(side, in ? 0.0 : w, in ? 0.0 : (double)u.s - (double)u.c);
   }
-  __device__ __forceinline__ void fold(const UnitSumP& u, double, F2 wf, double*) {
+  __device__ __forceinline__ void fold(const UnitSumP& u, int, double, F2 wf, double*) {
     s = f2_add(s, f2_mul(two_sum(u.hi, u.lo), wf));
   }
   __device__ __forceinline__ Acc value() const { return Acc{(double)s.hi, (double)s.lo}; }
@@ -437,7 +457,7 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_kernel(WsumArgs a) {
       for (; i < len; i += 64) batch(i, std::false_type{}, std::integral_constant<int, 2>{});
       F2 wqf{0.f, 0.f};
       if (F32 || PAIR) wqf = F2{__shfl_sync(0xffffffffu, wf.hi, q), __shfl_sync(0xffffffffu, wf.lo, q)};
-      sum.fold(us, wq, wqf, &side);
+      sum.fold(us, (len - lo + 31) / 32, wq, wqf, &side);  // at most so many values a lane
     }
   }
   Acc r = sum.value();
@@ -663,10 +683,11 @@ static int wsum_launch(int dtype, int rule, int dim, int64_t n_per_dim, const vo
                     n_per_dim <= kPairMax && (dim - 1) * n_per_dim <= kPairMax;
   int64_t gx = wsum_ctas(count, n_values);
   if (gx > slots / n_values) gx = slots / n_values;
-  // segments: long, unless that leaves warps without work
+  // segments: long (a lane's 32 values where its groups of fp64 values end),
+  // unless that leaves warps without work
   const int64_t warps = gx * (kBlock / 32);
   const int64_t least = n_values == 1 ? 128 : 32;
-  int64_t seg = 2048;
+  int64_t seg = f_dtype == TQ_F64 && n_values == 1 && !pair ? 1024 : 2048;
   while (seg / 2 >= least && make_walk(start, count, R, seg).units < warps) seg /= 2;
   a.w = make_walk(start, count, R, seg);
   cudaStream_t s = (cudaStream_t)stream;
