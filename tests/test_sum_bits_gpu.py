@@ -1,5 +1,8 @@
 """GPU: how many bits the sums keep, by inputs whose exact sum is known and
 of which shorter sums lose a visible part."""
+from fractions import Fraction
+
+import numpy as np
 import pytest
 import torch
 
@@ -26,3 +29,21 @@ def test_long_fp64_row(cuda):
     v = 1.0 + 2.0**-47
     got = total(T, 1, n, torch.full((n, 1), v, dtype=torch.float64, device=cuda), cuda)
     assert abs(got - v) <= 2.0**-51, got - v
+
+
+@pytest.mark.parametrize("S_", [1, 3])
+@pytest.mark.parametrize("dim,n", [(5, 13), (3, 33)])
+def test_scale_of_the_weights(dim, n, S_, cuda):
+    """Ones: the result is the product of the dimensions' weight scales times
+    a whole number, rounded once (the product itself to about 2^-104)."""
+    rng = np.random.default_rng(dim)
+    for _ in range(20):
+        dom = [[0.0, float(w)] for w in rng.uniform(0.3, 3.0, dim)]
+        want = Fraction(1)
+        for _, b in dom:
+            step = b / (n - 1)  # the second node less the first (0)
+            want *= Fraction(step / 2.0) * (2 * (n - 1))
+        d = torch.tensor(dom, dtype=torch.float64, device=cuda)
+        ones = torch.ones(n**dim, S_, dtype=torch.float64, device=cuda)
+        for got in K.weighted_result(T, dim, n, d, None, 0, ones, torch.float64).tolist():
+            assert abs(Fraction(got) - want) <= want * Fraction(1.01 * 2.0**-53), (got, float(want))

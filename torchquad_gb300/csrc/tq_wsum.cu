@@ -320,35 +320,34 @@ struct ExactSum<float> {
 };
 
 // Shared set-up of the kernels: the product of the dimensions' weight scales
-// (a CTA's sums take it at the very end, in fp64: folded into the rows'
-// double-float weights it would be rounded to 2^-48 for all of them alike) and
-// the join table.
+// (a CTA's sums take it at the very end, so its rounding is the same for all
+// nodes: a pair, by a warp of its own while the others read; visible from the
+// next barrier on) and the join table.
 struct WsumSetup {
-  double scale;
+  Acc scale;
   FastDiv fd;
 };
+// v s for unevaluated pairs
+__device__ __forceinline__ Acc wsum_scaled(Acc v, Acc s) {
+  const double p = v.s * s.s;
+  return Acc{p, fma(v.c, s.s, fma(v.s, s.c, fma(v.s, s.s, -p)))};
+}
 template <typename T, typename D, bool GL, bool JOIN>
 __device__ __forceinline__ void wsum_setup(const WsumArgs& a, Geo<T>& g, WsumSetup& su, double* tab) {
   geo_setup<T, D>(g, a.rule, a.dim, a.n, (const D*)a.domain);
   if constexpr (JOIN) wsum_join_table<GL>(a, tab);
+  if (threadIdx.x == 0) su.fd = make_fastdiv((uint32_t)a.n);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 1.0;
-    for (int k = 0; k < a.dim; ++k) s *= g.wscale[k];
+  if (threadIdx.x == kBlock - 32) {
+    Acc s{g.wscale[0], 0.0};
+    for (int k = 1; k < a.dim; ++k) s = wsum_scaled(s, Acc{g.wscale[k], 0.0});
     su.scale = s;
-    su.fd = make_fastdiv((uint32_t)a.n);
   }
-  __syncthreads();
-}
-// (hi + lo) times s, rounded once
-__device__ __forceinline__ Acc wsum_scaled(Acc v, double s) {
-  const double p = v.s * s;
-  return Acc{p, fma(v.c, s, fma(v.s, s, -p))};
 }
 
 // The CTAs' sums into the running sum or the result, by the last of them.
 template <typename D>
-__device__ __forceinline__ void wsum_finish(const WsumArgs& a, Acc mine, double scale) {
+__device__ __forceinline__ void wsum_finish(const WsumArgs& a, Acc mine, const Acc& scale) {
   const Acc acc = block_reduce<kBlock>(mine);
   if (threadIdx.x == 0) a.partials[blockIdx.x] = wsum_scaled(acc, scale);
   if (last_block_arrives(a.ticket)) {
@@ -485,7 +484,7 @@ __global__ void __launch_bounds__(kBlock, 4) sample_sum_kernel(WsumArgs a) {
     for (int p = 0; p < 8; ++p) sum.add(v[p]);
   }
   for (; i < a.w.count; i += step) sum.add(__ldg(f + i));
-  wsum_finish<D>(a, sum.value(), 1.0);
+  wsum_finish<D>(a, sum.value(), Acc{1.0, 0.0});
 }
 
 // Several values per node: lane = component + chunk * node, partials[CTA of
