@@ -47,3 +47,17 @@ def test_scale_of_the_weights(dim, n, S_, cuda):
         ones = torch.ones(n**dim, S_, dtype=torch.float64, device=cuda)
         for got in K.weighted_result(T, dim, n, d, None, 0, ones, torch.float64).tolist():
             assert abs(Fraction(got) - want) <= want * Fraction(1.01 * 2.0**-53), (got, float(want))
+
+
+@pytest.mark.parametrize("bits", [60, 90, 105])
+@pytest.mark.parametrize("rule", [L.TQ_RULE_MC, T])
+def test_values_that_cancel(rule, bits, cuda):
+    """2^bits, a small value and -2^bits in different lanes: the sums over the
+    lanes keep the small one (bits of a value down to 2^-106 of the largest)."""
+    n = 2 if rule == L.TQ_RULE_MC else 5
+    values = torch.zeros(n**2, 1, dtype=torch.float64, device=cuda)
+    at = [0, 1, 2] if rule == L.TQ_RULE_MC else [6, 7, 8]  # interior nodes of equal weight
+    values[at, 0] = torch.tensor([2.0**bits, 1.5, -(2.0**bits)], dtype=torch.float64, device=cuda)
+    got = total(rule, 2, n, values, cuda, width=4.0)
+    want = 1.5 * 16.0 / 4 if rule == L.TQ_RULE_MC else 1.5
+    assert got == want

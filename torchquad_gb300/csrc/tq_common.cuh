@@ -69,35 +69,39 @@ __device__ __forceinline__ Acc acc_shfl_down(const Acc& a, int off) {
 // CTA takes about 130 dependent FP64 warp instructions, and on GB300 each
 // holds a sub-partition's FP64 unit for about 64 cycles (4 us a reduction,
 // more than the work of a small launch).  Here every value is placed in a
-// 96-bit window below the CTA's largest binary exponent, as four signed
-// 24-bit limbs (integer shifts only), the limbs are summed over a warp by
-// redux.sync and over the CTA as 64-bit integers, and one thread turns the
-// total into hi + lo doubles by bit moves.  Integer sums are exact and do
-// not depend on their order; a value loses only bits below 2^-95 of the
-// largest.  A 101^3 fused Simpson launch by nodes (252 CTAs): 26.4 us with the
+// 112-bit window below the CTA's largest binary exponent, as five signed
+// limbs of 24 bits (the lowest of 16; integer shifts only), the limbs are
+// summed over a warp by redux.sync and over the CTA as 64-bit integers, and
+// one thread turns the total into hi + lo doubles by bit moves.  Integer sums
+// are exact and do not depend on their order; a value loses only bits below
+// 2^-111 of the largest (the pair hi + lo holds 106).  A 101^3 fused Simpson launch by nodes (252 CTAs): 26.4 us with the
 // fp64 trees, 18.7 us with these sums and the dimensions set up in parallel; a
 // 10001-node rule over 200 components (50 reductions a component group): 969
 // and 431 us.
 __device__ __forceinline__ int exp_field(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
 
-// L += v in units of 2^(emax - 1118) (limb i has weight 2^(24 i)); v finite,
-// its exponent field at most emax, emax >= 1.
-__device__ __forceinline__ void fix_add(int (&L)[4], double v, int emax) {
+constexpr int kLimbs = 5;  // limb 0 has weight 1, limb i > 0 weight 2^(24 i - 8)
+
+// L += v in units of 2^(emax - 1134); v finite, its exponent field at most
+// emax, emax >= 1.
+__device__ __forceinline__ void fix_add(int (&L)[kLimbs], double v, int emax) {
   const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
   const int ef = (int)(hi >> 20) & 0x7ff;
   const uint32_t mh = (hi & 0xfffffu) | (ef ? 0x100000u : 0u);
   const int s = emax - (ef ? ef : 1);
-  const uint32_t w2 = (mh << 11) | (lo >> 21), w1 = lo << 11;  // mantissa << 43, 96 bits
-  uint32_t a2 = w2 >> (s & 31), a1 = __funnelshift_r(w1, w2, s), a0 = __funnelshift_r(0u, w1, s);
+  const uint32_t w3 = (mh << 11) | (lo >> 21), w2 = lo << 11;  // mantissa << 75, 128 bits
+  uint32_t a3 = w3 >> (s & 31), a2 = __funnelshift_r(w2, w3, s), a1 = __funnelshift_r(0u, w2, s), a0 = 0u;
   const int q = s >> 5;
-  a0 = q == 0 ? a0 : q == 1 ? a1 : q == 2 ? a2 : 0u;
-  a1 = q == 0 ? a1 : q == 1 ? a2 : 0u;
-  a2 = q == 0 ? a2 : 0u;
+  a0 = q == 1 ? a1 : q == 2 ? a2 : q == 3 ? a3 : 0u;
+  a1 = q == 0 ? a1 : q == 1 ? a2 : q == 2 ? a3 : 0u;
+  a2 = q == 0 ? a2 : q == 1 ? a3 : 0u;
+  a3 = q == 0 ? a3 : 0u;
   const int sg = (int)hi >> 31;
-  L[0] += ((int)(a0 & 0xffffffu) ^ sg) - sg;
-  L[1] += ((int)(__funnelshift_r(a0, a1, 24) & 0xffffffu) ^ sg) - sg;
-  L[2] += ((int)(__funnelshift_r(a1, a2, 16) & 0xffffffu) ^ sg) - sg;
-  L[3] += ((int)(a2 >> 8) ^ sg) - sg;
+  L[0] += ((int)(a0 >> 16) ^ sg) - sg;
+  L[1] += ((int)(a1 & 0xffffffu) ^ sg) - sg;
+  L[2] += ((int)(__funnelshift_r(a1, a2, 24) & 0xffffffu) ^ sg) - sg;
+  L[3] += ((int)(__funnelshift_r(a2, a3, 16) & 0xffffffu) ^ sg) - sg;
+  L[4] += ((int)(a3 >> 8) ^ sg) - sg;
 }
 
 // The leading 53 bits of A 2^p as a double (truncated); A keeps the rest.
@@ -118,14 +122,16 @@ __device__ __forceinline__ double fix_take(unsigned __int128& A, int p) {
     return __longlong_as_double((long long)(((uint64_t)e << 52) | (top & 0xfffffffffffffull)));
   return scalbn((double)(long long)top, n - 52 + p);  // subnormal or infinite
 }
-// The total of the limb sums S in units of 2^(emax - 1118) as hi + lo.
-__device__ __forceinline__ Acc fix_value(const int64_t (&S)[4], int emax) {
-  __int128 t = (__int128)S[0] + ((__int128)S[1] << 24) + ((__int128)S[2] << 48) + ((__int128)S[3] << 72);
+// The total of the limb sums S in units of 2^(emax - 1134) as hi + lo (up to
+// 2^14 values stay inside 127 bits).
+__device__ __forceinline__ Acc fix_value(const int64_t (&S)[kLimbs], int emax) {
+  __int128 t = (__int128)S[0] + ((__int128)S[1] << 16) + ((__int128)S[2] << 40) + ((__int128)S[3] << 64) +
+               ((__int128)S[4] << 88);
   const bool neg = t < 0;
   unsigned __int128 A = neg ? (unsigned __int128)(-t) : (unsigned __int128)t;
   Acc r;
-  r.s = fix_take(A, emax - 1118);
-  r.c = fix_take(A, emax - 1118);
+  r.s = fix_take(A, emax - 1134);
+  r.c = fix_take(A, emax - 1134);
   if (neg) {
     r.s = -r.s;
     r.c = -r.c;
@@ -218,16 +224,16 @@ __device__ __forceinline__ Acc warp_sum(int n, Get get) {
     for (int off = 16; off > 0; off >>= 1) acc_merge(a, acc_shfl_down(a, off));
     return a;
   }
-  int64_t S[4] = {0, 0, 0, 0};
+  int64_t S[kLimbs] = {0, 0, 0, 0, 0};
   for (int base = 0; base < n; base += 32) {
-    int L[4] = {0, 0, 0, 0};
+    int L[kLimbs] = {0, 0, 0, 0, 0};
     if (base + lane < n) {
       const Acc v = get(base + lane);
       fix_add(L, v.s, emax);
       fix_add(L, v.c, emax);
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) S[i] += __reduce_add_sync(0xffffffffu, L[i]);
+    for (int i = 0; i < kLimbs; ++i) S[i] += __reduce_add_sync(0xffffffffu, L[i]);
   }
   return fix_value(S, emax);
 }
@@ -243,7 +249,7 @@ template <int BLOCK, typename Get>
 __device__ __forceinline__ Acc block_sum(int n, Get get) {
   constexpr int kW = BLOCK / 32;
   __shared__ int wexp[kW];
-  __shared__ int64_t wlimb[kW][4];
+  __shared__ int64_t wlimb[kW][kLimbs];
   __shared__ Acc part[kW];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
   int e = 1;
@@ -268,9 +274,9 @@ __device__ __forceinline__ Acc block_sum(int n, Get get) {
     __syncthreads();
     return a;
   }
-  int64_t S[4] = {0, 0, 0, 0};
+  int64_t S[kLimbs] = {0, 0, 0, 0, 0};
   for (int base = 0; base < n; base += blockDim.x) {
-    int L[4] = {0, 0, 0, 0};
+    int L[kLimbs] = {0, 0, 0, 0, 0};
     const int i = base + (int)threadIdx.x;
     if (i < n) {
       const Acc v = get(i);
@@ -278,17 +284,17 @@ __device__ __forceinline__ Acc block_sum(int n, Get get) {
       fix_add(L, v.c, emax);
     }
 #pragma unroll
-    for (int q = 0; q < 4; ++q) S[q] += __reduce_add_sync(0xffffffffu, L[q]);
+    for (int q = 0; q < kLimbs; ++q) S[q] += __reduce_add_sync(0xffffffffu, L[q]);
   }
   if (lane == 0) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) wlimb[warp][i] = S[i];
+    for (int i = 0; i < kLimbs; ++i) wlimb[warp][i] = S[i];
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < nw; ++w) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) S[i] += wlimb[w][i];
+      for (int i = 0; i < kLimbs; ++i) S[i] += wlimb[w][i];
     }
     a = fix_value(S, emax);
   }
