@@ -61,3 +61,17 @@ def test_values_that_cancel(rule, bits, cuda):
     got = total(rule, 2, n, values, cuda, width=4.0)
     want = 1.5 * 16.0 / 4 if rule == L.TQ_RULE_MC else 1.5
     assert got == want
+
+
+def test_fp32_samples_beyond_a_float(cuda):
+    """2^32 samples of one fp32 value: a thread's sum needs 24 + 15 bits, and
+    its error term more than a float where it is not brought back into line."""
+    n, c = 2**32, float(np.float32(1.2345678))
+    lib = L.lib()
+    dom = torch.tensor([[0.0, 1.0]], dtype=torch.float32, device=cuda)
+    par = torch.tensor([c, 0.0, 0.0, 0.0], dtype=torch.float64, device=cuda)
+    out = torch.empty((), dtype=torch.float64, device=cuda)
+    ws = L.workspace.get(lib.tq_mc_fused_workspace_size(1, n), "fused")
+    L.check(lib.tq_mc_fused(L.TQ_F32, 1, n, dom.data_ptr(), L.TQ_FN_EXP_SUM, par.data_ptr(), 1, 0, 0, None,
+                            out.data_ptr(), ws.data_ptr(), ws.numel(), L.stream_handle()), "tq_mc_fused")
+    assert abs(out.item() - c) <= 2.0**-44 * c  # f2_add: 2^-47 an addition of 2^15, mostly cancelling

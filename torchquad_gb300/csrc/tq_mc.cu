@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(kBlock, mc_ctas<FAM, D>()) mc_f32_kernel(McArg
     l[k] = lo[k];
     w[k] = width[k];
   }
-  float hi = 0.f, err = 0.f;  // the sum as a double-float
+  F2 sum{0.f, 0.f};
   const int64_t groups = (a.n_points + G - 1) / G;
   for (int64_t g = (int64_t)blockIdx.x * kBlock + threadIdx.x; g < groups; g += (int64_t)gridDim.x * kBlock) {
     uint32_t r[4 * NB];
@@ -225,13 +225,10 @@ __global__ void __launch_bounds__(kBlock, mc_ctas<FAM, D>()) mc_f32_kernel(McArg
         const float t = fam_term<FAM, float>(f, k, x);
         s = k == 0 ? t : s + t;
       }
-      const float v = p < left ? fam_outer<FAM, float>(f, s) : 0.f;
-      const F2 t = two_sum(hi, v);
-      hi = t.hi;
-      err = __fadd_rn(err, t.lo);
+      sum = f2_add(sum, p < left ? fam_outer<FAM, float>(f, s) : 0.f);
     }
   }
-  mc_finish<float>(a, Acc{(double)hi, (double)err}, width);
+  mc_finish<float>(a, Acc{(double)sum.hi, (double)sum.lo}, width);
 }
 
 }  // namespace tq
