@@ -408,8 +408,9 @@ __device__ void chain_table(ChainTab& tb, const Family<double>& fam, int rule, d
 // coordinate) of the weighted integrand into *out.  Returns false where the
 // factors could leave the range of doubles: the exponent has to stay within
 // [-600, 600] at both ends (that of a Gaussian, a >= 0, is at most 0) and
-// change by at most 300 over a block.  The rules' end weights are half of
-// the interior's at the same place.
+// change by at most 300 over a block; the factor c joins the sum at its end,
+// as c times the first node's value may leave it.  The rules' end weights are
+// half of the interior's at the same place.
 template <int FAM>
 __device__ __forceinline__ bool chain_sum(const Family<double>& fam, const ChainTab& tb, int rule, double x0,
                                           double x1, double h, int64_t j0, int cnt, int64_t n, double* out) {
@@ -423,7 +424,7 @@ __device__ __forceinline__ bool chain_sum(const Family<double>& fam, const Chain
     if (!(a >= 0.0 && e0 >= -600.0 && e1 >= -600.0 && fabs(r0) <= 15.0 &&
           2.0 * a * h * h * (kBlk * kBlk) <= 200.0 && fabs(2.0 * a * h * d1) <= 15.0))
       return false;
-    double F = fam.c * exp(e0), R = exp(r0), P = exp(r0 * (double)kBlk) * tb.q[0];
+    double F = exp(e0), R = exp(r0), P = exp(r0 * (double)kBlk) * tb.q[0];
     if (first) acc = -half * F;
     int left = cnt;
     for (; left >= kBlk; left -= kBlk) {
@@ -440,11 +441,11 @@ __device__ __forceinline__ bool chain_sum(const Family<double>& fam, const Chain
       for (int i = left - 2; i >= 0; --i) p = fma(p, R, tb.t[i]);
       acc = fma(F, p, acc);
     }
-    if (final) acc = fma(-half * fam.c, exp(e1), acc);
+    if (final) acc = fma(-half, exp(e1), acc);
   } else if (FAM == TQ_FN_EXP_SUM) {
     const double e0 = fma(a, x0, fam.b), e1 = fma(a, x1, fam.b);
     if (!(fabs(e0) <= 600.0 && fabs(e1) <= 600.0 && fabs(a * h) <= 15.0)) return false;
-    double f = fam.c * exp(e0);
+    double f = exp(e0);
     if (first) acc = -half * f;
     int left = cnt;
     for (; left >= kBlk; left -= kBlk) {
@@ -452,7 +453,7 @@ __device__ __forceinline__ bool chain_sum(const Family<double>& fam, const Chain
       f *= tb.q[0];
     }
     for (int i = 0; i < left; ++i) acc = fma(f, tb.t[i], acc);
-    if (final) acc = fma(-half * fam.c, exp(e1), acc);
+    if (final) acc = fma(-half, exp(e1), acc);
   } else {
     // f = cos(angle) (oscillatory) or sin(angle) (sum of sines)
     const double ph = FAM == TQ_FN_OSCILLATORY ? 2.0 * CUDART_PI * fam.b : 0.0;
@@ -470,9 +471,8 @@ __device__ __forceinline__ bool chain_sum(const Family<double>& fam, const Chain
     for (int i = 0; i < left; ++i)
       acc = osc ? fma(cs, tb.t[i], fma(-sn, tb.t2[i], acc)) : fma(sn, tb.t[i], fma(cs, tb.t2[i], acc));
     if (final) acc = fma(-half, osc ? cos(fma(a, x1, ph)) : sin(a * x1), acc);
-    acc *= fam.c;
   }
-  *out = acc;
+  *out = acc * fam.c;
   return true;
 }
 
