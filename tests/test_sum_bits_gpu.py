@@ -75,3 +75,15 @@ def test_fp32_samples_beyond_a_float(cuda):
     L.check(lib.tq_mc_fused(L.TQ_F32, 1, n, dom.data_ptr(), L.TQ_FN_EXP_SUM, par.data_ptr(), 1, 0, 0, None,
                             out.data_ptr(), ws.data_ptr(), ws.numel(), L.stream_handle()), "tq_mc_fused")
     assert abs(out.item() - c) <= 2.0**-44 * c  # f2_add: 2^-47 an addition of 2^15, mostly cancelling
+
+
+@pytest.mark.parametrize("S_", [1, 3])
+@pytest.mark.parametrize("rule,dim,n", [(L.TQ_RULE_BOOLE, 3, 13), (L.TQ_RULE_BOOLE, 3, 33), (L.TQ_RULE_BOOLE, 1, 101),
+                                        (L.TQ_RULE_SIMPSON, 1, 4001), (L.TQ_RULE_SIMPSON, 4, 9), (T, 2, 300)])
+def test_values_near_the_top_of_the_range(rule, dim, n, S_, cuda):
+    """The whole-number weights of a rule times fp64 values of 1e305 leave the
+    range of doubles; the integral over the unit cube does not."""
+    values = torch.full((n**dim, S_), 1e305, dtype=torch.float64, device=cuda)
+    dom = torch.tensor([[0.0, 1.0]] * dim, dtype=torch.float64, device=cuda)
+    got = K.weighted_result(rule, dim, n, dom, None, 0, values, torch.float64)
+    assert torch.allclose(got, torch.full_like(got, 1e305), rtol=1e-13, atol=0.0), got

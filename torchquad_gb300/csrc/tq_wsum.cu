@@ -98,12 +98,21 @@ __device__ __forceinline__ F wsum_weight(int rule, int j, bool end) {
   if (rule == TQ_RULE_SIMPSON) return end ? (F)1 : ((j & 1) ? (F)4 : (F)2);
   return end ? (F)7 : ((j & 1) ? (F)32 : ((j & 3) == 2 ? (F)12 : (F)14));
 }
+// 2^e, -1022 <= e <= 1023.
+__device__ __forceinline__ double exp2i(int e) { return __hiloint2double((1023 + e) << 20, 0); }
+// Joined whole-number weights are held 2^join_exp down, no larger than one
+// dimension's.
+__device__ __forceinline__ int join_exp(const WsumArgs& a) {
+  const int bits = a.rule == TQ_RULE_TRAPEZOID ? 1 : a.rule == TQ_RULE_SIMPSON ? 2 : a.rule == TQ_RULE_BOOLE ? 5 : 0;
+  return bits * (a.m - 1);
+}
 template <bool GL>
 __device__ void wsum_join_table(const WsumArgs& a, double* tab) {
   const uint32_t n = (uint32_t)a.n;
+  const double down = exp2i(-join_exp(a));
   for (int j = threadIdx.x; j < (int)a.w.R; j += blockDim.x) {
     uint32_t r = (uint32_t)j;
-    double w = 1.0;
+    double w = down;
     for (int k = 0; k < a.m; ++k) {
       const uint32_t q = r / n, digit = r - q * n;
       r = q;
@@ -319,11 +328,15 @@ struct ExactSum<float> {
   }
 };
 
-// Shared set-up of the kernels: the product of the dimensions' weight scales
-// (a CTA's sums take it at the very end, so its rounding is the same for all
-// nodes: a pair, by a warp of its own while the others read; visible from the
-// next barrier on) and the join table.
+// Shared set-up of the kernels: the join table, and the product of the
+// dimensions' weight scales.  Its power of two (with that of the join table)
+// goes into the rows' outer weights of fp64 sums and the lanes' sums of others
+// (exact; sums of unscaled terms could leave the range of doubles where the
+// integral does not).  The rest, between one and 2^dim, multiplies a CTA's
+// sums at the very end, so its rounding is the same for all nodes: a pair, by
+// a warp of its own while the others read; visible from the next barrier on.
 struct WsumSetup {
+  double pow2;
   Acc scale;
   FastDiv fd;
 };
@@ -332,15 +345,32 @@ __device__ __forceinline__ Acc wsum_scaled(Acc v, Acc s) {
   const double p = v.s * s.s;
   return Acc{p, fma(v.c, s.s, fma(v.s, s.c, fma(v.s, s.s, -p)))};
 }
+__device__ __forceinline__ int scale_exp(double w) {
+  const int f = exp_field(w);
+  return f == 0 || f == 0x7ff ? 0 : min(f - 1023, 1022);
+}
 template <typename T, typename D, bool GL, bool JOIN>
 __device__ __forceinline__ void wsum_setup(const WsumArgs& a, Geo<T>& g, WsumSetup& su, double* tab) {
   geo_setup<T, D>(g, a.rule, a.dim, a.n, (const D*)a.domain);
   if constexpr (JOIN) wsum_join_table<GL>(a, tab);
-  if (threadIdx.x == 0) su.fd = make_fastdiv((uint32_t)a.n);
+  if (threadIdx.x < 32) {
+    const int e = __reduce_add_sync(0xffffffffu, threadIdx.x < a.dim ? scale_exp(g.wscale[threadIdx.x]) : 0);
+    if (threadIdx.x == 0) {
+      su.pow2 = exp2i(max(-900, min(900, e)) + (JOIN ? join_exp(a) : 0));
+      su.fd = make_fastdiv((uint32_t)a.n);
+    }
+  }
   __syncthreads();
   if (threadIdx.x == kBlock - 32) {
-    Acc s{g.wscale[0], 0.0};
-    for (int k = 1; k < a.dim; ++k) s = wsum_scaled(s, Acc{g.wscale[k], 0.0});
+    Acc s{1.0, 0.0};
+    int sum = 0;
+    for (int k = 0; k < a.dim; ++k) {
+      const int e = scale_exp(g.wscale[k]);
+      sum += e;
+      s = wsum_scaled(s, Acc{g.wscale[k] * exp2i(-e), 0.0});
+    }
+    const int left = sum - max(-900, min(900, sum));
+    if (left) s = Acc{scalbn(s.s, left), scalbn(s.c, left)};
     su.scale = s;
   }
 }
@@ -386,10 +416,11 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_kernel(WsumArgs a) {
   const double wi = wsum_weight<double>(a.rule, lane, false);
   for (int64_t u0 = ub; u0 < ue; u0 += 32) {
     const int cnt = (int)min((int64_t)32, ue - u0);
-    double w = 0.0;  // outer weight of unit u0 + lane
+    double wu = 0.0, w = 0.0;  // outer weight of unit u0 + lane, without and with the scales' power of two
     if (lane < cnt) {
       const RowPart pt = row_part(a.w, u0 + lane);
-      w = wsum_outer<GL>(a, su.fd, a.w.row0 + pt.row);
+      wu = wsum_outer<GL>(a, su.fd, a.w.row0 + pt.row);
+      w = wu * su.pow2;
       if (ONE) {
         const int64_t p0 = pt.r0, p1 = p0 + a.w.R - 1;
         double e = 0.0;
@@ -399,7 +430,7 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_kernel(WsumArgs a) {
       }
     }
     F2 wf{0.f, 0.f};
-    if (F32 || PAIR) wf = f2_from_double(w);
+    if (F32 || PAIR) wf = f2_from_double(wu);
     for (int q = 0; q < cnt; ++q) {
       const RowPart pt = row_part(a.w, u0 + q);
       const int64_t j0 = pt.j0;
@@ -460,6 +491,10 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_kernel(WsumArgs a) {
     }
   }
   Acc r = sum.value();
+  if (F32 || PAIR) {
+    r.s *= su.pow2;
+    r.c *= su.pow2;
+  }
   if (side != 0.0) acc_add(r, side);
   if (ONE) {  // the lane's weight (a small integer), then the end nodes
     r.s *= wi;
@@ -509,11 +544,12 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_vec_kernel(WsumArgs a)
   const F* __restrict__ f = (const F*)a.f + s0 + comp;
   const int64_t nwarps = (int64_t)gridDim.x * (kBlock / 32);
   const int64_t units = a.w.units;
+  const double up = F32 ? 1.0 : su.pow2;
   ExactSum<F> sum;
   for (int64_t u = (int64_t)warp * gridDim.x + blockIdx.x; u < units; u += nwarps) {
     const RowPart pt = row_part(a.w, u);
     const int64_t j1 = pt.j0 + pt.len;
-    const double wo = mc ? 1.0 : wsum_outer<GL>(a, su.fd, a.w.row0 + pt.row);
+    const double wo = mc ? 1.0 : wsum_outer<GL>(a, su.fd, a.w.row0 + pt.row) * up;
     for (int64_t jb = pt.j0 + pt.lo; jb < j1; jb += batch) {
       const int nb = (int)min((int64_t)batch, j1 - jb);
       double w = 0.0;  // weight of the batch's node `lane`
@@ -548,7 +584,9 @@ __global__ void __launch_bounds__(kBlock, 4) weighted_sum_vec_kernel(WsumArgs a)
       }
     }
   }
-  part[threadIdx.x] = sum.value();
+  Acc r = sum.value();
+  if (F32) r = Acc{r.s * su.pow2, r.c * su.pow2};
+  part[threadIdx.x] = r;
   __syncthreads();
   const int entries = (kBlock / 32) * per;  // a component's lanes: warp e / per, node e % per
   for (int c = warp; c < ncomp; c += kBlock / 32) {
