@@ -68,7 +68,7 @@ def weighted_sum_into(acc, rule, dim, n, domain, gl_weights, start, values2d):
         ),
         "tq_weighted_sum",
     )
-    L.count_launches(1)
+    L.count_launches(1 if S == 1 else 2)
 
 
 def finalize(acc, rule, dim, domain, n_points, S, out_dtype):
