@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(kBlock)
     const uint4 r = philox_block(seed, sid, offset + (uint64_t)b);
     const int64_t e0 = b * PB;
     int k = small ? (int)((uint32_t)e0 - fdiv((uint32_t)e0, fd) * fd.d) : (int)(e0 % dim);
-    T v[PB];
+    alignas(16) T v[PB];
 #pragma unroll
     for (int l = 0; l < PB; ++l) {
       const T u = Uniform<T>::from(r, l);
