@@ -72,16 +72,12 @@ __device__ Acc grid_tile_sum(const BatchArgs& a, const BatchDesc& d, int64_t til
       return block_reduce<256>(v);
     }
   }
-  // fp64: last-dimension tables of this tile's integral (one
-  // outer-function evaluation per row)
-  bool use_tab = false;
-  if constexpr (std::is_same<T, double>::value) {
-    if (dim >= 2 && n <= kTabMax) use_tab = build_inner_tab<FAM>(*tab, g, fam, last, n32, gl, rule, gln, glw);
-  }
   Acc acc{0.0, 0.0};
   RecurConst rc{1.0, 1.0, 0.0};
   if constexpr (std::is_same<T, double>::value) {
-    if (use_tab) {
+    // last-dimension tables of this tile's integral (one outer-function
+    // evaluation per row)
+    if (dim >= 2 && n <= kTabMax && build_inner_tab<FAM>(*tab, g, fam, last, n32, gl, rule, gln, glw)) {
       if (threadIdx.x == 0) *fdn = make_fastdiv((uint32_t)n);
       __syncthreads();
       acc = tab_rows_sum<FAM>(g, fam, *tab, *rt, dim, rule, gl, n, *fdn, gln, glw, begin, end);
@@ -189,18 +185,6 @@ __device__ Acc grid_tile_sum(const BatchArgs& a, const BatchDesc& d, int64_t til
           const double x1 = linspace_node<double>(a_l, b_l, st_l, n, seg_end - 1);
           if (recur_seg_rule<FAM>(rule, fam, rc, last, s_outer, x0, x1, st_l, jl, seg_end, n32, &v)) {
             sum = v;
-            tabbed = true;
-          }
-        }
-        if (use_tab) {
-          const RowFactor rf = row_factor<FAM>(fam, s_outer);
-          if (rf.ok) {
-            for (int j = jl; j < seg_end; ++j) {
-              const double y = tab_accum<FAM>(0.0, rf.r1, rf.r2, *tab, j) - comp;
-              const double tt = sum + y;
-              comp = (tt - sum) - y;
-              sum = tt;
-            }
             tabbed = true;
           }
         }

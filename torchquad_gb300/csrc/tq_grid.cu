@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kBlock, 2) grid_fused_kernel(FusedArgs args) {
   }
   RecurConst rc{1.0, 1.0, 0.0};
   if constexpr (std::is_same<T, double>::value) {
-    if (!rows_done && !use_tab && !GL) rc = recur_const<FAM>(fam, last, st_l);
+    if (!rows_done && !GL) rc = recur_const<FAM>(fam, last, st_l);
   }
   const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * P; base < total && !rows_done;
@@ -209,13 +209,7 @@ __global__ void __launch_bounds__(kBlock, 2) grid_fused_kernel(FusedArgs args) {
       SegSum<T> seg;
       bool tabbed = false;
       if constexpr (std::is_same<T, double>::value) {
-        if (use_tab) {
-          const RowFactor rf = row_factor<FAM>(fam, s_outer);
-          if (rf.ok) {
-            for (int j = jl; j < seg_end; ++j) seg.add(tab_accum<FAM>(0.0, rf.r1, rf.r2, *tab, j));
-            tabbed = true;
-          }
-        } else if (!GL) {
+        if (!GL) {
           // rows longer than a table: equally spaced nodes by recurrence
           double v;
           const double x0 = linspace_node<double>(a_l, b_l, st_l, n, jl);
