@@ -48,7 +48,7 @@ struct BatchArgs {
 template <typename T, int FAM, int P>
 __device__ Acc grid_tile_sum(const BatchArgs& a, const BatchDesc& d, int64_t tile, int64_t tile0,
                              const Geo<T>& g, const Family<T>& fam, const uint64_t* rstride,
-                             InnerTab* tab, RowTab* rt, ChainTab* ct, FastDiv* fdn, const F2* wsf) {
+                             InnerTab* tab, RowTab* rt, ChainTab* ct, ChainTodo* todo, FastDiv* fdn, const F2* wsf) {
   const int dim = d.dim, rule = d.rule, last = dim - 1;
   const int64_t n = d.n;
   const int n32 = (int)n;
@@ -62,11 +62,13 @@ __device__ Acc grid_tile_sum(const BatchArgs& a, const BatchDesc& d, int64_t til
   const int half = n32 / 2;
   if constexpr (std::is_same<T, double>::value) {
     if (dim == 1 && !gl) {
-      // chains of as many nodes as the tile has for each thread
-      const int len = (int)min((int64_t)kChain, max((int64_t)kBlk, (a.tile_pts / blockDim.x) / kBlk * kBlk));
+      // chains of as many nodes as a whole tile has for each thread, or fewer
+      const int longest = (int)min((int64_t)kChain, max((int64_t)kBlk, (a.tile_pts / blockDim.x) / kBlk * kBlk));
+      const int len = chain_len(end - begin, longest);
       chain_table<FAM>(*ct, fam, rule, st_l, begin);
       __syncthreads();
-      Acc v = chain_rows<FAM>(g, fam, *ct, rule, n, begin, end, len, threadIdx.x, blockDim.x);
+      Acc v = chain_rows<FAM>(g, fam, *ct, *todo, rule, n, begin, end, len, threadIdx.x, blockDim.x,
+                              ((end - begin + len - 1) / len + blockDim.x - 1) / blockDim.x);
       v.s *= wlast;
       v.c *= wlast;
       return block_reduce<256>(v);
@@ -238,15 +240,18 @@ __global__ void __launch_bounds__(256) batch_grid_kernel(BatchArgs a) {
   InnerTab* tab = nullptr;
   RowTab* rt = nullptr;
   ChainTab* ct = nullptr;
+  ChainTodo* todo = nullptr;
   __shared__ FastDiv fdn;
   __shared__ F2 wsf[kMaxDim];  // fp32: the dimensions' weight scales as double-floats
   if constexpr (std::is_same<T, double>::value) {
     __shared__ InnerTab tab_s;
     __shared__ RowTab rt_s;
     __shared__ ChainTab ct_s;
+    __shared__ ChainTodo todo_s;
     tab = &tab_s;
     rt = &rt_s;
     ct = &ct_s;
+    todo = &todo_s;
   }
   __shared__ int64_t ti[8], ts[8], te[8];  // a round's integrals and their tile ranges
   __shared__ int tsep[8];
@@ -323,7 +328,7 @@ __global__ void __launch_bounds__(256) batch_grid_kernel(BatchArgs a) {
       const int64_t tile = base + (int64_t)r * gridDim.x;
       setup(r);
       Acc acc{CUDART_NAN, 0.0};
-      TQ_BATCH_FAMILY((acc = grid_tile_sum<T, FAMC, P>(a, d, tile, tile0, g, fam, rstride, tab, rt, ct, &fdn, wsf)))
+      TQ_BATCH_FAMILY((acc = grid_tile_sum<T, FAMC, P>(a, d, tile, tile0, g, fam, rstride, tab, rt, ct, todo, &fdn, wsf)))
       if (threadIdx.x == 0) a.partials[tile] = acc;
       __syncthreads();
     }

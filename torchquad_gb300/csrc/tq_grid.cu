@@ -171,12 +171,15 @@ __global__ void __launch_bounds__(kBlock, 2) grid_fused_kernel(FusedArgs args) {
       // (a chain's start costs as much as 60 of its nodes), warps in turn
       // over the CTAs
       __shared__ ChainTab ct;
+      __shared__ ChainTodo todo;
       chain_table<FAM>(ct, fam, RULE, st_l, 0);
       __syncthreads();
       const int64_t blk = total / (kBlk * (int64_t)args.sms * 128) + 1;
+      const int len = (int)min((int64_t)kChain, blk * kBlk);
       const int64_t chain = ((int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
-      acc = chain_rows<FAM>(g, fam, ct, RULE, n, 0, total, (int)min((int64_t)kChain, blk * kBlk), chain,
-                            (int64_t)gridDim.x * blockDim.x);
+      const int64_t step = (int64_t)gridDim.x * blockDim.x;
+      acc = chain_rows<FAM>(g, fam, ct, todo, RULE, n, 0, total, len, chain, step,
+                            ((total + len - 1) / len + step - 1) / step);
       acc.s *= wlast;
       acc.c *= wlast;
       rows_done = true;

@@ -476,35 +476,80 @@ __device__ __forceinline__ bool chain_sum(const Family<double>& fam, const Chain
   return true;
 }
 
-// The thread's part of the nodes [begin, end) of a one-dimensional fp64
-// Newton-Cotes grid, without the weight scale: chains of `len` nodes (a
-// multiple of kBlk) from begin + first * len, first + step, ...; nodes of a
-// chain that chain_sum refuses are evaluated one by one.
+// Nodes per chain for `count` nodes of a CTA: as few as leave the number of
+// its warps with chains what it is with the longest (1001 nodes: one warp of
+// 32 chains of 32, not of 8 chains of 128).
+__device__ __forceinline__ int chain_len(int64_t count, int longest) {
+  const int64_t lanes = (count + 32 * longest - 1) / (32 * longest) * 32;
+  return (int)(((count + lanes - 1) / lanes + kBlk - 1) / kBlk * kBlk);
+}
+
+// Chains of a round that chain_sum refused.
+struct ChainTodo {
+  int64_t first[8];         // a warp's chain of lane 0
+  unsigned mask[8];         // its lanes whose chains are refused
+  unsigned char list[256];  // the CTA's threads whose chains are
+};
+
+// The CTA's part of the nodes [begin, end) of a one-dimensional fp64
+// Newton-Cotes grid, without the weight scale (each thread's share is
+// returned): chains of `len` nodes (a multiple of kBlk), in rounds of one a
+// thread, this thread's the chains first, first + step, ... (consecutive over
+// a warp; `round` the number of rounds, equal in the whole CTA).  The nodes of
+// chains that chain_sum refuses are evaluated one by one, spread over all
+// threads of the CTA: left to the chains' own threads, a row of 1001 nodes
+// whose chains are all refused kept 8 threads busy (256 narrow Gaussian rows
+// 151 us; 45 in strips of 16 nodes a thread, 41 this way).
 template <int FAM>
-__device__ Acc chain_rows(const Geo<double>& g, const Family<double>& fam, const ChainTab& tb, int rule, int64_t n,
-                          int64_t begin, int64_t end, int len, int64_t first, int64_t step) {
+__device__ Acc chain_rows(const Geo<double>& g, const Family<double>& fam, const ChainTab& tb, ChainTodo& todo,
+                          int rule, int64_t n, int64_t begin, int64_t end, int len, int64_t first, int64_t step,
+                          int64_t rounds) {
   Acc acc{0.0, 0.0};
   const double h = g.step[0];
-  for (int64_t j0 = begin + first * len; j0 < end; j0 += step * len) {
-    const int cnt = (int)min((int64_t)len, end - j0);
-    const double x0 = linspace_node<double>(g.a[0], g.b[0], h, n, j0);
-    const double x1 = linspace_node<double>(g.a[0], g.b[0], h, n, j0 + cnt - 1);
-    double v;
-    if (chain_sum<FAM>(fam, tb, rule, x0, x1, h, j0, cnt, n, &v)) {
-      acc_add(acc, v);
-    } else {
-      double sum = 0.0, comp = 0.0;
-      for (int64_t j = j0; j < j0 + cnt; ++j) {
-        const double x = linspace_node<double>(g.a[0], g.b[0], h, n, j);
-        const double f = fam_outer<FAM, double>(fam, fam_term<FAM, double>(fam, 0, x));
-        const double y = (double)nc_int(rule, j, n) * f - comp;
-        const double t = sum + y;
-        comp = (t - sum) - y;
-        sum = t;
-      }
-      acc_add(acc, sum);
-      acc_add(acc, -comp);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+  for (int64_t r = 0; r < rounds; ++r) {
+    const int64_t chain = first + r * step, j0 = begin + chain * len;
+    bool refused = false;
+    if (j0 < end) {
+      const int cnt = (int)min((int64_t)len, end - j0);
+      const double x0 = linspace_node<double>(g.a[0], g.b[0], h, n, j0);
+      const double x1 = linspace_node<double>(g.a[0], g.b[0], h, n, j0 + cnt - 1);
+      double v;
+      refused = !chain_sum<FAM>(fam, tb, rule, x0, x1, h, j0, cnt, n, &v);
+      if (!refused) acc_add(acc, v);
     }
+    const unsigned mask = __ballot_sync(0xffffffffu, refused);
+    if (lane == 0) {
+      todo.first[warp] = chain;
+      todo.mask[warp] = mask;
+    }
+    if (!__syncthreads_or(refused)) continue;
+    int before = 0, all = 0;  // refused chains of the warps before this one, of all
+    for (int w = 0; w < nw; ++w) {
+      const int k = __popc(todo.mask[w]);
+      before += w < warp ? k : 0;
+      all += k;
+    }
+    if (refused) todo.list[before + __popc(mask & ((1u << lane) - 1u))] = (unsigned char)threadIdx.x;
+    __syncthreads();
+    double sum = 0.0;
+    int held = 0;  // values in sum
+    for (int e = threadIdx.x; e < all * len; e += blockDim.x) {
+      const int q = e / len, t = todo.list[q];
+      const int64_t j = begin + (todo.first[t >> 5] + (t & 31)) * len + (e - q * len);
+      if (j >= end) continue;
+      const double x = linspace_node<double>(g.a[0], g.b[0], h, n, j);
+      const int place = j == 0 || j == n - 1 ? 0 : 4 + (int)(j & 3);  // an end, or like the node
+      sum = fma((double)nc_coef_f(rule, place, 1 << 30),
+                fam_outer<FAM, double>(fam, fam_term<FAM, double>(fam, 0, x)), sum);
+      if (++held == 16) {
+        acc_add(acc, sum);
+        sum = 0.0;
+        held = 0;
+      }
+    }
+    acc_add(acc, sum);
+    __syncthreads();  // the round's list is rewritten
   }
   return acc;
 }
