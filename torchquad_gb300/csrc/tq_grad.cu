@@ -649,7 +649,7 @@ __device__ void batch_adj_dispatch(const BatchGradArgs& a, const tq_batch_desc& 
 // spread over the sub-partitions' FP64 units (1024 integrals of d = 4, 32
 // nodes: 154 us a call with set-up and products integral by integral in warp 0,
 // 139 this way, 121 with the finalize reading one row of such an integral, 107
-// on the CTAs resident at once).
+// on the CTAs resident at once; 110 since the reductions hold 112 bits).
 constexpr int kAdjWarps = kBlock / 32;
 template <int DM>
 struct AdjRound {

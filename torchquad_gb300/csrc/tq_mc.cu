@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(kBlock) mc_fused_kernel(McArgs a) {
 // looks for its block), their terms unrolled with the parameters in
 // registers.  Instruction issue bounds it: at d = 6 about 70 instructions of
 // Philox and 60 of coordinates, terms and exp a point.  10^7 points, d = 6:
-// 125 us with a block test per draw, 68 us here.
+// 125 us with a block test per draw, 70 us here.
 template <int FAM, int D>
 constexpr int mc_ctas() {  // resident CTAs an SM: registers for parameters and draws without spills
   constexpr int regs = (FAM == TQ_FN_GAUSSIAN ? 4 : 3) * D + 4 * D / gcd_c(D, 4) + 24;

@@ -357,8 +357,11 @@ __device__ void sep_adjoint(const Acc (*dsum)[kSepMaxM<true>], const T* av, int 
 // chain's start, where stepping node by node from strips of 16 took 3 and a
 // start (two exp and the guards, 70 operations) every 16 nodes; the FP64 unit
 // bounds both.  Rounding accumulates over at most kChain / kBlk steps of a
-// factor, fewer than the 16 of the strips.  4096 mixed integrals, a quarter
-// of them such rows: 2.0 ms by strips, 0.63 ms by chains (and the
+// factor, fewer than the 16 of the strips (rms errors of 200 random rows, strips
+// and chains of 128: Gaussians 1.2e-15 and 0.9e-15 of the sum of magnitudes,
+// exponentials 3.7e-16 and 2.3e-16; compensated sums in the chain: the same to
+// two digits).  4096 mixed integrals, a quarter
+// of them such rows: 2.0 ms by strips, 0.62 ms by chains (and the
 // factored integrals spread over the CTAs by integral).
 constexpr int kBlk = 16;    // nodes per block (a multiple of 4: the rules' weight period)
 constexpr int kChain = 128;  // nodes per chain at most
