@@ -41,6 +41,12 @@ static __device__ void nh_body(const NhArgs& a, unsigned bid, unsigned nblk) {
     }
     T f = floor(mul_rn(dh, (T)nevals_exp));  // :102
     f = f < (T)2 ? (T)2 : f;                    // :103 clip(nh, 2, None)
+    // A cube whose variance is not a number (an integrand that overflowed or
+    // is undefined there) keeps two points in a run on the device, whose
+    // result is then not a number; as an integer it would be -2^63, and the
+    // sampler's shares of such a total wrap to endless ranges of tiles.  The
+    // staged form returns it, and the host refuses the negative count.
+    if (a.split && !(f >= (T)2)) f = (T)2;
     nh = (int64_t)f;
     st.neval[c] = nh;
     st.jf[c] = 0.0;
