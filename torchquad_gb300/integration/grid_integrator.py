@@ -24,6 +24,7 @@ from . import _kernels as K
 from .base_integrator import BaseIntegrator
 from .utils import (
     _assemble_result,
+    _in_memory,
     _setup_integration_domain,
     _split_integrand_values,
     _host_domain_check,
@@ -119,7 +120,7 @@ class GridIntegrator(BaseIntegrator):
     def calculate_result(self, function_values, dim, n_per_dim, hs, integration_domain):
         """Apply the composite rule to function values of a calculate_grid
         grid (grid_integrator.py:57-91) with the weighted-sum kernel."""
-        domain = integration_domain
+        domain = _in_memory(integration_domain)
         values, shape, is_complex = _split_integrand_values(function_values)
         gl_w = self._gl_tables(n_per_dim, domain.device)[1]
         if torch.is_grad_enabled() and domain.requires_grad:

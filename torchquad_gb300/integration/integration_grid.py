@@ -14,7 +14,7 @@ import torch
 
 from .. import _lib as L
 from . import _kernels as K
-from .utils import _check_integration_domain, _setup_integration_domain
+from .utils import _check_integration_domain, _in_memory, _setup_integration_domain
 
 
 def _unit01(domain):
@@ -50,6 +50,7 @@ class IntegrationGrid:
                 integration_domain = integration_domain.to(torch.float64)
             if not integration_domain.is_cuda:
                 integration_domain = integration_domain.to(L.require_cuda())
+            integration_domain = _in_memory(integration_domain)
         self._dim = integration_domain.shape[0]
         self._N = int(N ** (1.0 / self._dim) + 1e-8)
         requires_grad = bool(integration_domain.requires_grad)

@@ -8,7 +8,7 @@ from ..integrands import BuiltinIntegrand
 from . import _kernels as K
 from .base_integrator import BaseIntegrator
 from .rng import RNG
-from .utils import _assemble_result, _setup_integration_domain, _split_integrand_values
+from .utils import _assemble_result, _in_memory, _setup_integration_domain, _split_integrand_values
 
 
 class MonteCarlo(BaseIntegrator):
@@ -46,7 +46,7 @@ class MonteCarlo(BaseIntegrator):
 
     def calculate_result(self, function_values, integration_domain):
         """V * sum(f) / N (monte_carlo.py:60-82) with the reduction kernel."""
-        domain = integration_domain
+        domain = _in_memory(integration_domain)
         values, shape, is_complex = _split_integrand_values(function_values)
         n = values.shape[0]
         dim = domain.shape[0]

@@ -82,6 +82,13 @@ def _remember_valid(t):
     _VALID[key] = (ref, t._version, t.data_ptr())
 
 
+def _in_memory(t):
+    """t (differentiably) as the kernels read it: row by row, the values
+    themselves.  A transposed or sliced tensor keeps other strides, a lazily
+    negated one the negated values."""
+    return t.resolve_neg().contiguous()
+
+
 def _setup_integration_domain(dim, integration_domain, backend):
     """Return the domain as a [dim, 2] CUDA tensor (utils.py:110-159).
 
@@ -121,6 +128,7 @@ def _setup_integration_domain(dim, integration_domain, backend):
         t = t.to(torch.float64)
     if t.device != device:
         t = t.to(device)
+    t = _in_memory(t)
     if tuple(t.shape) != (dim, 2):
         raise ValueError(
             "The integration domain has an unexpected shape. "
