@@ -6,6 +6,7 @@ import torch
 
 import torchquad_gb300 as tq
 from torchquad_gb300 import _lib as L
+from torchquad_gb300.integration.utils import _split_integrand_values
 
 F64 = torch.float64
 
@@ -18,6 +19,17 @@ def test_plain_tensor_refuses_lazy_values():
     assert L.plain_tensor(z.conj().imag.resolve_neg())
     assert not L.plain_tensor(z.conj())
     assert not L.plain_tensor(torch._efficientzerotensor(()))
+
+
+def test_integrand_values_are_resolved():
+    z = torch.tensor([[1.0 + 2.0j], [3.0 - 4.0j]])
+    v, shape, is_complex = _split_integrand_values(z.conj())
+    assert is_complex and shape == (1,) and not v.is_neg()
+    assert torch.equal(v, torch.tensor([[1.0, -2.0], [3.0, 4.0]]))
+    one = z[:1, 0].conj().imag  # one value: contiguous and lazily negated
+    assert one.is_neg() and one.is_contiguous()
+    v, _, _ = _split_integrand_values(one)
+    assert not v.is_neg() and v.item() == -2.0
 
 
 def _case(cuda, dtype):

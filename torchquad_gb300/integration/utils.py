@@ -176,11 +176,11 @@ def _split_integrand_values(values):
     is_complex = values.is_complex()
     v = values
     if is_complex:
-        v = torch.view_as_real(v.contiguous())
+        v = torch.view_as_real(v.resolve_conj().contiguous())
     v = v.reshape(values.shape[0], -1)
     if v.dtype not in (torch.float32, torch.float64):
         v = v.to(torch.float64)
-    return v.contiguous(), shape, is_complex
+    return _in_memory(v), shape, is_complex
 
 
 def _assemble_result(flat, shape, is_complex):
